@@ -11,6 +11,7 @@
 
 #include "element.cuh"
 #include "force_pipe.cuh"
+#include "straight.cuh"
 
 namespace tlfea {
 
@@ -165,6 +166,63 @@ __global__ void k_dndu_pre(int n_slots, int E, const int* __restrict__ tile_elem
             ji64[jb + (size_t)(3 * k + j) * TE] = Jinv[k][j];
             ji32[jb + (size_t)(3 * k + j) * TE] = (float)Jinv[k][j];
         }
+}
+
+// The straight-sided geometry (J^-1 and det J from the corners) of every tile slot, and
+// *curved = 1 if an element does not qualify: a mid-edge node further than 4 units in the
+// last place of the coordinates from its edge's midpoint, or a degenerate or non-finite J.
+template <int NPE>
+__global__ void k_straight_geo(int n_slots, int E, const int* __restrict__ tile_elem, const int* __restrict__ conn,
+                               const double* __restrict__ x, const double* __restrict__ y,
+                               const double* __restrict__ z, double* __restrict__ geo64, float* __restrict__ geo32,
+                               int* curved) {
+    constexpr int TE = TILE_ELEMS;
+    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= n_slots) return;
+    const int e = tile_elem[slot];
+    const size_t o = (size_t)(slot / TE) * 10 * TE + slot % TE;
+    double v[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
+    if (e >= 0) {
+        double X[NPE][3], big = 0.0;
+        for (int a = 0; a < NPE; ++a) {
+            const int n = conn[e + (size_t)a * E];
+            X[a][0] = x[n];
+            X[a][1] = y[n];
+            X[a][2] = z[n];
+            for (int d = 0; d < 3; ++d) big = fmax(big, fabs(X[a][d]));
+        }
+        bool ok = big < 1e300;  // (also false for a NaN coordinate below)
+        if constexpr (NPE == 10) {
+            const double tol = 4.0 * 2.220446049250313e-16 * big;
+            for (int k = 0; k < 6; ++k)
+                for (int d = 0; d < 3; ++d)
+                    ok = ok && fabs(X[4 + k][d] - 0.5 * (X[edge_i(k)][d] + X[edge_j(k)][d])) <= tol;
+        }
+        double J[3][3];  // J[d][k] = x_(k+1) - x_0
+        for (int d = 0; d < 3; ++d)
+            for (int k = 0; k < 3; ++k) J[d][k] = X[k + 1][d] - X[0][d];
+        const double dj = det3(J);
+        double JT[3][3];
+        for (int i = 0; i < 3; ++i)
+            for (int j = 0; j < 3; ++j) JT[i][j] = J[j][i];
+        for (int k = 0; k < 3; ++k) {
+            const double ek[3] = {k == 0 ? 1.0 : 0.0, k == 1 ? 1.0 : 0.0, k == 2 ? 1.0 : 0.0};
+            double r[3];
+            solve3_pivot(JT, ek, r);
+            ok = ok && (r[0] != 0.0 || r[1] != 0.0 || r[2] != 0.0);  // a tiny pivot gives zeros
+            for (int j = 0; j < 3; ++j) {
+                ok = ok && fabs(r[j]) < 1e300;
+                v[3 * k + j] = r[j];
+            }
+        }
+        ok = ok && fabs(dj) < 1e300 && dj != 0.0;
+        v[9] = dj;
+        if (!ok) *curved = 1;
+    }
+    for (int m = 0; m < 10; ++m) {
+        geo64[o + (size_t)m * TE] = v[m];
+        geo32[o + (size_t)m * TE] = (float)v[m];
+    }
 }
 
 template <typename R, int NPE, int NQP, int MODE, bool DAMP, bool MR>
@@ -327,6 +385,13 @@ static void free_tiling(Tiling& tl) {
     dfree(tl.ji32);
     dfree(tl.partial64);
     dfree(tl.partial32);
+    dfree(tl.node_soff);
+    dfree(tl.pad_slot);
+    dfree(tl.own_off);
+    dfree(tl.own_gid);
+    dfree(tl.own_ln);
+    dfree(tl.geo64);
+    dfree(tl.geo32);
     tl = Tiling();
 }
 
@@ -398,7 +463,7 @@ static int build_tiling(tlfea_element_s* h, const double* x, const double* y, co
     std::vector<uint16_t> ln_inc_end;
     std::vector<uint16_t> inc((size_t)n_tiles * TE * npe, 0);
     std::vector<uint16_t> lconn((size_t)n_tiles * npe * TE, 0);
-    std::vector<int> stamp((size_t)N, -1), lidx((size_t)N, 0);
+    std::vector<int> stamp((size_t)N, -1), lidx((size_t)N, 0), in_tile((size_t)N, 0);
     std::vector<std::vector<int>> node_slots;  // per boundary gid: pslots (tile order)
     std::vector<int> gid_to_b((size_t)N, -1);
     std::vector<int> bnode_gid;
@@ -413,11 +478,18 @@ static int build_tiling(tlfea_element_s* h, const double* x, const double* y, co
                 const int n = conn[e + (size_t)a * E];
                 if (stamp[n] != tile) {
                     stamp[n] = tile;
+                    in_tile[n] = 0;
                     nodes.push_back(n);
                 }
+                in_tile[n]++;
             }
         }
-        std::sort(nodes.begin(), nodes.end());
+        // local nodes by the number of the tile's elements that touch them, most first, then by
+        // node id: the scatter's loop over a node's elements is as long as the longest in its
+        // warp, so nodes of like counts sit side by side
+        std::sort(nodes.begin(), nodes.end(), [&](int a, int b) {
+            return in_tile[a] != in_tile[b] ? in_tile[a] > in_tile[b] : a < b;
+        });
         const int nl = (int)nodes.size();
         max_local = std::max(max_local, nl);
         for (int l = 0; l < nl; ++l) lidx[nodes[l]] = l;
@@ -514,6 +586,51 @@ static int build_tiling(tlfea_element_s* h, const double* x, const double* y, co
         }
         pad_off[tile + 1] = pad_off[tile] + np;
     }
+    // node slots: counted per node, then handed out in tile order
+    std::vector<int> soff((size_t)N + 1, 0), pad_slot(pad_gid.size(), -1);
+    for (int g : ln_gid) soff[(size_t)g + 1]++;
+    for (int i = 0; i < N; ++i) soff[(size_t)i + 1] += soff[i];
+    std::vector<int> own_off((size_t)n_tiles + 1, 0), own_gid;
+    std::vector<uint16_t> own_ln;
+    {
+        std::vector<int> next(soff.begin(), soff.end() - 1), slot_tile(ln_gid.size()), slot_ln(ln_gid.size());
+        for (int tile = 0; tile < n_tiles; ++tile)
+            for (int k = pad_off[tile]; k < pad_off[tile + 1]; ++k)
+                if (pad_gid[k] >= 0) {
+                    const int sl = next[pad_gid[k]]++;
+                    pad_slot[k] = sl;
+                    slot_tile[sl] = tile;
+                    slot_ln[sl] = k - pad_off[tile];
+                }
+        // owners: the nodes of one tile first, then the shared ones to the emptiest tile
+        std::vector<int> owner((size_t)N, -1), load((size_t)n_tiles, 0);
+        for (int i = 0; i < N; ++i)
+            if (soff[i + 1] - soff[i] == 1) load[slot_tile[soff[i]]]++;
+        for (int i = 0; i < N; ++i) {
+            int best = soff[i];
+            if (soff[i + 1] == best) continue;
+            for (int sl = best + 1; sl < soff[i + 1]; ++sl)
+                if (load[slot_tile[sl]] < load[slot_tile[best]]) best = sl;
+            if (soff[i + 1] - soff[i] > 1) load[slot_tile[best]]++;
+            owner[i] = best;
+        }
+        std::vector<int> mine;
+        for (int tile = 0; tile < n_tiles; ++tile) {
+            mine.clear();
+            for (int k = pad_off[tile]; k < pad_off[tile + 1]; ++k)
+                if (pad_gid[k] >= 0 && owner[pad_gid[k]] == pad_slot[k]) mine.push_back(pad_gid[k]);
+            std::sort(mine.begin(), mine.end(), [&](int a, int b) {
+                const int na = soff[a + 1] - soff[a], nb = soff[b + 1] - soff[b];
+                return na != nb ? na > nb : a < b;
+            });
+            for (int g : mine) {
+                own_gid.push_back(g);
+                own_ln.push_back((uint16_t)slot_ln[owner[g]]);
+            }
+            own_off[tile + 1] = (int)own_gid.size();
+            tl.max_own = std::max(tl.max_own, (int)mine.size());
+        }
+    }
     tl.n_pad = (long long)pad_gid.size();
     tl.max_local_pad = std::max(max_pad, TILE_NODE_PAD);
 
@@ -522,6 +639,14 @@ static int build_tiling(tlfea_element_s* h, const double* x, const double* y, co
     if ((st = upload(&tl.pad_gid, pad_gid, h->stream))) return st;
     if ((st = upload(&tl.pad_dst, pad_dst, h->stream))) return st;
     if ((st = upload(&tl.pad_iend, pad_iend, h->stream))) return st;
+    if ((st = upload(&tl.node_soff, soff, h->stream))) return st;
+    if ((st = upload(&tl.pad_slot, pad_slot, h->stream))) return st;
+    if ((st = upload(&tl.own_off, own_off, h->stream))) return st;
+    if ((st = upload(&tl.own_gid, own_gid, h->stream))) return st;
+    if ((st = upload(&tl.own_ln, own_ln, h->stream))) return st;
+    const size_t ngeo = (size_t)n_tiles * 10 * TE;
+    if ((st = dalloc(&tl.geo64, ngeo)) || (st = dalloc(&tl.geo32, ngeo))) return st;
+    tl.straight = false;
     if ((st = dalloc(&tl.sx, (size_t)tl.n_pad)) || (st = dalloc(&tl.sy, (size_t)tl.n_pad)) ||
         (st = dalloc(&tl.sz, (size_t)tl.n_pad)))
         return st;
@@ -1318,6 +1443,34 @@ int tlfea_element_calc_dndu_pre(tlfea_element h) {
     TLFEA_CUDA(cudaMemcpyAsync(h->X0x, h->x, nb, cudaMemcpyDeviceToDevice, h->stream));
     TLFEA_CUDA(cudaMemcpyAsync(h->X0y, h->y, nb, cudaMemcpyDeviceToDevice, h->stream));
     TLFEA_CUDA(cudaMemcpyAsync(h->X0z, h->z, nb, cudaMemcpyDeviceToDevice, h->stream));
+    // straight-sided meshes: the one-Jacobian geometry beside the per-point streams
+    tl.straight = false;
+    const bool rule_ok = rule_is_symmetric(h);
+    int curved = 1;
+    if (rule_ok) {
+        int* d_curved = nullptr;
+        int st = dalloc(&d_curved, 1);
+        if (st) return st;
+        cudaError_t ec = cudaMemsetAsync(d_curved, 0, sizeof(int), h->stream);
+        const unsigned gb = (unsigned)((n_slots + 127) / 128);
+        if (h->npe == 10)
+            k_straight_geo<10><<<gb, 128, 0, h->stream>>>(n_slots, h->E, tl.tile_elem, h->d_conn, h->x, h->y, h->z,
+                                                         tl.geo64, tl.geo32, d_curved);
+        else
+            k_straight_geo<4><<<gb, 128, 0, h->stream>>>(n_slots, h->E, tl.tile_elem, h->d_conn, h->x, h->y, h->z,
+                                                        tl.geo64, tl.geo32, d_curved);
+        if (ec == cudaSuccess) ec = cudaGetLastError();
+        TLFEA_LAUNCHED(1);
+        if (ec == cudaSuccess)
+            ec = cudaMemcpyAsync(&curved, d_curved, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
+        if (ec == cudaSuccess) ec = cudaStreamSynchronize(h->stream);
+        dfree(d_curved);
+        if (ec != cudaSuccess) {
+            set_error(std::string("calc_dndu_pre: ") + cudaGetErrorString(ec));
+            return TLFEA_CUDA_ERROR;
+        }
+    }
+    tl.straight = (curved == 0);
     positions_changed(h);
     h->precomputed = true;
     SYNC(h);

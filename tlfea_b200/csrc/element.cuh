@@ -74,6 +74,24 @@ struct Tiling {
     double* partial64 = nullptr;
     float* partial32 = nullptr;
     std::vector<int> h_tile_elem;  // host copy of tile_elem
+    // Node slots: every (tile, local node) pair has one, numbered by node (in node order,
+    // a node's slots in tile order), so a node's tile sums are the contiguous range
+    // [node_soff[i], node_soff[i + 1]).  pad_slot: the slot of each padded local node
+    // (-1 = padding).
+    int* node_soff = nullptr;       // N + 1
+    int* pad_slot = nullptr;        // n_pad
+    // Owned nodes: every node belongs to one of the tiles that hold it (the one with the
+    // fewest so far, so the tiles' shares are even); tile t owns entries [own_off[t],
+    // own_off[t + 1]), most slots first: the node, its local index in the tile.
+    int max_own = 0;
+    int* own_off = nullptr;         // n_tiles + 1
+    int* own_gid = nullptr;         // one per node of an element
+    uint16_t* own_ln = nullptr;
+    // Straight-sided elements (straight.cuh): J^-1 (rows dL_1..dL_3 / dx) and det J of each
+    // element, [tile][10][TILE_ELEMS], zero in padding slots; valid while `straight`.
+    bool straight = false;
+    double* geo64 = nullptr;
+    float* geo32 = nullptr;
 };
 
 // Per-call arguments of the tile routine.

@@ -9,6 +9,7 @@
 #include <cstring>
 #include <vector>
 
+#include "lin_cg.cuh"
 #include "mf_tangent.cuh"
 #include "solver.cuh"
 
@@ -644,13 +645,12 @@ static int build_cg_graph(tlfea_solver_s* s, int iters) {
     return TLFEA_OK;
 }
 
-int linear_static_prepare(tlfea_solver_s* s) {
+// The vectors of every CG.
+static int linear_static_prepare(tlfea_solver_s* s) {
     tlfea_element_s* el = s->el;
-    int st = element_build_pattern(el);
-    if (st) return st;
-    if (!s->K) {
+    int st;
+    if (!s->ctl) {
         const size_t n3 = 3 * (size_t)el->N;
-        if ((st = dalloc(&s->K, 9 * (size_t)std::max(el->pat_nnz, 1LL)))) return st;
         if ((st = dalloc(&s->u, n3)) || (st = dalloc(&s->f, n3)) || (st = dalloc(&s->r, n3)) ||
             (st = dalloc(&s->p, n3)) || (st = dalloc(&s->q, n3)))
             return st;
@@ -667,6 +667,27 @@ int linear_static_prepare(tlfea_solver_s* s) {
         s->cg_blocks = std::max(1, std::min(rows_warps, std::max(per_sm, 1) * sms));
         if ((st = dalloc(&s->cg_part, 2 * (size_t)s->cg_blocks))) return st;
     }
+    return TLFEA_OK;
+}
+
+// The stiffness pattern and K's storage, for the solves and calls that assemble it.
+static int prepare_k(tlfea_solver_s* s) {
+    int st = element_build_pattern(s->el);
+    if (st) return st;
+    if (!s->K && (st = dalloc(&s->K, 9 * (size_t)std::max(s->el->pat_nnz, 1LL)))) return st;
+    return TLFEA_OK;
+}
+
+// Positions of a solve that does not assemble K, kept for the products and for assembling
+// it on demand.
+static int keep_positions(tlfea_solver_s* s) {
+    tlfea_element_s* el = s->el;
+    const size_t N = el->N;
+    int st;
+    if (!s->xk && ((st = dalloc(&s->xk, N)) || (st = dalloc(&s->yk, N)) || (st = dalloc(&s->zk, N)))) return st;
+    TLFEA_CUDA(cudaMemcpyAsync(s->xk, el->x, sizeof(double) * N, cudaMemcpyDeviceToDevice, el->stream));
+    TLFEA_CUDA(cudaMemcpyAsync(s->yk, el->y, sizeof(double) * N, cudaMemcpyDeviceToDevice, el->stream));
+    TLFEA_CUDA(cudaMemcpyAsync(s->zk, el->z, sizeof(double) * N, cudaMemcpyDeviceToDevice, el->stream));
     return TLFEA_OK;
 }
 
@@ -692,6 +713,226 @@ static int assemble_k(tlfea_solver_s* s, const double* x, const double* y, const
     return TLFEA_OK;
 }
 
+// The result of a solve and UpdatePositions.
+static int finish_solve(tlfea_solver_s* s, const CgCtl& h) {
+    tlfea_element_s* el = s->el;
+    if (h.status == 1) {
+        set_error("LinearStaticSolver CG: non-positive p*Kp detected; aborting.");
+        // the reference leaves last_iter_count = max_iter and residual = 1 on breakdown
+        s->last_iters = s->max_iter;
+        s->last_res = 1.0;
+    } else {
+        s->last_iters = h.iters;
+        s->last_res = h.rel;
+    }
+    k_update_positions<<<(el->N + 255) / 256, 256, 0, el->stream>>>(el->N, el->x, el->y, el->z, s->u);
+    positions_changed(el);
+    TLFEA_CHECK_LAUNCH();
+    TLFEA_CUDA(cudaStreamSynchronize(el->stream));
+    return TLFEA_OK;
+}
+
+// ---- the linear operator at the reference configuration (lin_cg.cuh).  It applies to the
+// SVK law without damping on straight-sided TET10 meshes, unpreconditioned, unless the
+// assembled K was asked for; whether the positions are the reference configuration is decided
+// on the device.  It is the faster operator at every size, per iteration on a B200: 7.6
+// against 13.8 us at 240 elements and 10.6 against 27 us at 15,360 (both against the assembled
+// K), 111 against 195 us at 480,000 (against the per-point tangent stream).  TET4 keeps the
+// assembled K: its product rounds so much less that CG takes 7% fewer iterations than the
+// reference's, more than its parity tests allow.  So does a mesh of one tile (12.7 us an
+// iteration), where condition numbers of 1e9 (a unit cube of six elements) amplify any
+// change of rounding beyond them.
+constexpr int LIN_MIN_TILES = 2;
+
+static bool lin_applies(const tlfea_solver_s* s) {
+    const tlfea_element_s* el = s->el;
+    return el->npe == 10 && el->tl.n_tiles >= LIN_MIN_TILES && el->tl.straight && el->precomputed && el->tl.n_orphans == 0 && s->precond == 0 && s->op_mode != 1 &&
+           el->material != TLFEA_MATERIAL_MOONEY_RIVLIN && el->eta_d == 0.0 && el->lambda_d == 0.0;
+}
+
+static LinArgs lin_args(tlfea_solver_s* s, CgCtl* ctl) {
+    tlfea_element_s* el = s->el;
+    const Tiling& tl = el->tl;
+    LinArgs A;
+    memset(&A, 0, sizeof(A));  // the key of the captured chunks compares bytes
+    A.N = el->N;
+    A.n_tiles = tl.n_tiles;
+    A.max_local = tl.max_local_pad;
+    A.node_off = tl.node_off;
+    A.pad_off = tl.pad_off;
+    A.pad_gid = tl.pad_gid;
+    A.pad_slot = tl.pad_slot;
+    A.pad_iend = tl.pad_iend;
+    A.inc = tl.inc;
+    A.lconn = tl.lconn;
+    A.geo = tl.geo64;
+    A.node_soff = tl.node_soff;
+    A.own_off = tl.own_off;
+    A.own_gid = tl.own_gid;
+    A.own_ln = tl.own_ln;
+    A.is_fixed = s->is_fixed;
+    A.f = s->f;
+    A.p = s->lin_p;
+    A.u = s->u;
+    A.r = s->r;
+    A.slots = s->lin_slots;
+    A.part = s->lin_part;
+    A.lambda = el->lambda;
+    A.mu = el->mu;
+    A.tol = s->tol;
+    A.max_iter = s->max_iter;
+    A.rule = lin_rule(el);
+    A.ctl = ctl;
+    return A;
+}
+
+static const void* lin_cg_kernel(int threads) {
+    return threads == 512 ? (const void*)k_lin_cg<10, 512>
+                          : (threads == 256 ? (const void*)k_lin_cg<10, 256> : (const void*)k_lin_cg<10, 128>);
+}
+static const void* lin_tiles_kernel() { return (const void*)k_lin_tiles<10>; }
+static size_t lin_smem(const tlfea_solver_s* s, int buffers) {
+    return LinLayout<10>(s->el->tl.max_local_pad, buffers).total;
+}
+
+// A launch that may start while its predecessor drains.
+static cudaError_t launch_dependent(const void* kern, int grid, int block, size_t smem, void** args, cudaStream_t st) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, kern, args);
+}
+
+static int lin_node_blocks(const tlfea_solver_s* s) { return (s->el->N + LIN_NODE_THREADS - 1) / LIN_NODE_THREADS; }
+
+// One iteration: tiles, update, direction.
+static cudaError_t lin_enqueue_iteration(tlfea_solver_s* s, LinArgs& A, cudaStream_t st) {
+    void* tiles[] = {&A, &s->el->d_err};
+    cudaError_t e = launch_dependent(lin_tiles_kernel(), s->lin_tile_blocks, TILE_ELEMS, lin_smem(s, 2), tiles, st);
+    void* args[] = {&A};
+    if (e == cudaSuccess)
+        e = launch_dependent((const void*)k_lin_update, s->lin_update_blocks, LIN_NODE_THREADS, 0, args, st);
+    if (e == cudaSuccess)
+        e = launch_dependent((const void*)k_lin_direction, lin_node_blocks(s), LIN_NODE_THREADS, 0, args, st);
+    return e;
+}
+
+static void lin_drop_graphs(tlfea_solver_s* s) {
+    for (auto& g : s->lin_graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+    s->lin_key.clear();
+}
+
+static constexpr int LIN_CHUNK[2] = {32, 4};  // the tail of a capped solve runs in the short chunks
+
+static int lin_graphs(tlfea_solver_s* s, LinArgs& A) {
+    std::vector<unsigned char> key(sizeof(LinArgs));
+    memcpy(key.data(), &A, sizeof(LinArgs));
+    if (key == s->lin_key && s->lin_graph[0] && s->lin_graph[1]) return TLFEA_OK;
+    lin_drop_graphs(s);
+    cudaStream_t st = s->el->stream;
+    for (int k = 0; k < 2; ++k) {
+        cudaGraph_t g = nullptr;
+        TLFEA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        cudaError_t e1 = cudaSuccess;
+        for (int j = 0; j < LIN_CHUNK[k] && e1 == cudaSuccess; ++j) e1 = lin_enqueue_iteration(s, A, st);
+        const cudaError_t e2 = cudaStreamEndCapture(st, &g);
+        const cudaError_t e3 =
+            (e1 == cudaSuccess && e2 == cudaSuccess) ? cudaGraphInstantiate(&s->lin_graph[k], g, 0) : cudaErrorUnknown;
+        if (g) cudaGraphDestroy(g);
+        if (e3 != cudaSuccess) {
+            s->lin_graph[k] = nullptr;
+            cudaGetLastError();
+            lin_drop_graphs(s);
+            set_error("CG graph capture failed");
+            return TLFEA_CUDA_ERROR;
+        }
+    }
+    s->lin_key = key;
+    return TLFEA_OK;
+}
+
+// The solve on the linear operator; *solved = false (and nothing done) where the positions
+// are not the reference configuration.
+static int lin_solve(tlfea_solver_s* s, bool* solved) {
+    tlfea_element_s* el = s->el;
+    cudaStream_t st = el->stream;
+    const int N = el->N, n3 = 3 * N;
+    *solved = false;
+    if (lin_smem(s, 2) > STRAIGHT_MAX_SMEM) return TLFEA_OK;  // a tile touches too many nodes: the other operators
+    int rc;
+    const size_t np = std::max<size_t>(2 * (size_t)el->tl.n_tiles, (size_t)lin_node_blocks(s));
+    if (!s->lin_slots && (rc = dalloc(&s->lin_slots, 4 * (size_t)el->tl.n_local_total))) return rc;
+    if (!s->lin_p && (rc = dalloc(&s->lin_p, 4 * (size_t)N))) return rc;
+    if (!s->lin_part && (rc = dalloc(&s->lin_part, np))) return rc;
+    TLFEA_CUDA(allow_tile_smem(lin_tiles_kernel()));
+    if (s->lin_threads < 0) {  // the widest blocks of which every tile is resident, 0 = none
+        int sms = 0, per_sm = 0, threads_fit = 0;
+        TLFEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, el->device));
+        TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lin_tiles_kernel(), TILE_ELEMS, lin_smem(s, 2)));
+        s->lin_tile_blocks = std::max(1, std::min(el->tl.n_tiles, per_sm * sms));
+        TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lin_update, LIN_NODE_THREADS, 0));
+        s->lin_update_blocks = std::max(1, std::min((lin_node_blocks(s) + 1) / 2, per_sm * sms));
+        for (int threads : {128, 256, 512}) {
+            TLFEA_CUDA(allow_tile_smem(lin_cg_kernel(threads)));
+            TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lin_cg_kernel(threads), threads,
+                                                                     lin_smem(s, 1)));
+            if (el->tl.n_tiles <= per_sm * sms) threads_fit = threads;
+        }
+        s->lin_threads = threads_fit;
+    }
+    if (el->n_constraint > 0) {
+        k_zero_fixed<<<(n3 + 255) / 256, 256, 0, st>>>(n3, s->is_fixed, s->f);
+        TLFEA_CHECK_LAUNCH();
+    }
+    TLFEA_CUDA(cudaMemsetAsync(s->ctl, 0, sizeof(CgCtl), st));
+    k_at_reference<<<(N + 255) / 256, 256, 0, st>>>(N, el->x, el->y, el->z, el->X0x, el->X0y, el->X0z, s->ctl);
+    TLFEA_CHECK_LAUNCH();
+    LinArgs A = lin_args(s, s->ctl);
+    const bool resident = s->lin_threads > 0;
+    if (resident) A.r = s->lin_p;  // r as node records in the phased form's p (p stays on chip)
+    if (resident) {
+        void* args[] = {&A};
+        TLFEA_CUDA(cudaLaunchCooperativeKernel(lin_cg_kernel(s->lin_threads), dim3(el->tl.n_tiles),
+                                               dim3(s->lin_threads), args, lin_smem(s, 1), st));
+        TLFEA_LAUNCHED(1);
+    } else {
+        k_lin_init<<<lin_node_blocks(s), LIN_NODE_THREADS, 0, st>>>(A);
+        TLFEA_CHECK_LAUNCH();
+    }
+    CgCtl h{};
+    for (long long launched = 0;;) {
+        TLFEA_CUDA(cudaMemcpyAsync(&h, s->ctl, sizeof(CgCtl), cudaMemcpyDeviceToHost, st));
+        TLFEA_CUDA(cudaStreamSynchronize(st));
+        if (h.deformed) return TLFEA_OK;
+        if (resident || h.done || launched >= s->max_iter) break;
+        if ((rc = lin_graphs(s, A))) return rc;
+        const int k = (s->max_iter - launched >= LIN_CHUNK[0]) ? 0 : 1;
+        TLFEA_CUDA(cudaGraphLaunch(s->lin_graph[k], st));
+        TLFEA_LAUNCHED(3LL * LIN_CHUNK[k]);
+        launched += LIN_CHUNK[k];
+    }
+    if (h.status == 3 || (resident && !h.done)) {
+        set_error("LinearStaticSolver CG: a wait between its blocks ran out");
+        return TLFEA_BUDGET_EXCEEDED;
+    }
+    *solved = true;
+    s->lin_last = true;
+    s->mf_last = false;
+    s->k_built = false;
+    if ((rc = keep_positions(s))) return rc;
+    return finish_solve(s, h);
+}
+
 int linear_static_solve(tlfea_solver_s* s) {
     tlfea_element_s* el = s->el;
     if (!el->is_setup) {
@@ -710,18 +951,19 @@ int linear_static_solve(tlfea_solver_s* s) {
         k_mark_fixed<<<(nf + 255) / 256, 256, 0, stream>>>(nf, el->fixed, s->is_fixed);
         TLFEA_CHECK_LAUNCH();
     }
+    if (lin_applies(s)) {
+        bool solved = false;
+        if ((st = lin_solve(s, &solved))) return st;
+        if (solved) return TLFEA_OK;
+    }
+    s->lin_last = false;
     const bool mf = use_matrix_free(s);
     if (mf) {
         // matrix-free K p at these positions: keep a copy (the products' tangent stream is
         // formed from it, and K can still be assembled at them after the update)
         k_zero_fixed<<<(n3 + 255) / 256, 256, 0, stream>>>(n3, s->is_fixed, s->f);
         TLFEA_CHECK_LAUNCH();
-        if (!s->xk && ((st = dalloc(&s->xk, (size_t)N)) || (st = dalloc(&s->yk, (size_t)N)) ||
-                       (st = dalloc(&s->zk, (size_t)N))))
-            return st;
-        TLFEA_CUDA(cudaMemcpyAsync(s->xk, el->x, sizeof(double) * N, cudaMemcpyDeviceToDevice, stream));
-        TLFEA_CUDA(cudaMemcpyAsync(s->yk, el->y, sizeof(double) * N, cudaMemcpyDeviceToDevice, stream));
-        TLFEA_CUDA(cudaMemcpyAsync(s->zk, el->z, sizeof(double) * N, cudaMemcpyDeviceToDevice, stream));
+        if ((st = keep_positions(s))) return st;
         TLFEA_CUDA(cudaMemsetAsync(s->q, 0, sizeof(double) * n3, stream));  // nodes of no element stay 0
         const size_t need = (size_t)el->tl.n_tiles + std::max(1, (el->tl.n_bnodes + 255) / 256);
         if (!s->mf_part && (st = dalloc(&s->mf_part, need))) return st;
@@ -750,6 +992,7 @@ int linear_static_solve(tlfea_solver_s* s) {
         s->k_built = false;
         s->mf_last = true;
     } else {
+        if ((st = prepare_k(s))) return st;
         if ((st = assemble_k(s, el->x, el->y, el->z))) return st;
         s->mf_last = false;
     }
@@ -780,26 +1023,12 @@ int linear_static_solve(tlfea_solver_s* s) {
         launched += chunk;
         if (chunk < 64) chunk *= 2;
     }
-    if (h.status == 1) set_error("LinearStaticSolver CG: non-positive p*Kp detected; aborting.");
-    if (h.status == 1) {
-        // the reference leaves last_iter_count = max_iter and residual = 1 on breakdown
-        s->last_iters = s->max_iter;
-        s->last_res = 1.0;
-    } else {
-        s->last_iters = h.iters;
-        s->last_res = h.rel;
-    }
-    // UpdatePositions
-    k_update_positions<<<(N + 255) / 256, 256, 0, stream>>>(N, el->x, el->y, el->z, s->u);
-    positions_changed(el);
-    TLFEA_CHECK_LAUNCH();
-    TLFEA_CUDA(cudaStreamSynchronize(stream));
-    return TLFEA_OK;
+    return finish_solve(s, h);
 }
 
 int linear_static_apply(tlfea_solver_s* s, const double* d_x, double* d_y) {
     tlfea_element_s* el = s->el;
-    if (!s->k_built && !s->mf_last) {
+    if (!s->k_built && !s->mf_last && !s->lin_last) {
         set_error("LinearStaticSolver::Solve has not assembled K yet");
         return TLFEA_NOT_SETUP;
     }
@@ -807,6 +1036,20 @@ int linear_static_apply(tlfea_solver_s* s, const double* d_x, double* d_y) {
         int st = dalloc(&s->ctl_apply, 1);
         if (st) return st;
         TLFEA_CUDA(cudaMemsetAsync(s->ctl_apply, 0, sizeof(CgCtl), el->stream));
+    }
+    if (s->lin_last) {
+        cudaStream_t st = el->stream;
+        TLFEA_CUDA(cudaMemsetAsync(s->ctl_apply, 0, sizeof(CgCtl), st));
+        LinArgs A = lin_args(s, s->ctl_apply);
+        k_lin_mask<<<(el->N + 255) / 256, 256, 0, st>>>(A, d_x);
+        TLFEA_CHECK_LAUNCH();
+        void* tiles[] = {&A, &el->d_err};
+        TLFEA_CUDA(launch_dependent(lin_tiles_kernel(), s->lin_tile_blocks, TILE_ELEMS, lin_smem(s, 2), tiles, st));
+        TLFEA_LAUNCHED(1);
+        k_lin_collect<<<(el->N + 255) / 256, 256, 0, st>>>(A, d_x, d_y);
+        TLFEA_CHECK_LAUNCH();
+        if (el->blocking) TLFEA_CUDA(cudaStreamSynchronize(st));
+        return TLFEA_OK;
     }
     if (s->mf_last) {
         // matrix-free, at the positions of the last solve (its tangent stream); the
@@ -828,9 +1071,11 @@ int linear_static_apply(tlfea_solver_s* s, const double* d_x, double* d_y) {
 int linear_static_retrieve_k(tlfea_solver_s* s, long long* nnz, int* offsets, int* columns, double* values) {
     tlfea_element_s* el = s->el;
     TLFEA_CUDA(cudaStreamSynchronize(el->stream));
-    if (!s->k_built && s->mf_last) {
-        // the last solve ran matrix-free: assemble K at its positions now
-        int st = assemble_k(s, s->xk, s->yk, s->zk);
+    if (!s->k_built && (s->mf_last || s->lin_last)) {
+        // the last solve did not assemble K: do it at its positions now
+        int st = prepare_k(s);
+        if (st) return st;
+        st = assemble_k(s, s->xk, s->yk, s->zk);
         if (st) return st;
         TLFEA_CUDA(cudaStreamSynchronize(el->stream));
     }
@@ -883,6 +1128,10 @@ void linear_static_free(tlfea_solver_s* s) {
     dfree(s->mf_prec);
     dfree(s->mf_tan);
     dfree(s->mf_pfix);
+    lin_drop_graphs(s);
+    dfree(s->lin_slots);
+    dfree(s->lin_p);
+    dfree(s->lin_part);
     dfree(s->xk);
     dfree(s->yk);
     dfree(s->zk);

@@ -20,6 +20,8 @@ struct CgCtl {
     double rr0, rr, alpha, beta, rel;  // preconditioned: rr holds r.z, rres the true r.r
     double pq;
     double rres;
+    int deformed;  // the positions differ from the reference configuration (lin_cg.cuh)
+    unsigned int arrived;  // grid barrier count of the resident solve (lin_cg.cuh)
 };
 
 // Load of step k of a multi-step run: f_ext = f_base + amp * sin(omega * t_k + phase) * f_var,
@@ -79,6 +81,15 @@ struct tlfea_solver_s {
     uint16_t* mf_pfix = nullptr;   // fixed-DOF flags per padded slot
     double* mf_tan = nullptr;      // F and S per element QP at the last solve's positions
     double *xk = nullptr, *yk = nullptr, *zk = nullptr;  // positions of the last matrix-free solve
+    bool lin_last = false;       // the last solve ran on the linear operator (lin_cg.cuh)
+    double* lin_slots = nullptr;  // 4 per node slot
+    double* lin_p = nullptr;      // 4 per node: p, or the resident solve's r
+    int lin_tile_blocks = 0;      // resident blocks of the tile kernel
+    int lin_update_blocks = 0;    // and of the node update
+    double* lin_part = nullptr;   // partial sums
+    int lin_threads = -1;         // block size of the resident solve (0 = does not fit, -1 = not asked yet)
+    cudaGraphExec_t lin_graph[2] = {nullptr, nullptr};  // chunks of 32 and 4 iterations
+    std::vector<unsigned char> lin_key;                 // what those chunks bake in
     int cg_blocks = 0;
     cudaGraphExec_t cg_graph = nullptr;
     int cg_graph_iters = 0;
