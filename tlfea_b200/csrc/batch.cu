@@ -36,6 +36,7 @@
 #include <cstring>
 #include <vector>
 
+#include "batch_lin.cuh"
 #include "element.cuh"
 
 namespace cg = cooperative_groups;
@@ -87,6 +88,10 @@ struct tlfea_batch_s {
     };
     std::vector<PhaseGraph> phase_graphs;
     // FP32 element work: iterations summed over the refinement passes
+    // straight-sided meshes (batch_lin.cuh)
+    bool lin = false;
+    double *lin_p = nullptr, *lin_slots = nullptr, *lin_pair = nullptr;
+    int *stamp = nullptr, *tile_pair = nullptr, *inst_pair = nullptr, *node_inst = nullptr;
     std::vector<int> iters_total;
     bool refined = false;
     double *rhs = nullptr, *uacc = nullptr;  // correction right-hand side, accumulated solution
@@ -973,7 +978,84 @@ static BatchArgs<R> batch_args(tlfea_batch_s* b) {
 }
 
 template <typename R>
+static size_t general_smem(const tlfea_batch_s* b);
+
+template <typename R>
+static BLinArgs<R> blin_args(tlfea_batch_s* b) {
+    tlfea_element_s* el = b->el;
+    const Tiling& tl = el->tl;
+    BLinArgs<R> A;
+    memset(&A, 0, sizeof(A));
+    A.node_off = tl.node_off;
+    A.pad_off = tl.pad_off;
+    A.pad_gid = tl.pad_gid;
+    A.pad_slot = tl.pad_slot;
+    A.pad_iend = tl.pad_iend;
+    A.inc = tl.inc;
+    A.lconn = tl.lconn;
+    A.node_soff = tl.node_soff;
+    if constexpr (sizeof(R) == 8) {
+        A.geo = tl.geo64;
+        A.lam = b->lam;
+        A.mu = b->mu;
+    } else {
+        A.geo = tl.geo32;
+        A.lam = b->lam32;
+        A.mu = b->mu32;
+    }
+    A.n_tiles = tl.n_tiles;
+    A.max_local = tl.max_local_pad;
+    A.nodes_per_inst = b->shared ? el->N : 0;
+    A.slots_per_inst = b->shared ? (int)tl.n_local_total : 0;
+    A.N = b->N;
+    A.n_inst = b->n_inst;
+    A.n_chunks = b->n_chunks;
+    A.fixed = b->fixed;
+    A.chunk_inst = b->chunk_inst;
+    A.chunk_beg = b->chunk_beg;
+    A.inst_chunk = b->inst_chunk;
+    A.tile_inst = b->tile_inst;
+    A.tile_pair = b->tile_pair;
+    A.inst_pair = b->inst_pair;
+    A.node_inst = b->node_inst;
+    A.u = b->u;
+    A.r = b->r;
+    A.p = b->lin_p;
+    A.slots = b->lin_slots;
+    A.pair = b->lin_pair;
+    A.cpa = b->cpa;
+    A.cpb = b->cpb;
+    A.rr = b->rr;
+    A.fnorm = b->fnorm;
+    A.rel = b->rel;
+    A.alpha = b->alpha;
+    A.f = b->f;
+    A.u0 = b->u0;
+    A.iters = b->iters;
+    A.status = b->status;
+    A.done = b->done;
+    A.n_done = b->n_done;
+    A.stamp = b->stamp;
+    A.flag = b->flag;
+    A.rule = lin_rule(el);
+    A.err = el->d_err;
+    return A;
+}
+
+template <typename R, int NPE>
+static size_t blin_smem(const tlfea_batch_s* b) {
+    return BLinLayout<R, NPE>(b->el->tl.max_local_pad).total;
+}
+
+template <typename R>
 static size_t batch_smem(const tlfea_batch_s* b) {
+    if (b->lin) return b->el->npe == 10 ? blin_smem<R, 10>(b) : blin_smem<R, 4>(b);
+    return general_smem<R>(b);
+}
+
+// Shared memory of the per-point tile routine (curved meshes, and Apply).
+template <typename R>
+static size_t general_smem(const tlfea_batch_s* b) {
     const size_t ml = (size_t)b->el->tl.max_local;
     if (b->shared)
         return (b->el->npe == 10) ? GroupLayout<R, 10>((int)ml).total : GroupLayout<R, 4>((int)ml).total;
@@ -984,6 +1066,7 @@ static size_t batch_smem(const tlfea_batch_s* b) {
 // The kernel instantiation of this batch (shared-mesh or general).
 template <typename R, int NPE, int NQP>
 static const void* batch_kernel(const tlfea_batch_s* b, bool apply) {
+    if (b->lin && !apply) return b->shared ? (const void*)k_bl_cg<R, NPE, true> : (const void*)k_bl_cg<R, NPE, false>;
     if (b->shared)
         return apply ? (const void*)k_batch_apply<R, NPE, NQP, true> : (const void*)k_batch_cg<R, NPE, NQP, true>;
     return apply ? (const void*)k_batch_apply<R, NPE, NQP, false> : (const void*)k_batch_cg<R, NPE, NQP, false>;
@@ -992,12 +1075,15 @@ static const void* batch_kernel(const tlfea_batch_s* b, bool apply) {
 template <typename R, int NPE, int NQP>
 static int batch_grid(tlfea_batch_s* b, int blocks_per_sm, int* grid_out, bool apply = false) {
     const void* kern = batch_kernel<R, NPE, NQP>(b, apply);
-    const size_t smem = batch_smem<R>(b);
+    const size_t smem = apply ? general_smem<R>(b) : batch_smem<R>(b);
     if (smem > 200 * 1024) {
         set_error("batch: a tile touches too many nodes for shared memory");
         return TLFEA_UNSUPPORTED;
     }
-    TLFEA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (b->lin && !apply)
+        TLFEA_CUDA(allow_tile_smem(kern));
+    else
+        TLFEA_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0, sms = 0;
     TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TILE_ELEMS, smem));
     TLFEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->el->device));
@@ -1014,10 +1100,11 @@ template <typename R, int NPE, int NQP>
 static int launch_batch_cg(tlfea_batch_s* b, int grid, double tol, int max_iter, bool warm, cudaStream_t st,
                            const double* f_over = nullptr, const double* u0_over = nullptr) {
     BatchArgs<R> A = batch_args<R>(b);
-    if (f_over) A.f = f_over;
-    if (u0_over) A.u0 = u0_over;
+    BLinArgs<R> B = blin_args<R>(b);
+    if (f_over) A.f = B.f = f_over;
+    if (u0_over) A.u0 = B.u0 = u0_over;
     int w = warm ? 1 : 0;
-    void* args[] = {&A, &tol, &max_iter, &w};
+    void* args[] = {b->lin ? (void*)&B : (void*)&A, &tol, &max_iter, &w};
     TLFEA_CUDA(cudaLaunchCooperativeKernel(batch_kernel<R, NPE, NQP>(b, false), dim3(grid), dim3(TILE_ELEMS), args,
                                            batch_smem<R>(b), st));
     TLFEA_LAUNCHED(1);
@@ -1155,10 +1242,127 @@ static int run_phased(tlfea_batch_s* b, double tol, int max_iter, bool warm, cud
     return TLFEA_OK;
 }
 
+// ---- the same on straight-sided meshes (batch_lin.cuh): three launches per iteration, each
+// allowed to start while its predecessor drains.
+template <typename... P, typename... A>
+static cudaError_t launch_next(void (*kern)(P...), int grid, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(TILE_ELEMS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// The tile kernel's resident grid.
+template <typename R, int NPE, bool SH>
+static int blin_tile_grid(const tlfea_batch_s* b, int* grid) {
+    auto tiles = k_bl_tiles<R, NPE, SH>;
+    TLFEA_CUDA(allow_tile_smem((const void*)tiles));
+    int per_sm = 0, sms = 0;
+    TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tiles, TILE_ELEMS, blin_smem<R, NPE>(b)));
+    TLFEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->el->device));
+    const long long items = (long long)b->el->tl.n_tiles * (SH ? (b->n_inst + BL_GROUP - 1) / BL_GROUP : 1);
+    *grid = (int)std::max(1LL, std::min<long long>(items, (long long)per_sm * sms));
+    return TLFEA_OK;
+}
+
+template <typename R, int NPE, bool SH>
+static int blin_apply(tlfea_batch_s* b, const double* x, double* y, cudaStream_t st) {
+    const BLinArgs<R> A = blin_args<R>(b);
+    int grid = 0;
+    const int rc = blin_tile_grid<R, NPE, SH>(b, &grid);
+    if (rc) return rc;
+    k_bl_mask<R><<<(A.N + 255) / 256, 256, 0, st>>>(A, x);
+    TLFEA_CUDA(launch_next(k_bl_tiles<R, NPE, SH>, grid, blin_smem<R, NPE>(b), st, A, (const int*)nullptr, 0, 0, 0));
+    k_bl_collect<R><<<(A.N + 255) / 256, 256, 0, st>>>(A, x, y);
+    TLFEA_CUDA(cudaGetLastError());
+    TLFEA_LAUNCHED(3);
+    return TLFEA_OK;
+}
+
+template <typename R, int NPE, bool SH>
+static int blin_phased(tlfea_batch_s* b, double tol, int max_iter, bool warm, cudaStream_t st, const double* f_over,
+                       const double* u0_over) {
+    BLinArgs<R> A = blin_args<R>(b);
+    if (f_over) A.f = f_over;
+    if (u0_over) A.u0 = u0_over;
+    const int w = warm ? 1 : 0;
+    const size_t smem = blin_smem<R, NPE>(b);
+    auto tiles = k_bl_tiles<R, NPE, SH>;
+    int tile_grid = 0;
+    {
+        const int rc = blin_tile_grid<R, NPE, SH>(b, &tile_grid);
+        if (rc) return rc;
+    }
+    const int chunk_grid = (b->n_chunks + TILE_ELEMS / 32 - 1) / (TILE_ELEMS / 32);  // one warp per chunk
+    int* base = b->n_done + 1;
+    TLFEA_CUDA(cudaMemsetAsync(b->n_done, 0, 2 * sizeof(int), st));
+    k_bl_start<R><<<chunk_grid, TILE_ELEMS, 0, st>>>(A, w);
+    if (warm) TLFEA_CUDA(launch_next(tiles, tile_grid, smem, st, A, (const int*)base, 0, 0, max_iter));
+    k_bl_residual<R><<<chunk_grid, TILE_ELEMS, 0, st>>>(A, w);
+    k_bl_init<R><<<(b->n_inst + 3) / 4, TILE_ELEMS, 0, st>>>(A, tol);
+    TLFEA_CUDA(cudaGetLastError());
+    TLFEA_LAUNCHED(warm ? 4 : 3);
+    const int prec = sizeof(R) == 4 ? TLFEA_PRECISION_FP32 : TLFEA_PRECISION_FP64;
+    int ctl[2] = {0, 0};
+    for (int chunk = 16; max_iter > 0; chunk = 64) {
+        cudaGraphExec_t ge = nullptr;
+        for (auto& g : b->phase_graphs)
+            if (g.precision == prec && g.tol == tol && g.max_iter == max_iter && g.iters == chunk) ge = g.exec;
+        if (!ge) {
+            cudaGraph_t g = nullptr;
+            TLFEA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+            cudaError_t e = cudaSuccess;
+            for (int j = 0; j < chunk && e == cudaSuccess; ++j) {
+                e = launch_next(tiles, tile_grid, smem, st, A, (const int*)base, j, 1, max_iter);
+                if (e == cudaSuccess) e = launch_next(k_bl_update<R>, chunk_grid, 0, st, A, (const int*)base, j, max_iter);
+                if (e == cudaSuccess)
+                    e = launch_next(k_bl_direction<R>, chunk_grid, 0, st, A, (const int*)base, j, tol, max_iter);
+            }
+            if (e == cudaSuccess) {
+                k_bl_advance<<<1, 1, 0, st>>>(base, chunk);
+                e = cudaGetLastError();
+            }
+            const cudaError_t e2 = cudaStreamEndCapture(st, &g);
+            const cudaError_t e3 = (e == cudaSuccess && e2 == cudaSuccess) ? cudaGraphInstantiate(&ge, g, 0) : e2;
+            if (g) cudaGraphDestroy(g);
+            if (e != cudaSuccess || e3 != cudaSuccess || !ge) {
+                cudaGetLastError();
+                set_error("batch_solve: capture of the iteration chunk failed");
+                return TLFEA_CUDA_ERROR;
+            }
+            b->phase_graphs.push_back({prec, max_iter, chunk, tol, ge});
+        }
+        TLFEA_CUDA(cudaGraphLaunch(ge, st));
+        TLFEA_LAUNCHED(3 * chunk + 1);
+        TLFEA_CUDA(cudaMemcpyAsync(ctl, b->n_done, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
+        TLFEA_CUDA(cudaStreamSynchronize(st));
+        if (ctl[0] >= b->n_inst || ctl[1] >= max_iter) break;
+    }
+    k_bl_finish<R><<<(b->n_inst + 127) / 128, 128, 0, st>>>(A);
+    TLFEA_CUDA(cudaGetLastError());
+    TLFEA_LAUNCHED(1);
+    return TLFEA_OK;
+}
+
 // Dispatch on precision and element type; mode 1 keeps the persistent launch.
 static int bcg_run(tlfea_batch_s* b, bool f32, int grid, double tol, int max_iter, bool warm, cudaStream_t st,
                    const double* f_over = nullptr, const double* u0_over = nullptr) {
     const bool t10 = (b->el->npe == 10);
+    if (b->mode == 0 && b->lin) {
+#define TLFEA_BLIN(R_, NPE_)                                                                    \
+    (b->shared ? blin_phased<R_, NPE_, true>(b, tol, max_iter, warm, st, f_over, u0_over)       \
+               : blin_phased<R_, NPE_, false>(b, tol, max_iter, warm, st, f_over, u0_over))
+        if (t10) return f32 ? TLFEA_BLIN(float, 10) : TLFEA_BLIN(double, 10);
+        return f32 ? TLFEA_BLIN(float, 4) : TLFEA_BLIN(double, 4);
+#undef TLFEA_BLIN
+    }
     if (b->mode == 0) {
         if (t10)
             return f32 ? run_phased<float, 10, 5>(b, tol, max_iter, warm, st, f_over, u0_over)
@@ -1287,6 +1491,40 @@ static int batch_alloc_state(tlfea_batch_s* b) {
         if ((st = dalloc(&b->part64, np)) || (st = dalloc(&b->part32, np))) return st;
     }
     cudaStream_t s = b->el->stream;
+    const Tiling& tl = b->el->tl;
+    const long long lin_slots = tl.n_local_total * (b->shared ? n_inst : 1);
+    if (tl.straight && BLinLayout<double, 10>(tl.max_local_pad).total <= 200 * 1024 && lin_slots < (1LL << 31)) {
+        std::vector<int> tp, ip((size_t)n_inst + 1, 0), ni;
+        size_t pairs = 0;
+        if (b->shared) {
+            for (int i = 0; i <= n_inst; ++i) ip[i] = i * tl.n_tiles;
+            pairs = (size_t)n_inst * tl.n_tiles;
+        } else {
+            std::vector<int> ti(2 * (size_t)tl.n_tiles);
+            TLFEA_CUDA(cudaMemcpy(ti.data(), b->tile_inst, ti.size() * sizeof(int), cudaMemcpyDeviceToHost));
+            tp.resize((size_t)tl.n_tiles);
+            for (int t = 0; t < tl.n_tiles; ++t) {
+                tp[t] = (int)pairs;
+                pairs += (size_t)(ti[2 * t + 1] - ti[2 * t] + 1);
+                for (int i = ti[2 * t]; i <= ti[2 * t + 1]; ++i) ip[(size_t)i + 1]++;
+            }
+            for (int i = 0; i < n_inst; ++i) ip[(size_t)i + 1] += ip[i];
+            ni.resize((size_t)b->N);
+            for (int i = 0; i < n_inst; ++i)
+                for (int n = b->node_off[i]; n < b->node_off[i + 1]; ++n) ni[n] = i;
+        }
+        if ((st = dalloc(&b->lin_p, 4 * (size_t)b->N)) || (st = dalloc(&b->lin_slots, 4 * (size_t)lin_slots)) ||
+            (st = dalloc(&b->lin_pair, pairs)) || (st = dalloc(&b->stamp, (size_t)n_inst)) ||
+            (st = dalloc(&b->tile_pair, tp.size())) || (st = dalloc(&b->inst_pair, ip.size())) ||
+            (st = dalloc(&b->node_inst, ni.size())))
+            return st;
+        TLFEA_CUDA(cudaMemcpy(b->inst_pair, ip.data(), ip.size() * sizeof(int), cudaMemcpyHostToDevice));
+        if (!b->shared) {
+            TLFEA_CUDA(cudaMemcpy(b->tile_pair, tp.data(), tp.size() * sizeof(int), cudaMemcpyHostToDevice));
+            TLFEA_CUDA(cudaMemcpy(b->node_inst, ni.data(), ni.size() * sizeof(int), cudaMemcpyHostToDevice));
+        }
+        b->lin = true;
+    }
     const std::vector<unsigned char> fx = untouched_nodes(b);
     TLFEA_CUDA(cudaMemcpyAsync(b->fixed, fx.data(), (size_t)b->N, cudaMemcpyHostToDevice, s));
     TLFEA_CUDA(cudaMemsetAsync(b->f, 0, n3 * sizeof(double), s));
@@ -1477,6 +1715,8 @@ int tlfea_batch_destroy(tlfea_batch b) {
     dfree(b->cpa); dfree(b->cpb); dfree(b->rr); dfree(b->fnorm); dfree(b->rel);
     dfree(b->alpha); dfree(b->beta); dfree(b->flag); dfree(b->ticket);
     dfree(b->part64); dfree(b->part32);
+    dfree(b->lin_p); dfree(b->lin_slots); dfree(b->lin_pair);
+    dfree(b->stamp); dfree(b->tile_pair); dfree(b->inst_pair); dfree(b->node_inst);
     dfree(b->iters); dfree(b->status); dfree(b->done); dfree(b->n_done);
     if (b->el) tlfea_element_destroy(b->el);
     delete b;
@@ -1761,12 +2001,23 @@ int tlfea_batch_apply(tlfea_batch b, const double* d_x, double* d_y) {
         return TLFEA_NOT_SETUP;
     }
     if (!d_x || !d_y) return TLFEA_INVALID_ARG;
-    int grid = 0;
-    int s = batch_dispatch_grid(b, 0, &grid, true);
-    if (s) return s;
     cudaStream_t st = b->el->stream;
     const bool f32 = b->precision == TLFEA_PRECISION_FP32;
     const bool t10 = b->el->npe == 10;
+    int grid = 0, s = 0;
+    if (b->lin) {
+#define TLFEA_BLIN_APPLY(R_, NPE_) \
+    (b->shared ? blin_apply<R_, NPE_, true>(b, d_x, d_y, st) : blin_apply<R_, NPE_, false>(b, d_x, d_y, st))
+        if (t10)
+            s = f32 ? TLFEA_BLIN_APPLY(float, 10) : TLFEA_BLIN_APPLY(double, 10);
+        else
+            s = f32 ? TLFEA_BLIN_APPLY(float, 4) : TLFEA_BLIN_APPLY(double, 4);
+#undef TLFEA_BLIN_APPLY
+        if (s) return s;
+        TLFEA_CUDA(cudaStreamSynchronize(st));
+        return TLFEA_OK;
+    }
+    if ((s = batch_dispatch_grid(b, 0, &grid, true))) return s;
     auto go = [&](auto tag, const void* fn, size_t smem) -> int {
         using R = typename decltype(tag)::type;
         BatchArgs<R> A = batch_args<R>(b);
@@ -1778,11 +2029,11 @@ int tlfea_batch_apply(tlfea_batch b, const double* d_x, double* d_y) {
     struct TD { using type = double; };
     struct TF { using type = float; };
     if (f32)
-        s = t10 ? go(TF{}, batch_kernel<float, 10, 5>(b, true), batch_smem<float>(b))
-                : go(TF{}, batch_kernel<float, 4, 1>(b, true), batch_smem<float>(b));
+        s = t10 ? go(TF{}, batch_kernel<float, 10, 5>(b, true), general_smem<float>(b))
+                : go(TF{}, batch_kernel<float, 4, 1>(b, true), general_smem<float>(b));
     else
-        s = t10 ? go(TD{}, batch_kernel<double, 10, 5>(b, true), batch_smem<double>(b))
-                : go(TD{}, batch_kernel<double, 4, 1>(b, true), batch_smem<double>(b));
+        s = t10 ? go(TD{}, batch_kernel<double, 10, 5>(b, true), general_smem<double>(b))
+                : go(TD{}, batch_kernel<double, 4, 1>(b, true), general_smem<double>(b));
     if (s) return s;
     TLFEA_CUDA(cudaStreamSynchronize(st));
     return TLFEA_OK;
