@@ -11,7 +11,7 @@
 
 #include "element.cuh"
 #include "force_pipe.cuh"
-#include "straight.cuh"
+#include "force_straight.cuh"
 
 namespace tlfea {
 
@@ -904,6 +904,48 @@ static int launch_pipe(tlfea_element_s* h, const TileArgs<R>& A) {
     return TLFEA_OK;
 }
 
+// The straight-sided kernel applies: SVK, a qualifying mesh, no other kernel asked for.
+static bool force_is_straight(const tlfea_element_s* h) {
+    if (h->force_kernel >= 0 || !h->tl.straight || h->material == TLFEA_MATERIAL_MOONEY_RIVLIN) return false;
+    const size_t smem = h->npe == 10 ? SForceLayout<double, 10>(h->tl.max_local_pad, true).total
+                                     : SForceLayout<double, 4>(h->tl.max_local_pad, true).total;
+    return smem <= STRAIGHT_MAX_SMEM;
+}
+
+// Resident blocks over the tiles (force_straight.cuh).
+template <typename R, int NPE, bool DAMP>
+static int launch_straight(tlfea_element_s* h, const TileArgs<R>& T) {
+    auto kern = k_force_straight<R, NPE, DAMP>;
+    const size_t smem = SForceLayout<R, NPE>(h->tl.max_local_pad, DAMP).total;
+    int& grid = h->straight_grid[(sizeof(R) == 4 ? 2 : 0) + (DAMP ? 1 : 0)];
+    if (grid == 0) {
+        TLFEA_CUDA(allow_tile_smem((const void*)kern));
+        int per_sm = 0, sms = 0;
+        TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, TILE_ELEMS, smem));
+        TLFEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
+        grid = std::max(1, std::min(h->tl.n_tiles, per_sm * sms));
+    }
+    SForceArgs<R> A{};
+    A.T = sforce_tables<R>(h, false);
+    A.x = h->x;
+    A.y = h->y;
+    A.z = h->z;
+    A.X0x = h->X0x;
+    A.X0y = h->X0y;
+    A.X0z = h->X0z;
+    A.v = T.v;
+    A.f_out = T.f_out;
+    A.partial = T.partial;
+    A.lambda = T.lambda;
+    A.mu = T.mu;
+    A.eta = T.eta;
+    A.lamd = T.lamd;
+    A.rule = svk_rule(h);
+    kern<<<grid, TILE_ELEMS, smem, h->stream>>>(A);
+    TLFEA_CHECK_LAUNCH();
+    return TLFEA_OK;
+}
+
 template <typename R, int NPE, int NQP>
 static int force_dispatch(tlfea_element_s* h, const double* d_v, bool fp32) {
     TileArgs<R> A = make_args<R>(h, fp32);
@@ -914,6 +956,8 @@ static int force_dispatch(tlfea_element_s* h, const double* d_v, bool fp32) {
     int st;
     if (h->material == TLFEA_MATERIAL_MOONEY_RIVLIN)  // Mooney-Rivlin runs on the compact-geometry kernel
         st = damp ? launch_tile_geo<R, NPE, NQP, true, true>(h, A) : launch_tile_geo<R, NPE, NQP, false, true>(h, A);
+    else if (force_is_straight(h))
+        st = damp ? launch_straight<R, NPE, true>(h, A) : launch_straight<R, NPE, false>(h, A);
     else if (h->force_kernel == 1)
         st = damp ? launch_tiles<R, NPE, NQP, TILE_FORCE, true>(h, A) : launch_tiles<R, NPE, NQP, TILE_FORCE, false>(h, A);
     else if (h->force_kernel == 2)
@@ -981,11 +1025,13 @@ int element_refresh_u64(tlfea_element_s* h) {
 int element_force(tlfea_element_s* h, const double* d_v, bool fp32) {
     int st;
     // the bulk-copy tile kernels (launch options 0 and 3, and Mooney-Rivlin's) stage the record
-    if ((h->force_kernel == 0 || h->force_kernel == 3 || h->material == TLFEA_MATERIAL_MOONEY_RIVLIN) &&
+    const bool straight = force_is_straight(h);
+    if (!straight &&
+        (h->force_kernel <= 0 || h->force_kernel == 3 || h->material == TLFEA_MATERIAL_MOONEY_RIVLIN) &&
         (st = element_refresh_record(h, fp32)))
         return st;
     if (fp32) {
-        if ((st = element_refresh_u64(h))) return st;
+        if (!straight && (st = element_refresh_u64(h))) return st;
         st = (h->npe == 10) ? force_dispatch<float, 10, 5>(h, d_v, true) : force_dispatch<float, 4, 1>(h, d_v, true);
     } else {
         st = (h->npe == 10) ? force_dispatch<double, 10, 5>(h, d_v, false)

@@ -958,9 +958,12 @@ struct tlfea_element_s {
     int* d_err = nullptr;
     // grid of the persistent force pipeline per (FP32?, damping?), 0 = not yet sized
     int pipe_grid[4] = {0, 0, 0, 0};
-    // launch configuration (tlfea_element_set_launch_config): force kernel
-    // 0 = TMA pipeline, 1 = one tile per block; cap on the pipeline grid (0 = none)
-    int force_kernel = 0;
+    int straight_grid[4] = {0, 0, 0, 0};  // the same of the straight-sided force kernel
+    // launch configuration (tlfea_element_set_launch_config): force kernel 0 = gradient stream,
+    // 1 = one tile per block, 2 = persistent pipeline, 3 = compact stream; -1 (until the caller
+    // chooses) = the straight-sided kernel where the mesh allows it, else 0; cap on the
+    // pipeline grid (0 = none)
+    int force_kernel = -1;
     int pipe_grid_limit = 0;
 };
 
