@@ -65,6 +65,12 @@ struct FOArgs {
     int check;
 };
 
+}  // namespace tlfea
+
+#include "fo_resident.cuh"
+
+namespace tlfea {
+
 // Every block folds the per-block partials of slot `k` in block order.
 __device__ __forceinline__ double fold_partials(const FOArgs& S, int k, double* sh) {
     __syncthreads();
@@ -776,6 +782,393 @@ __global__ void __launch_bounds__(FO_NODE_THREADS) k_fo_final(FOArgs S, FOCtl* C
     C->mode = FO_DONE;
 }
 
+void first_order_drop_graphs(tlfea_solver_s* s);
+
+// ---------------------------------------------------------------------------
+// Straight-sided meshes that are not resident (force_straight.cuh), Nesterov: two launches per
+// inner iteration.  The force tiles read node records and write node slots; the node kernel
+// sums a node's slots, forms the gradient and the norms, and ahead of the stop test the next
+// look-ahead and its records (v_k, kept beside, is what a loop that ends leaves with).  The
+// outer phases stand around eight iterations of a chunk instead of in every one.
+constexpr int FOS_INNER = 8;  // inner iterations per outer phases of a chunk
+
+struct FOStraight {
+    double *x4, *w4, *slots;
+    const int* node_soff;
+    double mass_scale;
+};
+
+__device__ __forceinline__ void fos_enter() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename R>
+__device__ __forceinline__ void fos_record(const FOArgs& S, const FOStraight& Q, int i, const double v[3],
+                                           const double vp[3], const double xp[3]) {
+    double x[3] = {xp[0] + S.dt * v[0], xp[1] + S.dt * v[1], xp[2] + S.dt * v[2]};
+    if constexpr (sizeof(R) == 4) {
+        x[0] -= S.X0x[i];
+        x[1] -= S.X0y[i];
+        x[2] -= S.X0z[i];
+    }
+    st_node(Q.x4 + 4 * (size_t)i, x[0], x[1], x[2]);
+    st_node(Q.w4 + 4 * (size_t)i, (v[0] - vp[0]) * Q.mass_scale, (v[1] - vp[1]) * Q.mass_scale,
+            (v[2] - vp[2]) * Q.mass_scale);
+}
+
+template <typename R>
+__global__ void __launch_bounds__(FO_NODE_THREADS) k_fos_outer_start(FOArgs S, FOStraight Q, FOCtl* C) {
+    __shared__ int flag_sh;
+    fos_enter();
+    if (__ldcg(&C->mode) != FO_OUTER_START) return;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.N; i += gridDim.x * blockDim.x) {
+        const size_t k = 3 * (size_t)i;
+        const double v[3] = {S.vg[k], S.vg[k + 1], S.vg[k + 2]}, vp[3] = {S.vp[k], S.vp[k + 1], S.vp[k + 2]};
+        const double xp[3] = {S.xp[i], S.yp[i], S.zp[i]};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) S.vk[k + d] = v[d];
+        fos_record<R>(S, Q, i, v, vp, xp);  // y = v: the first iteration's beta is 0
+    }
+    if (!fo_last_block(C, &flag_sh) || threadIdx.x != 0) return;
+    C->n_outer += 1;
+    C->t = 0.5 * (1.0 + sqrt(5.0));
+    C->prev_norm_g = C->norm_g = 0.0;
+    C->inner_flag = C->inner = 0;
+    C->last_inner = 0;
+    C->last_norm = 0.0;
+    C->mode = (S.max_inner > 0) ? FO_INNER : FO_OUTER;
+}
+
+template <typename R, int NPE>
+__global__ void __launch_bounds__(TILE_ELEMS, NPE != 10 || sizeof(R) == 4 ? 4 : 3)
+    k_fos_force(SeqForceArgs<R> A, const FOCtl* C) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    asm volatile("griddepcontrol.launch_dependents;");
+    sf_init_barriers(smem_u32(smem + SForceLayout<R, NPE>(A.T.max_local, true).bar));
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (__ldcg(&C->mode) != FO_INNER) return;
+    seq_force_tiles<R, NPE>(A, smem, [](int) { return true; });
+}
+
+template <typename R>
+__global__ void __launch_bounds__(FO_NODE_THREADS) k_fos_node(FOArgs S, FOStraight Q, FOCtl* C) {
+    __shared__ double red[FO_NODE_THREADS / 32][3];
+    __shared__ int flag_sh;
+    fos_enter();
+    if (__ldcg(&C->mode) != FO_INNER) return;
+    const double t = __ldcg(&C->t), tn = 0.5 * (1.0 + sqrt(1.0 + 4.0 * t * t)), beta = (t - 1.0) / tn;
+    double sm[3] = {0.0, 0.0, 0.0};  // ||g||^2, ||v_next||^2, ||v_k||^2
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.N; i += gridDim.x * blockDim.x) {
+        const size_t k = 3 * (size_t)i;
+        const int so = Q.node_soff[i], se = Q.node_soff[i + 1];
+        const bool held = S.nc > 0 && S.jt_off[k] != S.jt_off[k + 1];
+        double f[3], g[3], v[3], vk[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {  // every load before the first store
+            g[d] = S.f_ext[k + d];
+            v[d] = S.vg[k + d];
+            vk[d] = S.vk[k + d];
+        }
+        const double vp[3] = {S.vp[k], S.vp[k + 1], S.vp[k + 2]}, xp[3] = {S.xp[i], S.yp[i], S.zp[i]};
+        node_slot_sum(Q.slots, so, se, f);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) g[d] = f[d] - g[d];
+        if (held) {
+            const double xj[3] = {S.xj[i], S.yj[i], S.zj[i]};
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                for (int q = S.jt_off[k + d]; q < S.jt_off[k + d + 1]; ++q)
+                    g[d] += S.dt * (S.lam[S.jt_col[q]] + S.rho * (xp[d] + S.dt * v[d] - xj[d]));
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const double vn = v[d] - S.alpha * g[d];
+            sm[0] += g[d] * g[d];
+            sm[1] += vn * vn;
+            sm[2] += vk[d] * vk[d];
+            v[d] = vn + beta * (vn - vk[d]);
+            vk[d] = vn;
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            S.vk[k + d] = vk[d];
+            S.vg[k + d] = v[d];
+        }
+        fos_record<R>(S, Q, i, v, vp, xp);
+    }
+    block_sum3<FO_NODE_THREADS>(sm, red);
+    if (threadIdx.x == 0)
+        for (int j = 0; j < 3; ++j) S.red[(size_t)j * S.red_stride + blockIdx.x] = sm[j];
+    if (!fo_last_block(C, &flag_sh)) return;
+    double tot[3] = {0.0, 0.0, 0.0};
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) tot[j] += __ldcg(S.red + (size_t)j * S.red_stride + b);
+    block_sum3<FO_NODE_THREADS>(tot, red);
+    if (threadIdx.x != 0) return;
+    const double norm_g = sqrt(tot[0]);
+    const int inner = C->inner;
+    if (!isfinite(norm_g)) C->status = TLFEA_NONFINITE;
+    if (inner > 0 && fabs(norm_g - C->prev_norm_g) < S.inner_tol) C->inner_flag = 1;
+    if (inner > 0 && fabs(sqrt(tot[1]) - sqrt(tot[2])) < S.inner_tol) C->inner_flag = 1;
+    C->norm_g = C->prev_norm_g = norm_g;
+    C->t = tn;
+    if (C->status || C->inner_flag || inner + 1 >= S.max_inner) {
+        C->inner_total += inner + 1;
+        C->last_inner = inner + 1;
+        C->last_norm = norm_g;
+        C->mode = C->status ? FO_FINAL : FO_OUTER;
+    } else {
+        C->inner = inner + 1;
+    }
+}
+
+// v_prev = v, the constraints and multipliers, the outer stop test.
+__global__ void __launch_bounds__(FO_NODE_THREADS) k_fos_outer(FOArgs S, FOCtl* C) {
+    __shared__ double red_sh[32];
+    __shared__ double fold_sh;
+    __shared__ int flag_sh;
+    fos_enter();
+    if (__ldcg(&C->mode) != FO_OUTER) return;
+    double sc = 0.0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.N; i += gridDim.x * blockDim.x) {
+        const size_t k = 3 * (size_t)i;
+        const double v[3] = {S.vk[k], S.vk[k + 1], S.vk[k + 2]};
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            S.vp[k + d] = v[d];
+            S.vg[k + d] = v[d];
+        }
+        if (S.nc > 0 && S.jt_off[k] != S.jt_off[k + 1]) {
+            const double xp[3] = {S.xp[i], S.yp[i], S.zp[i]}, xj[3] = {S.xj[i], S.yj[i], S.zj[i]};
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                for (int q = S.jt_off[k + d]; q < S.jt_off[k + d + 1]; ++q) {
+                    const int ci = S.jt_col[q];
+                    const double cc = xp[d] + S.dt * v[d] - xj[d];
+                    S.c[ci] = cc;
+                    S.lam[ci] += S.rho * S.dt * cc;
+                    sc += cc * cc;
+                }
+        }
+    }
+    write_partial(S, 3, sc, red_sh);
+    if (!fo_last_block(C, &flag_sh)) return;
+    const double norm_c = sqrt(fold_partials(S, 3, &fold_sh));
+    if (threadIdx.x != 0) return;
+    if (fabs(norm_c) < S.outer_tol) C->outer_flag = 1;
+    if (C->outer_flag || C->outer + 1 >= fo_eff_outer(S)) {
+        C->mode = FO_FINAL;
+    } else {
+        C->outer += 1;
+        C->mode = FO_OUTER_START;
+    }
+}
+
+// Final positions, the force of the last evaluation and the statistics.
+template <typename R>
+__global__ void __launch_bounds__(FO_NODE_THREADS) k_fos_final(FOArgs S, FOStraight Q, FOCtl* C) {
+    __shared__ int flag_sh;
+    fos_enter();
+    if (__ldcg(&C->mode) != FO_FINAL) return;
+    const bool evaluated = __ldcg(&C->inner_total) > 0, moved = __ldcg(&C->n_outer) > 0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < S.N; i += gridDim.x * blockDim.x) {
+        const size_t k = 3 * (size_t)i;
+        const double* w = moved ? S.vk : S.vg;
+        const double v[3] = {w[k], w[k + 1], w[k + 2]};
+        double f[3];
+        node_slot_sum(Q.slots, Q.node_soff[i], evaluated ? Q.node_soff[i + 1] : Q.node_soff[i], f);
+        S.x[i] = S.xp[i] + S.dt * v[0];
+        S.y[i] = S.yp[i] + S.dt * v[1];
+        S.z[i] = S.zp[i] + S.dt * v[2];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            S.vg[k + d] = v[d];
+            if (evaluated) {
+                if constexpr (sizeof(R) == 4)
+                    S.f_int32[k + d] = (float)f[d];
+                else
+                    S.f_int64[k + d] = f[d];
+            }
+        }
+    }
+    if (!fo_last_block(C, &flag_sh) || threadIdx.x != 0) return;
+    S.stat[0] = C->n_outer;
+    S.stat[1] = C->inner_total;
+    S.stat[2] = C->last_inner;
+    S.stat[3] = C->status;
+    *S.stat_norm = C->last_norm;
+    *S.stat_rel = C->last_rel;
+    S.stat[8] = 0;
+    C->mode = FO_DONE;
+}
+
+template <typename... P, typename... Q>
+static cudaError_t launch_next(void (*kern)(P...), int grid, int block, size_t smem, cudaStream_t st, Q... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// The records and slots of the straight-sided paths.
+static int fos_alloc(tlfea_solver_s* s) {
+    if (s->fo_slots) return TLFEA_OK;
+    const size_t N = s->el->N;
+    int st = dalloc(&s->fo_x4, 4 * N) | dalloc(&s->fo_w4, 4 * N) | dalloc(&s->fo_bar, 2);
+    if (!st) st = dalloc(&s->fo_slots, 4 * (size_t)s->el->tl.n_local_total);
+    return st ? TLFEA_CUDA_ERROR : TLFEA_OK;
+}
+
+template <typename R>
+static SeqForceArgs<R> fos_force_args(const tlfea_solver_s* s) {
+    const tlfea_element_s* el = s->el;
+    SeqForceArgs<R> A;
+    memset(&A, 0, sizeof(A));
+    A.T = sforce_tables<R>(el, true);
+    A.x = s->fo_x4;
+    A.w = s->fo_w4;
+    A.slots = s->fo_slots;
+    A.n_seq = A.group = 1;
+    A.lambda = (R)el->lambda;
+    A.mu = (R)el->mu;
+    A.rule = svk_rule(el);
+    return A;
+}
+
+// One Solve() in per-phase launches on a straight-sided mesh (Nesterov).
+template <typename R, int NPE>
+static int run_phased_straight(tlfea_solver_s* s, const FOArgs& S, cudaStream_t st) {
+    tlfea_element_s* el = s->el;
+    FOCtl* C = static_cast<FOCtl*>(s->fo_ctl);
+    const SeqForceArgs<R> A = fos_force_args<R>(s);
+    const FOStraight Q{s->fo_x4, s->fo_w4, s->fo_slots, el->tl.node_soff, el->rho / S.dt};
+    std::vector<unsigned char> key(sizeof(int) + sizeof(S) + sizeof(A));
+    const int variant = 64 | (sizeof(R) == 4 ? 1 : 0) | (NPE == 10 ? 2 : 0);
+    memcpy(key.data(), &variant, sizeof(int));
+    memcpy(key.data() + sizeof(int), &S, sizeof(S));
+    memcpy(key.data() + sizeof(int) + sizeof(S), &A, sizeof(A));
+    const int gn = std::max(1, std::min(s->max_blocks / 4, (S.N + FO_NODE_THREADS - 1) / FO_NODE_THREADS));
+    if (key != s->fo_graph_key) {
+        first_order_drop_graphs(s);
+        auto force = k_fos_force<R, NPE>;
+        const size_t smem = SForceLayout<R, NPE>(el->tl.max_local_pad, true).total;
+        TLFEA_CUDA(allow_tile_smem((const void*)force));
+        int per_sm = 0, sms = 0;
+        TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, force, TILE_ELEMS, smem));
+        TLFEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, el->device));
+        const int gf = std::max(1, std::min(el->tl.n_tiles, per_sm * sms));
+        const int go = std::min(gn, std::max(1, s->max_blocks / 8));  // no-ops most of the time: a small grid
+        const int parts[2] = {1, 4};
+        for (int k = 0; k < 2; ++k) {
+            cudaGraph_t g = nullptr;
+            TLFEA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+            cudaError_t e = cudaSuccess;
+            for (int j = 0; j < parts[k] && e == cudaSuccess; ++j) {
+                e = launch_next(k_fos_outer_start<R>, go, FO_NODE_THREADS, 0, st, S, Q, C);
+                for (int n = 0; n < FOS_INNER && e == cudaSuccess; ++n) {
+                    e = launch_next(force, gf, TILE_ELEMS, smem, st, A, (const FOCtl*)C);
+                    if (e == cudaSuccess) e = launch_next(k_fos_node<R>, gn, FO_NODE_THREADS, 0, st, S, Q, C);
+                }
+                if (e == cudaSuccess) e = launch_next(k_fos_outer, go, FO_NODE_THREADS, 0, st, S, C);
+                if (e == cudaSuccess) e = launch_next(k_fos_final<R>, go, FO_NODE_THREADS, 0, st, S, Q, C);
+            }
+            const cudaError_t e2 = cudaStreamEndCapture(st, &g);
+            cudaGraphExec_t ge = nullptr;
+            const cudaError_t e3 = (e == cudaSuccess && e2 == cudaSuccess) ? cudaGraphInstantiate(&ge, g, 0) : e2;
+            if (g) cudaGraphDestroy(g);
+            if (e != cudaSuccess || e3 != cudaSuccess || !ge) {
+                cudaGetLastError();
+                first_order_drop_graphs(s);
+                set_error("first-order solve: capture of the per-phase chunk failed");
+                return TLFEA_CUDA_ERROR;
+            }
+            s->fo_graph[k] = ge;
+        }
+        s->fo_graph_key = key;
+    }
+    k_fo_start<<<gn, FO_NODE_THREADS, 0, st>>>(S, C);
+    TLFEA_CUDA(cudaGetLastError());
+    TLFEA_LAUNCHED(1);
+    // a part runs eight inner iterations or ends an outer one: a bound on the replays
+    const long long max_parts =
+        4 + (long long)std::max(S.max_outer, 1) * ((long long)std::max(S.max_inner, 0) / FOS_INNER + 2);
+    long long parts = 0;
+    for (int k = S.max_inner > 2 * FOS_INNER ? 1 : 0;; k = 1) {
+        TLFEA_CUDA(cudaGraphLaunch(s->fo_graph[k], st));
+        TLFEA_LAUNCHED((long long)(2 * FOS_INNER + 3) * (k ? 4 : 1));
+        parts += k ? 4 : 1;
+        int mode = 0;
+        TLFEA_CUDA(cudaMemcpyAsync(&mode, &C->mode, sizeof(int), cudaMemcpyDeviceToHost, st));
+        TLFEA_CUDA(cudaStreamSynchronize(st));
+        if (mode == FO_DONE) break;
+        if (parts > max_parts) {
+            set_error("first-order solve: the per-phase loop did not finish within its iteration bounds");
+            return TLFEA_CUDA_ERROR;
+        }
+    }
+    return TLFEA_OK;
+}
+
+// The resident solve's kernel for a block size (threads of the three columns below).
+template <typename R, int NPE>
+static const void* resident_kernel(int column) {
+    constexpr int W = sizeof(R) == 4 ? 512 : 384;
+    return column == 2 ? (const void*)k_fo_resident<R, NPE, W>
+                       : (column == 1 ? (const void*)k_fo_resident<R, NPE, W / 2>
+                                      : (const void*)k_fo_resident<R, NPE, 128>);
+}
+template <typename R>
+static int resident_threads(int column) {
+    constexpr int W = sizeof(R) == 4 ? 512 : 384;
+    return column == 2 ? W : (column == 1 ? W / 2 : 128);
+}
+
+// The widest blocks of which every tile is resident: column 2 (a tile per SM), 1 (two), 0 (as
+// many as fit); -1: not resident.  Asked once per precision.
+template <typename R, int NPE>
+static int resident_column(tlfea_solver_s* s, int* column) {
+    int& c = s->fo_column[sizeof(R) == 4 ? 1 : 0];
+    if (c == -2) {
+        int sms = 0, fit = -1;
+        TLFEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->el->device));
+        const size_t smem = SForceLayout<R, NPE>(s->el->tl.max_local_pad, true).total;
+        for (int k = 0; k < 3; ++k) {
+            int per_sm = 0;
+            TLFEA_CUDA(allow_tile_smem(resident_kernel<R, NPE>(k)));
+            TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resident_kernel<R, NPE>(k),
+                                                                     resident_threads<R>(k), smem));
+            if (s->el->tl.n_tiles <= std::min(per_sm * sms, s->max_blocks)) fit = k;
+        }
+        c = fit;
+    }
+    *column = c;
+    return TLFEA_OK;
+}
+
+template <typename R, int NPE>
+static int launch_resident(tlfea_solver_s* s, FOArgs& S, int column, cudaStream_t st) {
+    const Tiling& tl = s->el->tl;
+    SeqForceArgs<R> A = fos_force_args<R>(s);
+    FOResident Q{s->fo_x4, s->fo_w4,  tl.own_off, tl.own_gid, tl.node_soff, reinterpret_cast<unsigned int*>(s->fo_bar),
+                 s->fo_bar + 1, s->el->rho / S.dt};
+    TLFEA_CUDA(cudaMemsetAsync(s->fo_bar, 0, sizeof(int), st));
+    void* args[] = {&S, &A, &Q};
+    TLFEA_CUDA(cudaLaunchCooperativeKernel(resident_kernel<R, NPE>(column), dim3(tl.n_tiles),
+                                           dim3(resident_threads<R>(column)), args,
+                                           SForceLayout<R, NPE>(tl.max_local_pad, true).total, st));
+    TLFEA_LAUNCHED(1);
+    return TLFEA_OK;
+}
+
 template <typename R, int NPE, int NQP, bool DAMP, bool MR, bool MASS>
 static int launch_first_order(tlfea_solver_s* s, FOArgs& S, TileArgs<R>& A) {
     tlfea_element_s* el = s->el;
@@ -797,8 +1190,6 @@ static int launch_first_order(tlfea_solver_s* s, FOArgs& S, TileArgs<R>& A) {
     TLFEA_LAUNCHED(1);
     return TLFEA_OK;
 }
-
-void first_order_drop_graphs(tlfea_solver_s* s);
 
 // One slot of per-phase launches (every state's kernels, each a no-op unless the
 // state is its own).
@@ -917,6 +1308,7 @@ void first_order_free(tlfea_solver_s* s) {
     first_order_drop_graphs(s);
     if (s->fo_ctl) cudaFree(s->fo_ctl);
     s->fo_ctl = nullptr;
+    dfree(s->fo_x4); dfree(s->fo_w4); dfree(s->fo_slots); dfree(s->fo_bar); dfree(s->fo_stat);
 }
 
 // f_ext = f_base + a * f_var, rounded multiply then rounded add (no fused
@@ -929,6 +1321,77 @@ __global__ void k_step_load(int n3, const double* __restrict__ f_base, const dou
 
 static int first_order_finish(tlfea_solver_s* s, const std::vector<int>& hs, int n_steps, int* inner_iters,
                               float ms, bool fp32);
+
+// The steps on a straight-sided mesh: each step's load, its solve, its statistics.
+static int straight_steps(tlfea_solver_s* s, const FOArgs& S0, int n_steps, const StepLoad* load, int* inner_iters,
+                          bool fp32, int column) {
+    tlfea_element_s* el = s->el;
+    cudaStream_t stream = el->stream;
+    if (s->fo_stat_steps < n_steps) {
+        dfree(s->fo_stat);
+        s->fo_stat_steps = 0;
+        int rc = dalloc(&s->fo_stat, 16 * (size_t)n_steps);
+        if (rc) return rc;
+        s->fo_stat_steps = n_steps;
+    }
+    TLFEA_CUDA(cudaMemsetAsync(s->fo_bar, 0, 2 * sizeof(int), stream));
+    cudaEvent_t e0, e1;
+    cudaEventCreate(&e0);
+    cudaEventCreate(&e1);
+    cudaEventRecord(e0, stream);
+    int st = TLFEA_OK;
+    for (int k = 0; k < n_steps && !st; ++k) {
+        if (load) {
+            const double tk = load->t0 + (k + 1) * S0.dt;
+            const double a = load->amp * sin(load->omega * tk + load->phase);
+            const int n3 = 3 * el->N;
+            k_step_load<<<(n3 + 255) / 256, 256, 0, stream>>>(n3, load->f_base, load->f_var, a, el->f_ext);
+            if (cudaGetLastError() != cudaSuccess) st = TLFEA_CUDA_ERROR;
+        }
+        FOArgs S = S0;
+        S.stat = s->fo_stat + 16 * (size_t)k;
+        S.stat_norm = (double*)(S.stat + 4);
+        S.stat_rel = (double*)(S.stat + 6);
+        if (st) break;
+        if (column >= 0) {
+            st = fp32 ? (el->npe == 10 ? launch_resident<float, 10>(s, S, column, stream)
+                                       : launch_resident<float, 4>(s, S, column, stream))
+                      : (el->npe == 10 ? launch_resident<double, 10>(s, S, column, stream)
+                                       : launch_resident<double, 4>(s, S, column, stream));
+        } else {
+            S.stat = s->dstat;  // the captured chunks keep their arguments from step to step
+            S.stat_norm = S0.stat_norm;
+            S.stat_rel = S0.stat_rel;
+            st = fp32 ? (el->npe == 10 ? run_phased_straight<float, 10>(s, S, stream)
+                                       : run_phased_straight<float, 4>(s, S, stream))
+                      : (el->npe == 10 ? run_phased_straight<double, 10>(s, S, stream)
+                                       : run_phased_straight<double, 4>(s, S, stream));
+            if (!st && cudaMemcpyAsync(s->fo_stat + 16 * (size_t)k, s->dstat, 16 * sizeof(int), cudaMemcpyDeviceToDevice,
+                                       stream) != cudaSuccess)
+                st = TLFEA_CUDA_ERROR;
+        }
+    }
+    cudaEventRecord(e1, stream);
+    std::vector<int> hs(16 * (size_t)n_steps);
+    int bar[2] = {0, 0};
+    cudaError_t e = cudaMemcpyAsync(hs.data(), s->fo_stat, hs.size() * sizeof(int), cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(bar, s->fo_bar, sizeof(bar), cudaMemcpyDeviceToHost, stream);
+    const cudaError_t es = cudaStreamSynchronize(stream);
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventDestroy(e0);
+    cudaEventDestroy(e1);
+    if (st) return st;
+    if (e != cudaSuccess || es != cudaSuccess) {
+        set_error(std::string("first-order solve: ") + cudaGetErrorString(e != cudaSuccess ? e : es));
+        return TLFEA_CUDA_ERROR;
+    }
+    if (bar[1]) {
+        set_error("first-order solve: a wait between its blocks ran out");
+        return TLFEA_BUDGET_EXCEEDED;
+    }
+    return first_order_finish(s, hs, n_steps, inner_iters, ms, fp32);
+}
 
 // One Solve(), or n implicit steps with a time-varying load (new).
 int first_order_steps(tlfea_solver_s* s, int steps, const StepLoad* load, int* inner_iters) {
@@ -1049,6 +1512,22 @@ int first_order_steps(tlfea_solver_s* s, int steps, const StepLoad* load, int* i
     cudaStream_t stream = el->stream;
     const int n_steps = std::max(1, steps);
     st = TLFEA_OK;
+    // the straight-sided paths (explicit launch modes keep the general kernels): the resident
+    // solve where every tile fits, else Nesterov's per-phase launches
+    const size_t straight_smem = el->npe == 10 ? SForceLayout<double, 10>(el->tl.max_local_pad, true).total
+                                               : SForceLayout<double, 4>(el->tl.max_local_pad, true).total;
+    const bool straight = s->fo_mode == 0 && mass && !damp && el->tl.straight && el->tl.n_orphans == 0 &&
+                          straight_smem <= 200 * 1024;
+    if (straight) {
+        int column = -1;
+        st = fp32 ? (el->npe == 10 ? resident_column<float, 10>(s, &column) : resident_column<float, 4>(s, &column))
+                  : (el->npe == 10 ? resident_column<double, 10>(s, &column) : resident_column<double, 4>(s, &column));
+        if (st) return st;
+        if (column >= 0 || s->kind == KIND_NESTEROV) {
+            if ((st = fos_alloc(s))) return st;
+            return straight_steps(s, S, n_steps, load, inner_iters, fp32, column);
+        }
+    }
     // per-phase launches by default from FO_PHASED_MIN_NODES nodes: below it the host
     // round trip of each chunk outweighs the persistent kernel's latency (the 100x10x10
     // beam, 88,641 nodes: 97 against 127 steps/s), above it the phases' occupancy wins

@@ -53,6 +53,14 @@ struct tlfea_solver_s {
     void* fo_ctl = nullptr;  // per-phase mode: the device-side loop state
     cudaGraphExec_t fo_graph[2] = {nullptr, nullptr};  // per-phase mode: chunks of 8 and 32 slots
     std::vector<unsigned char> fo_graph_key;             // what the captured chunks bake in
+    // straight-sided meshes: node records, node slots, grid barrier count and failure word,
+    // statistics of each step, and the block size of the resident solve per precision (-1: not
+    // resident, -2: not asked yet)
+    double *fo_x4 = nullptr, *fo_w4 = nullptr, *fo_slots = nullptr;
+    int* fo_bar = nullptr;
+    int* fo_stat = nullptr;
+    int fo_stat_steps = 0;
+    int fo_column[2] = {-2, -2};
     tlfea_nesterov_params np{};
     tlfea_adamw_params ap{};
     bool params_set = false;
