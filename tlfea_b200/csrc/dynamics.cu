@@ -36,6 +36,7 @@
 #include <cstring>
 #include <vector>
 
+#include "force_straight.cuh"
 #include "solver.cuh"
 
 namespace tlfea {
@@ -81,6 +82,12 @@ struct DynArgs {
     int restart;
     int* mom;
     double* red2;
+    // straight-sided meshes: node records and node slots (force_straight.cuh)
+    double *x4, *w4, *slots;
+    const int* node_soff;
+    long long n_slots;   // per sequence
+    double mass_scale;   // rho / dt
+    int grad_blocks;     // blocks per sequence of the gradient
 };
 
 // ---------------------------------------------------------------- kernels
@@ -174,6 +181,36 @@ __global__ void __launch_bounds__(TILE_ELEMS, (DAMP || NPE != 10) ? 1 : 3) k_dyn
     process_tile<double, NPE, NQP, TILE_FORCE, DAMP, false, true, true>(A, tile, smem, &sq);
 }
 
+// End of a sequence's gradient phase (one thread): a = ||g_free||^2, a_dy = g . (y - v_k),
+// a_gg = ||g||^2.
+__device__ __forceinline__ void dyn_end_iteration(const DynArgs& D, int s, double a, double a_dy, double a_gg) {
+    D.ticket[s] = 0u;
+    // g . (v_next - v_k) = g . (y - v_k) - alpha ||g||^2 > 0: the step works against
+    // the momentum, so the next look-ahead starts the beta sequence afresh
+    const bool restart_now = D.restart && (a_dy - D.alpha_s[s] * a_gg > 0.0);
+    D.mom[s] = restart_now ? 0 : D.mom[s] + 1;
+    const double fe = *D.fext_norm;
+    const double rel = fe > 0.0 ? sqrt(a) / fe : sqrt(a);
+    D.rel[s] = rel;
+    const int it = D.inner[s] + 1;
+    D.inner[s] = it;
+    D.inner_total[s] += 1;
+    int nd = DYN_RUNNING;
+    if (!isfinite(rel)) {
+        D.status[s] = TLFEA_NONFINITE;
+        nd = DYN_RULE_MET;  // stop without another update
+    } else if (D.rel_tol > 0.0 && rel < D.rel_tol) {
+        D.rule_met[s] = 1;
+        nd = DYN_RULE_MET;  // keep v = y: the positions the residual was measured at
+    } else if (it >= D.max_inner) {
+        nd = DYN_OUT_OF_ITERS;  // one more velocity update, no look-ahead
+    }
+    if (nd != DYN_RUNNING) {
+        D.done[s] = nd;
+        atomicAdd(D.n_done, 1);
+    }
+}
+
 // Node force, gradient, ||g_free||^2 partials; the last block of a sequence folds them and
 // applies the stop rule.
 __global__ void __launch_bounds__(DYN_NODE_THREADS) k_dyn_grad(DynArgs D) {
@@ -258,33 +295,161 @@ __global__ void __launch_bounds__(DYN_NODE_THREADS) k_dyn_grad(DynArgs D) {
         a_dy = warp_sum(a_dy);
         a_gg = warp_sum(a_gg);
         if (threadIdx.x == 0) {
-            D.ticket[s] = 0u;
-            // g . (v_next - v_k) = g . (y - v_k) - alpha ||g||^2 > 0: the step works against
-            // the momentum, so the next look-ahead starts the beta sequence afresh
-            const bool restart_now = D.restart && (a_dy - D.alpha_s[s] * a_gg > 0.0);
-            D.mom[s] = restart_now ? 0 : D.mom[s] + 1;
-            const double fe = *D.fext_norm;
-            const double rel = fe > 0.0 ? sqrt(a) / fe : sqrt(a);
-            D.rel[s] = rel;
-            const int it = D.inner[s] + 1;
-            D.inner[s] = it;
-            D.inner_total[s] += 1;
-            int nd = DYN_RUNNING;
-            if (!isfinite(rel)) {
-                D.status[s] = TLFEA_NONFINITE;
-                nd = DYN_RULE_MET;  // stop without another update
-            } else if (D.rel_tol > 0.0 && rel < D.rel_tol) {
-                D.rule_met[s] = 1;
-                nd = DYN_RULE_MET;  // keep v = y: the positions the residual was measured at
-            } else if (it >= D.max_inner) {
-                nd = DYN_OUT_OF_ITERS;  // one more velocity update, no look-ahead
-            }
-            if (nd != DYN_RUNNING) {
-                D.done[s] = nd;
-                atomicAdd(D.n_done, 1);
-            }
+            dyn_end_iteration(D, s, a, a_dy, a_gg);
         }
     }
+}
+
+// ---- straight-sided meshes (force_straight.cuh).  The same iteration with the node values the
+// force needs, x and rho (y - v_prev) / dt, kept as 32-byte records (written by the velocity
+// update, so the tiles gather two records per node instead of nine scattered values) and the
+// tile sums in node slots.  The node kernels issue every load before their first store: with
+// the two interleaved the compiler has to keep their order, and each store waits for a round
+// trip (at 16 sequences of 88,641 nodes 149 us for the two kernels, 149 before).
+__device__ __forceinline__ void dyn_record(const DynArgs& D, size_t node, const double xp[3], const double vp[3],
+                                           const double y[3]) {
+    st_node(D.x4 + 4 * node, xp[0] + D.dt * y[0], xp[1] + D.dt * y[1], xp[2] + D.dt * y[2]);
+    st_node(D.w4 + 4 * node, (y[0] - vp[0]) * D.mass_scale, (y[1] - vp[1]) * D.mass_scale,
+            (y[2] - vp[2]) * D.mass_scale);
+}
+
+__global__ void __launch_bounds__(DYN_NODE_THREADS) k_dyn_start_straight(DynArgs D) {
+    const int s = blockIdx.y;
+    if (D.done[s] != DYN_RUNNING) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= D.N) return;
+    const size_t o = (size_t)s * D.N + i, b3 = 3 * o;
+    const double y[3] = {D.vg[b3], D.vg[b3 + 1], D.vg[b3 + 2]}, vp[3] = {D.vp[b3], D.vp[b3 + 1], D.vp[b3 + 2]};
+    const double xp[3] = {D.xp[o], D.yp[o], D.zp[o]};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) D.vk[b3 + d] = y[d];
+    dyn_record(D, o, xp, vp, y);
+}
+
+template <int NPE>
+__global__ void __launch_bounds__(TILE_ELEMS, NPE == 10 ? 3 : 4) k_dyn_force_straight(DynArgs D, SeqForceArgs<double> A) {
+    extern __shared__ __align__(128) unsigned char smem[];
+    asm volatile("griddepcontrol.launch_dependents;");
+    sf_init_barriers(smem_u32(smem + SForceLayout<double, NPE>(A.T.max_local, true).bar));
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // an out-of-iterations sequence has had its last velocity update: finished from now on
+    // (the blocks of this kernel read either value and skip alike)
+    if (blockIdx.x == 0)
+        for (int s = threadIdx.x; s < D.B; s += blockDim.x)
+            if (D.done[s] == DYN_OUT_OF_ITERS) D.done[s] = DYN_FINISHED;
+    seq_force_tiles<double, NPE>(A, smem, [&](int s) { return __ldcg(D.done + s) == DYN_RUNNING; });
+}
+
+// As k_dyn_grad, DYN_GRAD_NODES nodes per thread: a block that ends pays the reduction's fence
+// and ticket, so a sequence has few blocks.
+constexpr int DYN_GRAD_NODES = 4;
+__global__ void __launch_bounds__(DYN_NODE_THREADS) k_dyn_grad_straight(DynArgs D) {
+    __shared__ double red_sh[32];
+    __shared__ bool last;
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int s = blockIdx.y;
+    if (__ldcg(D.done + s) != DYN_RUNNING) return;
+    const size_t oN = (size_t)s * D.N, o3 = 3 * oN;
+    const double* slots = D.slots + 4 * (size_t)s * D.n_slots;
+    double sg = 0.0, gdy = 0.0, gg = 0.0;
+    const int stride = gridDim.x * blockDim.x;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < D.N; i += stride) {
+        const size_t k = o3 + 3 * (size_t)i;
+        const int so = D.node_soff[i], se = D.node_soff[i + 1];
+        const bool held = D.node_fixed[i] != 0;
+        double r[3], dv[3] = {0.0, 0.0, 0.0}, f[3];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            r[d] = -D.f_ext[3 * (size_t)i + d];
+            if (D.restart) dv[d] = D.vg[k + d] - D.vk[k + d];
+        }
+        node_slot_sum(slots, so, se, f);  // the mass term is already in f
+#pragma unroll
+        for (int d = 0; d < 3; ++d) r[d] += f[d];
+        if (held) {
+            const double xd[3] = {D.xp[oN + i] + D.dt * D.vg[k], D.yp[oN + i] + D.dt * D.vg[k + 1],
+                                  D.zp[oN + i] + D.dt * D.vg[k + 2]};
+            const double xj[3] = {D.xjx[i], D.xjy[i], D.xjz[i]};
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                for (int c = D.jt_off[3 * i + d]; c < D.jt_off[3 * i + d + 1]; ++c)
+                    r[d] += D.dt * (D.lam[(size_t)s * D.nc + D.jt_col[c]] + D.rho * (xd[d] - xj[d]));
+        }
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            D.g[k + d] = r[d];
+            if (!held) sg += r[d] * r[d];
+            gdy += r[d] * dv[d];
+            gg += r[d] * r[d];
+        }
+    }
+    if (D.restart) {
+        gdy = block_sum(gdy, red_sh);
+        gg = block_sum(gg, red_sh);
+    }
+    sg = block_sum(sg, red_sh);
+    if (threadIdx.x == 0) {
+        const size_t b = (size_t)s * D.blocks_per_seq + blockIdx.x;
+        D.red[b] = sg;
+        if (D.restart) {
+            D.red2[b] = gdy;
+            D.red2[(size_t)D.B * D.blocks_per_seq + b] = gg;
+        }
+        __threadfence();
+        last = atomicAdd(&D.ticket[s], 1u) == (unsigned int)gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (!last || threadIdx.x >= 32) return;
+    __threadfence();
+    double a = 0.0, a_dy = 0.0, a_gg = 0.0;
+    for (int bb = threadIdx.x; bb < (int)gridDim.x; bb += 32) {
+        const size_t b = (size_t)s * D.blocks_per_seq + bb;
+        a += __ldcg(D.red + b);
+        if (D.restart) {
+            a_dy += __ldcg(D.red2 + b);
+            a_gg += __ldcg(D.red2 + (size_t)D.B * D.blocks_per_seq + b);
+        }
+    }
+    a = warp_sum(a);
+    a_dy = warp_sum(a_dy);
+    a_gg = warp_sum(a_gg);
+    if (threadIdx.x == 0) dyn_end_iteration(D, s, a, a_dy, a_gg);
+}
+
+__global__ void __launch_bounds__(DYN_NODE_THREADS) k_dyn_update_straight(DynArgs D) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int s = blockIdx.y;
+    const int st = __ldcg(D.done + s);
+    if (st == DYN_RULE_MET || st == DYN_FINISHED) return;
+    const bool predict = (st == DYN_RUNNING);
+    const double beta = predict ? D.beta[__ldcg(D.mom + s)] : 0.0;
+    const double alpha = D.alpha_s[s];
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= D.N) return;
+    const size_t o = (size_t)s * D.N + i, k = 3 * o;
+    double y[3], vk[3], g[3], vp[3];
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        y[d] = D.vg[k + d];
+        vk[d] = D.vk[k + d];
+        g[d] = D.g[k + d];
+        vp[d] = D.vp[k + d];
+    }
+    const double xp[3] = {D.xp[o], D.yp[o], D.zp[o]};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double vn = y[d] - alpha * g[d];
+        y[d] = predict ? vn + beta * (vn - vk[d]) : vn;
+        vk[d] = vn;
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        D.vk[k + d] = vk[d];
+        D.vg[k + d] = y[d];
+    }
+    if (predict) dyn_record(D, o, xp, vp, y);
 }
 
 // v_next = y - alpha g; then the next look-ahead y' = v_next + beta_k (v_next - v_k) and
@@ -406,6 +571,9 @@ struct tlfea_dynbatch_s {
     int* outer_done = nullptr;
     int* mom = nullptr;       // momentum index per sequence (restart)
     double* red2 = nullptr;   // restart test partials
+    bool straight = false;    // the mesh qualifies and is undamped
+    double *x4 = nullptr, *w4 = nullptr, *slots = nullptr;
+    int force_blocks = 0, group = 1;
     double *rel = nullptr, *red = nullptr, *beta = nullptr, *fext_norm = nullptr;
     unsigned int *ticket = nullptr, *ticket2 = nullptr;
     int* counters = nullptr;    // [n_done]
@@ -421,6 +589,7 @@ struct tlfea_dynbatch_s {
     bool params_set = false;
     int chunk = 8;
     cudaGraphExec_t graph = nullptr;
+    bool graph_straight = false;  // the force kernel of the captured graph
     int beta_n = -1;
 };
 
@@ -481,8 +650,82 @@ int enqueue_force(tlfea_dynbatch_s* b, cudaStream_t stream) {
     return TLFEA_OK;
 }
 
+// Whether the straight-sided kernels run: decided when the graph is built and each step starts
+// (the damping may change between steps).
+bool use_straight(const tlfea_dynbatch_s* b) {
+    return b->straight && b->el->tl.straight && b->el->eta_d == 0.0 && b->el->lambda_d == 0.0;
+}
+
+template <typename... P, typename... Q>
+int launch_next(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, Q... args) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, args...);
+    if (e != cudaSuccess) {
+        set_error(std::string("batched dynamics launch: ") + cudaGetErrorString(e));
+        return TLFEA_CUDA_ERROR;
+    }
+    return TLFEA_OK;
+}
+
+template <int NPE>
+size_t straight_smem(const tlfea_element_s* el) {
+    return SForceLayout<double, NPE>(el->tl.max_local_pad, true).total;
+}
+
+template <int NPE>
+int enqueue_straight(tlfea_dynbatch_s* b, cudaStream_t stream) {
+    tlfea_element_s* el = b->el;
+    SeqForceArgs<double> A{};
+    A.T = sforce_tables<double>(el, true);
+    A.x = b->x4;
+    A.w = b->w4;
+    A.slots = b->slots;
+    A.n_seq = b->B;
+    A.group = b->group;
+    A.node_stride = el->N;
+    A.slot_stride = el->tl.n_local_total;
+    A.lam_s = b->lam_s;
+    A.mu_s = b->mu_s;
+    A.rule = svk_rule(el);
+    int st = launch_next(k_dyn_force_straight<NPE>, dim3((unsigned)b->force_blocks), TILE_ELEMS, straight_smem<NPE>(el),
+                         stream, b->D, A);
+    if (!st)
+        st = launch_next(k_dyn_grad_straight, dim3((unsigned)b->D.grad_blocks, (unsigned)b->B), DYN_NODE_THREADS, 0,
+                         stream, b->D);
+    if (!st)
+        st = launch_next(k_dyn_update_straight, dim3((unsigned)b->D.blocks_per_seq, (unsigned)b->B), DYN_NODE_THREADS, 0,
+                         stream, b->D);
+    return st;
+}
+
+// The resident grid of the force kernel and how many sequences share a pass of a tile's
+// tables: as many as leave each block about eight items (the last round is then a small part).
+template <int NPE>
+int prepare_straight(tlfea_dynbatch_s* b) {
+    int per_sm = 0, sms = 0;
+    TLFEA_CUDA(allow_tile_smem((const void*)k_dyn_force_straight<NPE>));
+    TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dyn_force_straight<NPE>, TILE_ELEMS,
+                                                             straight_smem<NPE>(b->el)));
+    TLFEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device));
+    const long long units = (long long)b->el->tl.n_tiles * b->B, blocks = std::max(1, per_sm * sms);
+    b->group = (int)std::max(1LL, std::min<long long>(std::min(b->B, 8), units / (8 * blocks)));
+    const long long items = (long long)b->el->tl.n_tiles * ((b->B + b->group - 1) / b->group);
+    b->force_blocks = (int)std::min(blocks, items);
+    return TLFEA_OK;
+}
+
 int enqueue_iteration(tlfea_dynbatch_s* b, cudaStream_t stream) {
     tlfea_element_s* el = b->el;
+    if (use_straight(b)) return el->npe == 10 ? enqueue_straight<10>(b, stream) : enqueue_straight<4>(b, stream);
     const bool damp = (el->eta_d != 0.0 || el->lambda_d != 0.0);
     int st;
     if (el->npe == 10)
@@ -501,8 +744,19 @@ int enqueue_iteration(tlfea_dynbatch_s* b, cudaStream_t stream) {
 // A CUDA graph of `chunk` inner iterations, built on first use after the parameters last
 // changed (the kernels' arguments are baked into it).
 int ensure_graph(tlfea_dynbatch_s* b) {
+    const bool straight = use_straight(b);
+    if (b->graph && b->graph_straight != straight) {
+        cudaGraphExecDestroy(b->graph);
+        b->graph = nullptr;
+    }
+    b->graph_straight = straight;
+    b->D.mass_scale = b->el->rho / b->np.time_step;
     if (b->graph) return TLFEA_OK;
     cudaStream_t stream = b->el->stream;
+    if (straight) {
+        const int rc = b->el->npe == 10 ? prepare_straight<10>(b) : prepare_straight<4>(b);
+        if (rc) return rc;
+    }
     const bool damp = (b->el->eta_d != 0.0 || b->el->lambda_d != 0.0);
     int st;
     if (b->el->npe == 10)
@@ -565,6 +819,7 @@ void dyn_free(tlfea_dynbatch_s* b) {
     dfree(b->done); dfree(b->inner); dfree(b->inner_total); dfree(b->rule_met); dfree(b->status);
     dfree(b->outer_done); dfree(b->rel); dfree(b->red); dfree(b->beta); dfree(b->fext_norm);
     dfree(b->mom); dfree(b->red2);
+    dfree(b->x4); dfree(b->w4); dfree(b->slots);
     dfree(b->ticket); dfree(b->ticket2); dfree(b->counters); dfree(b->node_fixed);
     dfree(b->f_base); dfree(b->f_var); dfree(b->zero_off);
     if (b->h_counters) cudaFreeHost(b->h_counters);
@@ -624,6 +879,11 @@ int tlfea_dynbatch_create(tlfea_element mesh, int n_seq, tlfea_dynbatch* out) {
     st |= dalloc(&b->ticket, B) | dalloc(&b->ticket2, B) | dalloc(&b->counters, 1);
     st |= dalloc(&b->node_fixed, N) | dalloc(&b->f_base, n3) | dalloc(&b->f_var, n3);
     if (el->n_constraint == 0) st |= dalloc(&b->zero_off, n3 + 1);
+    const size_t straight_need = el->npe == 10 ? straight_smem<10>(el) : straight_smem<4>(el);
+    b->straight = el->tl.straight && straight_need <= 200 * 1024;
+    if (b->straight)
+        st |= dalloc(&b->x4, 4 * B * N) | dalloc(&b->w4, 4 * B * N) |
+              dalloc(&b->slots, 4 * B * (size_t)el->tl.n_local_total);
     if (!st && cudaMallocHost((void**)&b->h_counters, sizeof(int)) != cudaSuccess) st = TLFEA_CUDA_ERROR;
     if (st) {
         dyn_free(b);
@@ -673,6 +933,12 @@ int tlfea_dynbatch_create(tlfea_element mesh, int n_seq, tlfea_dynbatch* out) {
     D.mom = b->mom;
     D.red2 = b->red2;
     D.restart = 0;
+    D.x4 = b->x4;
+    D.w4 = b->w4;
+    D.slots = b->slots;
+    D.node_soff = el->tl.node_soff;
+    D.n_slots = el->tl.n_local_total;
+    D.grad_blocks = (bps + DYN_GRAD_NODES - 1) / DYN_GRAD_NODES;
     cudaMemsetAsync(b->mom, 0, B * sizeof(int), stream);
     const dim3 grid(bps, n_seq);
     k_dyn_reset_state<<<grid, DYN_NODE_THREADS, 0, stream>>>(D, b->vhist, el->X0x, el->X0y, el->X0z);
@@ -820,7 +1086,10 @@ int tlfea_dynbatch_step(tlfea_dynbatch b, int warm_start, const double* d_v_gues
     for (int outer = 0; outer < b->np.max_outer; ++outer) {
         k_dyn_outer_ctl<<<1, 1024, 0, stream>>>(b->D, b->outer_done);
         TLFEA_CHECK_LAUNCH();
-        k_dyn_start<<<grid, DYN_NODE_THREADS, 0, stream>>>(b->D);
+        if (b->graph_straight)
+            k_dyn_start_straight<<<grid, DYN_NODE_THREADS, 0, stream>>>(b->D);
+        else
+            k_dyn_start<<<grid, DYN_NODE_THREADS, 0, stream>>>(b->D);
         TLFEA_CHECK_LAUNCH();
         for (int run = 0; run < b->np.max_inner; run += b->chunk) {
             TLFEA_CUDA(cudaGraphLaunch(b->graph, stream));
