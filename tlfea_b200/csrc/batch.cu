@@ -980,6 +980,14 @@ static BatchArgs<R> batch_args(tlfea_batch_s* b) {
 template <typename R>
 static size_t general_smem(const tlfea_batch_s* b);
 
+// Instances that share a pass of a tile's tables (shared mesh): up to eight, as long as every
+// resident block (about 600) still gets some four passes; a small batch gives each block one.
+static int blin_group(const tlfea_batch_s* b) {
+    if (!b->shared) return 1;
+    const long long units = (long long)b->el->tl.n_tiles * b->n_inst;
+    return (int)std::max(1LL, std::min<long long>(std::min(b->n_inst, 8), units / 2400));
+}
+
 template <typename R>
 static BLinArgs<R> blin_args(tlfea_batch_s* b) {
     tlfea_element_s* el = b->el;
@@ -1005,6 +1013,7 @@ static BLinArgs<R> blin_args(tlfea_batch_s* b) {
     }
     A.n_tiles = tl.n_tiles;
     A.max_local = tl.max_local_pad;
+    A.group = blin_group(b);
     A.nodes_per_inst = b->shared ? el->N : 0;
     A.slots_per_inst = b->shared ? (int)tl.n_local_total : 0;
     A.N = b->N;
@@ -1267,7 +1276,8 @@ static int blin_tile_grid(const tlfea_batch_s* b, int* grid) {
     int per_sm = 0, sms = 0;
     TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, tiles, TILE_ELEMS, blin_smem<R, NPE>(b)));
     TLFEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->el->device));
-    const long long items = (long long)b->el->tl.n_tiles * (SH ? (b->n_inst + BL_GROUP - 1) / BL_GROUP : 1);
+    const int group = blin_group(b);
+    const long long items = (long long)b->el->tl.n_tiles * (SH ? (b->n_inst + group - 1) / group : 1);
     *grid = (int)std::max(1LL, std::min<long long>(items, (long long)per_sm * sms));
     return TLFEA_OK;
 }
@@ -1300,7 +1310,7 @@ static int blin_phased(tlfea_batch_s* b, double tol, int max_iter, bool warm, cu
         const int rc = blin_tile_grid<R, NPE, SH>(b, &tile_grid);
         if (rc) return rc;
     }
-    const int chunk_grid = (b->n_chunks + TILE_ELEMS / 32 - 1) / (TILE_ELEMS / 32);  // one warp per chunk
+    const int chunk_grid = b->n_chunks;  // one block per chunk
     int* base = b->n_done + 1;
     TLFEA_CUDA(cudaMemsetAsync(b->n_done, 0, 2 * sizeof(int), st));
     k_bl_start<R><<<chunk_grid, TILE_ELEMS, 0, st>>>(A, w);

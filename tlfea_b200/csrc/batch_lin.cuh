@@ -9,7 +9,8 @@
 //               r -= alpha q per node chunk, r.r per chunk;
 //   direction   r.r folded the same way, the stop test, u += alpha p, p = r + beta p.
 //
-// One warp per node chunk in the last two; the warp of an instance's first chunk writes its
+// One block per node chunk in the last two (a warp per chunk left 7 warps per SM on 48 beams of
+// 260,000 nodes: 27 us for the update); the first chunk of an instance writes its
 // scalars.  An instance that ends in iteration it is stamped it + 1 and counts as done from the
 // next one, so the warps of one phase agree whatever their order.
 #pragma once
@@ -35,6 +36,7 @@ struct BLinArgs {
     const R* lam;  // per element slot; shared mesh: per instance
     const R* mu;
     int n_tiles, max_local;
+    int group;  // shared mesh: instances per pass of a tile's tables
     // shared mesh: nodes and node slots per instance (0 otherwise)
     int nodes_per_inst, slots_per_inst;
     int N, n_inst, n_chunks;
@@ -58,30 +60,32 @@ struct BLinArgs {
     int* err;
 };
 
-// Shared memory: [element forces][p][tables twice][barriers].
+// Shared memory: [element forces][p][local connectivity][the scatter's tables twice][barriers: the
+// tables', the connectivity's].  The connectivity is read before the scatter starts, so one copy
+// is refilled meanwhile; the fourth block per SM needs the room.
 template <typename R, int NPE>
 struct BLinLayout {
-    size_t p, tab, inc, lconn, slot, iend, tab_bytes, bar, total;
+    size_t p, lconn, tab, inc, slot, iend, tab_bytes, bar, total;
     __host__ __device__ explicit BLinLayout(int ml) {
         auto al = [](size_t v) { return (v + 15) & ~size_t(15); };
         p = al(3 * (size_t)NPE * TILE_ELEMS * sizeof(R));
-        tab = al(p + 3 * (size_t)ml * sizeof(double));
+        lconn = al(p + 3 * (size_t)ml * sizeof(double));
+        tab = lconn + NPE * TILE_ELEMS * sizeof(uint16_t);
         inc = 0;
-        lconn = inc + NPE * TILE_ELEMS * sizeof(uint16_t);
-        slot = lconn + NPE * TILE_ELEMS * sizeof(uint16_t);
+        slot = inc + NPE * TILE_ELEMS * sizeof(uint16_t);
         iend = slot + (size_t)ml * sizeof(int);
         tab_bytes = al(iend + (size_t)ml * sizeof(uint16_t));
         bar = tab + 2 * tab_bytes;
-        total = bar + 16;
+        total = bar + 24;
     }
 };
 
-constexpr int BL_GROUP = 8;  // instances per pass of a shared tile's tables
 
 __device__ __forceinline__ void bl_init_barriers(uint32_t bar) {
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         mbar_init(bar + 8, 1);
+        mbar_init(bar + 16, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
@@ -101,14 +105,14 @@ __device__ __forceinline__ void bl_tiles(const BLinArgs<R>& A, int it, bool skip
     R* fe = reinterpret_cast<R*>(smem);
     double* ps = reinterpret_cast<double*>(smem + L.p);
     const uint32_t bar0 = smem_u32(smem + L.bar);
-    const int groups = SH ? (A.n_inst + BL_GROUP - 1) / BL_GROUP : 1;
+    const int groups = SH ? (A.n_inst + A.group - 1) / A.group : 1;
     const int n_items = A.n_tiles * groups;
     auto running = [&](int b) { return !skip || __ldcg(A.stamp + b) > it; };
     // the first unit at or after (item, inst); item = n_items: none
     auto seek = [&](int& item, int& inst) {
         for (; item < n_items; item += gridDim.x) {
             if constexpr (SH) {
-                const int g0 = (item / A.n_tiles) * BL_GROUP, g1 = min(g0 + BL_GROUP, A.n_inst);
+                const int g0 = (item / A.n_tiles) * A.group, g1 = min(g0 + A.group, A.n_inst);
                 for (inst = max(inst, g0); inst < g1; ++inst)
                     if (running(inst)) return;
                 inst = 0;
@@ -125,11 +129,15 @@ __device__ __forceinline__ void bl_tiles(const BLinArgs<R>& A, int it, bool skip
         unsigned char* tab = smem + L.tab + (load & 1) * L.tab_bytes;
         const int pb = A.pad_off[tile];
         const uint32_t np = (uint32_t)(A.pad_off[tile + 1] - pb);
-        mbar_expect_tx(bar, 2 * TAB + np * (sizeof(int) + sizeof(uint16_t)));
+        mbar_expect_tx(bar, TAB + np * (sizeof(int) + sizeof(uint16_t)));
         bulk_g2s(smem_u32(tab + L.inc), A.inc + (size_t)tile * NPE * TE, TAB, bar);
-        bulk_g2s(smem_u32(tab + L.lconn), A.lconn + (size_t)tile * NPE * TE, TAB, bar);
         bulk_g2s(smem_u32(tab + L.slot), A.pad_slot + pb, np * sizeof(int), bar);
         bulk_g2s(smem_u32(tab + L.iend), A.pad_iend + pb, np * sizeof(uint16_t), bar);
+    };
+    auto issue_lconn = [&](int tile) {  // thread 0
+        constexpr uint32_t TAB = NPE * TE * sizeof(uint16_t);
+        mbar_expect_tx(bar0 + 16, TAB);
+        bulk_g2s(smem_u32(smem + L.lconn), A.lconn + (size_t)tile * NPE * TE, TAB, bar0 + 16);
     };
     R ji[9], det, lam, mu;
     double pv[NB][3];
@@ -157,16 +165,20 @@ __device__ __forceinline__ void bl_tiles(const BLinArgs<R>& A, int it, bool skip
     if (item >= n_items) return;
     int tile = item % A.n_tiles;
     int nl = A.node_off[tile + 1] - A.node_off[tile];
-    if (t == 0) issue(tile, loads);
+    if (t == 0) {
+        issue(tile, loads);
+        issue_lconn(tile);
+    }
     geometry(tile);
     gather(tile, inst, nl);
     bool fresh = true;  // this unit's tables are still on their way
     while (item < n_items) {
         const int load = loads;
-        if (fresh && !mbar_wait(bar0 + 8 * (load & 1), (load >> 1) & 1)) atomicExch(A.err, 3);
+        if (fresh && !(mbar_wait(bar0 + 8 * (load & 1), (load >> 1) & 1) && mbar_wait(bar0 + 16, load & 1)))
+            atomicExch(A.err, 3);
         const unsigned char* tab = smem + L.tab + (load & 1) * L.tab_bytes;
         const uint16_t* incs = reinterpret_cast<const uint16_t*>(tab + L.inc);
-        const uint16_t* lcs = reinterpret_cast<const uint16_t*>(tab + L.lconn);
+        const uint16_t* lcs = reinterpret_cast<const uint16_t*>(smem + L.lconn);
         const int* slot = reinterpret_cast<const int*>(tab + L.slot);
         const uint16_t* iends = reinterpret_cast<const uint16_t*>(tab + L.iend);
         if constexpr (SH) {
@@ -210,7 +222,9 @@ __device__ __forceinline__ void bl_tiles(const BLinArgs<R>& A, int it, bool skip
             }
             gather(tile2, inst2, nl);
         }
+        if (swap) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // reads of lconn before its refill
         __syncthreads();  // element forces complete
+        if (swap && t == 0) issue_lconn(tile2);
         double dot = 0.0;
         double* slots = A.slots + (SH ? 4 * (size_t)inst * A.slots_per_inst : 0);
         const int lo = SH ? inst : A.tile_inst[2 * tile], hi = SH ? inst : A.tile_inst[2 * tile + 1];
@@ -274,20 +288,23 @@ __device__ __forceinline__ double bl_fold(const double* v, int b, int e) {
     return warp_sum(s);
 }
 
-// One warp per chunk, over all chunks.
-template <typename F>
-__device__ __forceinline__ void bl_chunks(int n_chunks, F f) {
-    const int warps = blockDim.x / 32;
-    for (int c = blockIdx.x * warps + (threadIdx.x >> 5); c < n_chunks; c += gridDim.x * warps) f(c);
+// Sum over the block (warps in order), in thread 0; called by all its threads.
+__device__ __forceinline__ double bl_block_sum(double v) {
+    __shared__ double red[TILE_ELEMS / 32];
+    v = warp_sum(v);
+    __syncthreads();  // red free
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return (red[0] + red[1]) + (red[2] + red[3]);
 }
 
 // u = p = u0 (warm) or 0, r = f_free; ||f_free||^2 per chunk.
 template <typename R>
 __device__ __forceinline__ void bl_start(const BLinArgs<R>& A, int warm) {
-    const int lane = threadIdx.x & 31;
-    bl_chunks(A.n_chunks, [&](int c) {
+    const int t = threadIdx.x;
+    for (int c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
         double s = 0.0;
-        for (int i = A.chunk_beg[c] + lane; i < A.chunk_beg[c + 1]; i += 32) {
+        for (int i = A.chunk_beg[c] + t; i < A.chunk_beg[c + 1]; i += TILE_ELEMS) {
             const bool fx = A.fixed[i];
             double uv[3];
 #pragma unroll
@@ -301,19 +318,19 @@ __device__ __forceinline__ void bl_start(const BLinArgs<R>& A, int warm) {
             }
             st_node(A.p + 4 * (size_t)i, uv[0], uv[1], uv[2]);
         }
-        s = warp_sum(s);
-        if (lane == 0) A.cpa[c] = s;
-    });
+        s = bl_block_sum(s);
+        if (t == 0) A.cpa[c] = s;
+    }
 }
 
 // r -= K u0 (warm), p = r; ||r||^2 per chunk.
 template <typename R>
 __device__ __forceinline__ void bl_residual(const BLinArgs<R>& A, int warm) {
-    const int lane = threadIdx.x & 31;
-    bl_chunks(A.n_chunks, [&](int c) {
+    const int t = threadIdx.x;
+    for (int c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
         const int b = A.chunk_inst[c];
         double s = 0.0;
-        for (int i = A.chunk_beg[c] + lane; i < A.chunk_beg[c + 1]; i += 32) {
+        for (int i = A.chunk_beg[c] + t; i < A.chunk_beg[c + 1]; i += TILE_ELEMS) {
             double q[3] = {0.0, 0.0, 0.0}, rv[3];
             if (warm && !A.fixed[i]) bl_node_sum(A, i, b, q);
 #pragma unroll
@@ -324,9 +341,9 @@ __device__ __forceinline__ void bl_residual(const BLinArgs<R>& A, int warm) {
             }
             st_node(A.p + 4 * (size_t)i, rv[0], rv[1], rv[2]);
         }
-        s = warp_sum(s);
-        if (lane == 0) A.cpb[c] = s;
-    });
+        s = bl_block_sum(s);
+        if (t == 0) A.cpb[c] = s;
+    }
 }
 
 // Per instance, one warp each: ||f_free||, rr_0, the initial relative residual and state.
@@ -354,12 +371,12 @@ __device__ __forceinline__ void bl_init(const BLinArgs<R>& A, double tol) {
 // alpha, r -= alpha q, r.r per chunk.
 template <typename R>
 __device__ __forceinline__ void bl_update(const BLinArgs<R>& A, int it) {
-    const int lane = threadIdx.x & 31;
+    const int t = threadIdx.x;
     const double* rr_old = A.rr + (size_t)(it & 1) * A.n_inst;
-    bl_chunks(A.n_chunks, [&](int c) {
+    for (int c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
         const int b = A.chunk_inst[c];
-        if (__ldcg(A.stamp + b) <= it) return;
-        const bool first = lane == 0 && c == A.inst_chunk[b];
+        if (__ldcg(A.stamp + b) <= it) continue;  // uniform over the block, as every branch on b
+        const bool first = t == 0 && c == A.inst_chunk[b];
         const double pq = bl_fold(A.pair, A.inst_pair[b], A.inst_pair[b + 1]);
         if (!(pq > 0.0)) {  // non-positive p.Kp: the reference aborts this solve
             if (first) {
@@ -368,54 +385,54 @@ __device__ __forceinline__ void bl_update(const BLinArgs<R>& A, int it) {
                 A.stamp[b] = it + 1;
                 atomicAdd(A.n_done, 1);
             }
-            return;
+            continue;
         }
         const double alpha = __ldcg(rr_old + b) / pq;
         if (first) A.alpha[b] = alpha;
         const int i_end = A.chunk_beg[c + 1];
         double s = 0.0;
-        for (int i0 = A.chunk_beg[c] + lane; i0 < i_end; i0 += 64) {
+        for (int i0 = A.chunk_beg[c] + t; i0 < i_end; i0 += 2 * TILE_ELEMS) {
             double rv[2][3], q[2][3];
             bool ok[2];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const int i = min(i0 + 32 * j, i_end - 1);
-                ok[j] = i0 + 32 * j < i_end && !A.fixed[i];
+                const int i = min(i0 + TILE_ELEMS * j, i_end - 1);
+                ok[j] = i0 + TILE_ELEMS * j < i_end && !A.fixed[i];
 #pragma unroll
                 for (int d = 0; d < 3; ++d) rv[j][d] = __ldcg(A.r + 3 * (size_t)i + d);
             }
 #pragma unroll
-            for (int j = 0; j < 2; ++j) bl_node_sum(A, min(i0 + 32 * j, i_end - 1), b, q[j]);
+            for (int j = 0; j < 2; ++j) bl_node_sum(A, min(i0 + TILE_ELEMS * j, i_end - 1), b, q[j]);
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 if (!ok[j]) continue;
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
                     const double ri = rv[j][d] - alpha * q[j][d];
-                    A.r[3 * (size_t)(i0 + 32 * j) + d] = ri;
+                    A.r[3 * (size_t)(i0 + TILE_ELEMS * j) + d] = ri;
                     s += ri * ri;
                 }
             }
         }
-        s = warp_sum(s);
-        if (lane == 0) A.cpb[c] = s;
-    });
+        s = bl_block_sum(s);
+        if (t == 0) A.cpb[c] = s;
+    }
 }
 
 // The stop test and beta, u += alpha p, p = r + beta p.
 template <typename R>
 __device__ __forceinline__ void bl_direction(const BLinArgs<R>& A, int it, double tol, int max_iter) {
-    const int lane = threadIdx.x & 31;
+    const int t = threadIdx.x;
     const double* rr_old = A.rr + (size_t)(it & 1) * A.n_inst;
-    bl_chunks(A.n_chunks, [&](int c) {
+    for (int c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
         const int b = A.chunk_inst[c];
-        if (__ldcg(A.stamp + b) <= it || __ldcg(A.flag + b) == 2) return;
+        if (__ldcg(A.stamp + b) <= it || __ldcg(A.flag + b) == 2) continue;
         const double alpha = __ldcg(A.alpha + b);
         const double rrn = bl_fold(A.cpb, A.inst_chunk[b], A.inst_chunk[b + 1]);
         const double rel = sqrt(rrn) / __ldcg(A.fnorm + b);
         const bool conv = rel < tol;
         const double beta = rrn / __ldcg(rr_old + b);
-        if (lane == 0 && c == A.inst_chunk[b]) {
+        if (t == 0 && c == A.inst_chunk[b]) {
             A.rr[(size_t)((it + 1) & 1) * A.n_inst + b] = rrn;
             A.iters[b] = it + 1;
             A.rel[b] = rel;
@@ -427,11 +444,11 @@ __device__ __forceinline__ void bl_direction(const BLinArgs<R>& A, int it, doubl
             }
         }
         const int i_end = A.chunk_beg[c + 1];
-        for (int i0 = A.chunk_beg[c] + lane; i0 < i_end; i0 += 64) {
+        for (int i0 = A.chunk_beg[c] + t; i0 < i_end; i0 += 2 * TILE_ELEMS) {
             double rv[2][3], uv[2][3], pv[2][3];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {  // every load before the first store
-                const int i = min(i0 + 32 * j, i_end - 1);
+                const int i = min(i0 + TILE_ELEMS * j, i_end - 1);
                 ld_node_shared(A.p + 4 * (size_t)i, pv[j]);
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {
@@ -441,7 +458,7 @@ __device__ __forceinline__ void bl_direction(const BLinArgs<R>& A, int it, doubl
             }
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const int i = i0 + 32 * j;
+                const int i = i0 + TILE_ELEMS * j;
                 if (i >= i_end) continue;
 #pragma unroll
                 for (int d = 0; d < 3; ++d) A.u[3 * (size_t)i + d] = uv[j][d] + alpha * pv[j][d];
@@ -450,7 +467,7 @@ __device__ __forceinline__ void bl_direction(const BLinArgs<R>& A, int it, doubl
                             rv[j][2] + beta * pv[j][2]);
             }
         }
-    });
+    }
 }
 
 // Instances still running at the iteration cap end with status 2; the done flags.
