@@ -1089,13 +1089,11 @@ static int noalloc_scratch(int device, double** out) {
 
 // A kernel's bounded wait ran out: report it once and clear the word.
 static int check_device_error(tlfea_element_s* h) {
-    int e = 0;
-    if (cudaMemcpy(&e, h->d_err, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) {
-        set_error("reading the device error word failed");
-        return TLFEA_CUDA_ERROR;
-    }
+    // host memory that the kernels see (they write it only then): after the caller's
+    // synchronisation this is a plain read, where a copy back cost a force call 8 us
+    const int e = *static_cast<volatile int*>(h->h_err);
     if (e) {
-        cudaMemset(h->d_err, 0, sizeof(int));
+        *h->h_err = 0;
         set_error("a pipeline wait in the force kernel ran out (code " + std::to_string(e) + ")");
         return TLFEA_BUDGET_EXCEEDED;
     }
@@ -1208,7 +1206,13 @@ int tlfea_element_create(int type, int n_elem, int n_nodes, tlfea_element* out) 
     st |= dalloc(&h->d_conn, (size_t)n_elem * h->npe);
     st |= dalloc(&h->f_int, 3 * N) | dalloc(&h->f_ext, 3 * N) | dalloc(&h->f_int32, 3 * N);
     st |= dalloc(&h->detJ, (size_t)n_elem * h->nqp);
-    st |= dalloc(&h->d_err, 1);
+    if (cudaHostAlloc((void**)&h->h_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void**)&h->d_err, h->h_err, 0) != cudaSuccess) {
+        set_error("element_create: pinned error word");
+        st |= 1;
+    } else {
+        *h->h_err = 0;
+    }
     if (st) {
         tlfea_element_destroy(h);
         return TLFEA_CUDA_ERROR;
@@ -1217,7 +1221,6 @@ int tlfea_element_create(int type, int n_elem, int n_nodes, tlfea_element* out) 
     cudaMemsetAsync(h->f_ext, 0, 3 * N * sizeof(double), h->stream);
     cudaMemsetAsync(h->f_int32, 0, 3 * N * sizeof(float), h->stream);
     cudaMemsetAsync(h->detJ, 0, (size_t)n_elem * h->nqp * sizeof(double), h->stream);
-    cudaMemsetAsync(h->d_err, 0, sizeof(int), h->stream);
     cudaStreamSynchronize(h->stream);
     *out = h;
     return TLFEA_OK;
@@ -1230,7 +1233,9 @@ int tlfea_element_destroy(tlfea_element h) {
     dfree(h->xj); dfree(h->yj); dfree(h->zj);
     dfree(h->X0x); dfree(h->X0y); dfree(h->X0z); dfree(h->u64);
     dfree(h->d_conn); dfree(h->f_int); dfree(h->f_ext); dfree(h->f_int32);
-    dfree(h->detJ); dfree(h->Pst); dfree(h->d_err);
+    dfree(h->detJ); dfree(h->Pst);
+    if (h->h_err) cudaFreeHost(h->h_err);
+    h->h_err = h->d_err = nullptr;
     free_tiling(h->tl);
     dfree(h->inc_off); dfree(h->inc_e); dfree(h->inc_a);
     dfree(h->pat_off); dfree(h->pat_col); dfree(h->m_val);

@@ -955,7 +955,8 @@ struct tlfea_element_s {
     double* j_val = nullptr;
 
     // error word set by kernels whose bounded waits ran out (checked at sync points)
-    int* d_err = nullptr;
+    int* h_err = nullptr;  // pinned
+    int* d_err = nullptr;  // the same word as the kernels see it
     // grid of the persistent force pipeline per (FP32?, damping?), 0 = not yet sized
     int pipe_grid[4] = {0, 0, 0, 0};
     int straight_grid[4] = {0, 0, 0, 0};  // the same of the straight-sided force kernel
