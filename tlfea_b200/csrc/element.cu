@@ -5,8 +5,8 @@
 #include <cstring>
 #include <fstream>
 #include <mutex>
+#include <mutex>
 #include <numeric>
-#include <tuple>
 #include <vector>
 
 #include "element.cuh"
@@ -407,6 +407,27 @@ static int upload(T** d, const std::vector<T>& v, cudaStream_t stream) {
     return TLFEA_OK;
 }
 
+// Stable sort of `order` by the low `bits` bits of key(element): radix passes of 11 bits (480k
+// elements of 63-bit codes in 15 ms, where std::sort of (group, code, element) took 70).
+template <typename Key>
+static void radix_order(std::vector<int>& order, int bits, Key key) {
+    constexpr int RADIX = 11, BINS = 1 << RADIX;
+    std::vector<int> other(order.size());
+    for (int shift = 0; shift < bits; shift += RADIX) {
+        int at[BINS] = {0};
+        for (int e : order) at[(key(e) >> shift) & (BINS - 1)]++;
+        if (order.empty() || at[(key(order[0]) >> shift) & (BINS - 1)] == (int)order.size()) continue;
+        int run = 0;
+        for (int b = 0; b < BINS; ++b) {
+            const int n = at[b];
+            at[b] = run;
+            run += n;
+        }
+        for (int e : order) other[at[(key(e) >> shift) & (BINS - 1)]++] = e;
+        order.swap(other);
+    }
+}
+
 // Host-side construction of the tiles (see element.cuh for the layout).
 static int build_tiling(tlfea_element_s* h, const double* x, const double* y, const double* z) {
     Tiling& tl = h->tl;
@@ -424,9 +445,8 @@ static int build_tiling(tlfea_element_s* h, const double* x, const double* y, co
     }
     double ext = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
     if (!(ext > 0.0)) ext = 1.0;
-    // (group, Morton code, element): a batch of meshes sorts instance by instance
-    std::vector<std::tuple<int, unsigned long long, int>> key((size_t)E);
     const bool grouped = h->elem_group.size() == (size_t)E;
+    std::vector<unsigned long long> code((size_t)E);
     for (int e = 0; e < E; ++e) {
         double c[3] = {0, 0, 0};
         for (int a = 0; a < 4; ++a) {
@@ -442,122 +462,98 @@ static int build_tiling(tlfea_element_s* h, const double* x, const double* y, co
             const unsigned long long qd = (unsigned long long)(u * 2097151.0);
             m |= spread3(qd) << d;
         }
-        key[e] = {grouped ? h->elem_group[e] : 0, m, e};
+        code[e] = m;
     }
-    std::sort(key.begin(), key.end());
+    // by (group, Morton code, element): a batch of meshes sorts instance by instance
+    std::vector<int> order((size_t)E);
+    std::iota(order.begin(), order.end(), 0);
+    radix_order(order, 63, [&](int e) { return code[e]; });
+    if (grouped) radix_order(order, 32, [&](int e) { return (unsigned long long)((unsigned)h->elem_group[e] ^ 0x80000000u); });
 
     // 2. Tiles.
     const int n_tiles = (E + TE - 1) / TE;
     tl.n_tiles = n_tiles;
     std::vector<int> tile_elem((size_t)n_tiles * TE, -1);
-    for (int s = 0; s < E; ++s) tile_elem[s] = std::get<2>(key[s]);
-
-    std::vector<int> total_inc((size_t)N, 0);
-    for (size_t k = 0; k < conn.size(); ++k) total_inc[conn[k]]++;
-    int orphans = 0;
-    for (int i = 0; i < N; ++i) orphans += (total_inc[i] == 0);
-    tl.n_orphans = orphans;
+    std::copy(order.begin(), order.end(), tile_elem.begin());
 
     std::vector<int> node_off((size_t)n_tiles + 1, 0);
     std::vector<int> ln_gid, ln_pslot;
     std::vector<uint16_t> ln_inc_end;
     std::vector<uint16_t> inc((size_t)n_tiles * TE * npe, 0);
     std::vector<uint16_t> lconn((size_t)n_tiles * npe * TE, 0);
-    std::vector<int> stamp((size_t)N, -1), lidx((size_t)N, 0), in_tile((size_t)N, 0);
-    std::vector<std::vector<int>> node_slots;  // per boundary gid: pslots (tile order)
-    std::vector<int> gid_to_b((size_t)N, -1);
-    std::vector<int> bnode_gid;
-    int n_pslots = 0, max_local = 0;
-    std::vector<int> nodes, cnt, pos;
+    struct Seen {
+        int tile, at;
+    };
+    std::vector<Seen> seen((size_t)N, Seen{-1, 0});  // per node: last tile and its place there
+    std::vector<int> soff((size_t)N + 1, 0);         // tiles of a node, counted here, then offsets
+    ln_gid.reserve((size_t)n_tiles * TE * (npe == 10 ? 4 : 1));
+    ln_inc_end.reserve(ln_gid.capacity());
+    int max_local = 0;
+    std::vector<int> at((size_t)TE * npe), gid((size_t)TE * npe), count((size_t)TE * npe), place((size_t)TE * npe),
+        pos((size_t)TE * npe);
+    std::vector<unsigned long long> sorted;
     for (int tile = 0; tile < n_tiles; ++tile) {
-        nodes.clear();
-        for (int t = 0; t < TE; ++t) {
+        const int elems = std::min(TE, E - tile * TE);
+        int nl = 0;
+        for (int t = 0; t < elems; ++t) {
             const int e = tile_elem[(size_t)tile * TE + t];
-            if (e < 0) continue;
             for (int a = 0; a < npe; ++a) {
                 const int n = conn[e + (size_t)a * E];
-                if (stamp[n] != tile) {
-                    stamp[n] = tile;
-                    in_tile[n] = 0;
-                    nodes.push_back(n);
+                if (seen[n].tile != tile) {
+                    seen[n] = Seen{tile, nl};
+                    gid[nl] = n;
+                    count[nl++] = 0;
                 }
-                in_tile[n]++;
+                at[(size_t)t * npe + a] = seen[n].at;
+                count[seen[n].at]++;
             }
         }
         // local nodes by the number of the tile's elements that touch them, most first, then by
         // node id: the scatter's loop over a node's elements is as long as the longest in its
         // warp, so nodes of like counts sit side by side
-        std::sort(nodes.begin(), nodes.end(), [&](int a, int b) {
-            return in_tile[a] != in_tile[b] ? in_tile[a] > in_tile[b] : a < b;
-        });
-        const int nl = (int)nodes.size();
+        sorted.resize((size_t)nl);
+        for (int k = 0; k < nl; ++k)
+            sorted[k] = (unsigned long long)(4095 - count[k]) << 43 | (unsigned long long)gid[k] << 12 | (unsigned)k;
+        std::sort(sorted.begin(), sorted.end());
         max_local = std::max(max_local, nl);
-        for (int l = 0; l < nl; ++l) lidx[nodes[l]] = l;
-        cnt.assign((size_t)nl, 0);
-        for (int t = 0; t < TE; ++t) {
-            const int e = tile_elem[(size_t)tile * TE + t];
-            for (int a = 0; a < npe; ++a) {
-                int l = 0;
-                if (e >= 0) {
-                    l = lidx[conn[e + (size_t)a * E]];
-                    cnt[l]++;
-                }
-                lconn[((size_t)tile * npe + a) * TE + t] = (uint16_t)l;
-            }
-        }
-        pos.assign((size_t)nl, 0);
         int run = 0;
         for (int l = 0; l < nl; ++l) {
+            const int k = (int)(sorted[l] & 4095);
+            place[k] = l;
             pos[l] = run;
-            run += cnt[l];
+            run += count[k];
             ln_inc_end.push_back((uint16_t)run);
+            ln_gid.push_back(gid[k]);
+            soff[(size_t)gid[k] + 1]++;
         }
-        for (int t = 0; t < TE; ++t) {
-            const int e = tile_elem[(size_t)tile * TE + t];
-            if (e < 0) continue;
+        for (int t = 0; t < elems; ++t)
             for (int a = 0; a < npe; ++a) {
-                const int l = lidx[conn[e + (size_t)a * E]];
+                const int l = place[at[(size_t)t * npe + a]];
+                lconn[((size_t)tile * npe + a) * TE + t] = (uint16_t)l;
                 inc[(size_t)tile * TE * npe + pos[l]++] = (uint16_t)((a << TILE_SHIFT) | t);
             }
-        }
-        for (int l = 0; l < nl; ++l) {
-            const int g = nodes[l];
-            ln_gid.push_back(g);
-            if (cnt[l] == total_inc[g]) {
-                ln_pslot.push_back(-1);
-            } else {
-                const int ps = n_pslots++;
-                ln_pslot.push_back(ps);
-                if (gid_to_b[g] < 0) {
-                    gid_to_b[g] = (int)bnode_gid.size();
-                    bnode_gid.push_back(g);
-                    node_slots.emplace_back();
-                }
-                node_slots[gid_to_b[g]].push_back(ps);
-            }
-        }
         node_off[tile + 1] = node_off[tile] + nl;
     }
-    // boundary CSR, sorted by node id (slots stay in tile order)
-    std::vector<int> border(bnode_gid.size());
-    std::iota(border.begin(), border.end(), 0);
-    std::sort(border.begin(), border.end(), [&](int a, int b) { return bnode_gid[a] < bnode_gid[b]; });
-    std::vector<int> bgid, boff(1, 0), bslots, node_bidx((size_t)N, -1);
-    // Partial slots are renumbered by shared node (in node-id order), each node's
-    // slots in tile order: a node's partials are one contiguous range, so the
-    // combine streams them coalesced; the summation order is unchanged.
-    std::vector<int> renum((size_t)std::max(n_pslots, 1), -1);
-    for (int k : border) {
-        node_bidx[bnode_gid[k]] = (int)bgid.size();
-        bgid.push_back(bnode_gid[k]);
-        for (int ps : node_slots[k]) {
-            renum[ps] = (int)bslots.size();
-            bslots.push_back((int)bslots.size());
+    // Partial slots, for the nodes of more than one tile: numbered by node id, a node's slots in
+    // tile order, so that its partials are one contiguous range and the combine streams them.
+    int orphans = 0, n_pslots = 0;
+    std::vector<int> bgid, boff(1, 0), bslots, node_bidx((size_t)N, -1), next_slot((size_t)N, -1);
+    for (int i = 0; i < N; ++i) {
+        const int tiles = soff[(size_t)i + 1];
+        orphans += tiles == 0;
+        if (tiles > 1) {
+            node_bidx[i] = (int)bgid.size();
+            next_slot[i] = n_pslots;
+            n_pslots += tiles;
+            bgid.push_back(i);
+            boff.push_back(n_pslots);
         }
-        boff.push_back((int)bslots.size());
     }
-    for (int& ps : ln_pslot)
-        if (ps >= 0) ps = renum[ps];
+    tl.n_orphans = orphans;
+    bslots.resize((size_t)n_pslots);
+    std::iota(bslots.begin(), bslots.end(), 0);
+    ln_pslot.resize(ln_gid.size());
+    for (size_t k = 0; k < ln_gid.size(); ++k) ln_pslot[k] = next_slot[ln_gid[k]] < 0 ? -1 : next_slot[ln_gid[k]]++;
     tl.max_local = std::max(max_local, 1);
     tl.n_local_total = (long long)ln_gid.size();
     tl.n_pslots = n_pslots;
@@ -565,30 +561,24 @@ static int build_tiling(tlfea_element_s* h, const double* x, const double* y, co
     tl.h_tile_elem = tile_elem;
 
     // the tile-ordered node record, each tile's block padded to TILE_NODE_PAD entries
-    std::vector<int> pad_off((size_t)n_tiles + 1, 0), pad_gid, pad_dst;
-    std::vector<uint16_t> pad_iend;
+    std::vector<int> pad_off((size_t)n_tiles + 1, 0);
     int max_pad = 0;
     for (int tile = 0; tile < n_tiles; ++tile) {
-        const int b = node_off[tile], nl = node_off[tile + 1] - b;
+        const int nl = node_off[tile + 1] - node_off[tile];
         const int np = (nl + TILE_NODE_PAD - 1) / TILE_NODE_PAD * TILE_NODE_PAD;
         max_pad = std::max(max_pad, np);
-        for (int l = 0; l < np; ++l) {
-            if (l < nl) {
-                const int g = ln_gid[(size_t)b + l], ps = ln_pslot[(size_t)b + l];
-                pad_gid.push_back(g);
-                pad_dst.push_back(ps < 0 ? g : -(ps + 1));
-                pad_iend.push_back(ln_inc_end[(size_t)b + l]);
-            } else {
-                pad_gid.push_back(-1);
-                pad_dst.push_back(0);
-                pad_iend.push_back(0);
-            }
-        }
         pad_off[tile + 1] = pad_off[tile] + np;
     }
-    // node slots: counted per node, then handed out in tile order
-    std::vector<int> soff((size_t)N + 1, 0), pad_slot(pad_gid.size(), -1);
-    for (int g : ln_gid) soff[(size_t)g + 1]++;
+    std::vector<int> pad_gid((size_t)pad_off[n_tiles], -1), pad_dst((size_t)pad_off[n_tiles], 0);
+    std::vector<uint16_t> pad_iend((size_t)pad_off[n_tiles], 0);
+    for (int tile = 0; tile < n_tiles; ++tile)
+        for (int k = node_off[tile], o = pad_off[tile]; k < node_off[tile + 1]; ++k, ++o) {
+            pad_gid[o] = ln_gid[k];
+            pad_dst[o] = ln_pslot[k] < 0 ? ln_gid[k] : -(ln_pslot[k] + 1);
+            pad_iend[o] = ln_inc_end[k];
+        }
+    // node slots: counted per node above, handed out in tile order
+    std::vector<int> pad_slot(pad_gid.size(), -1);
     for (int i = 0; i < N; ++i) soff[(size_t)i + 1] += soff[i];
     std::vector<int> own_off((size_t)n_tiles + 1, 0), own_gid;
     std::vector<uint16_t> own_ln;
@@ -614,16 +604,19 @@ static int build_tiling(tlfea_element_s* h, const double* x, const double* y, co
             if (soff[i + 1] - soff[i] > 1) load[slot_tile[best]]++;
             owner[i] = best;
         }
-        std::vector<int> mine;
+        std::vector<unsigned long long> mine;  // by descending number of tiles, then node id
+        own_gid.reserve((size_t)N);
+        own_ln.reserve((size_t)N);
         for (int tile = 0; tile < n_tiles; ++tile) {
             mine.clear();
-            for (int k = pad_off[tile]; k < pad_off[tile + 1]; ++k)
-                if (pad_gid[k] >= 0 && owner[pad_gid[k]] == pad_slot[k]) mine.push_back(pad_gid[k]);
-            std::sort(mine.begin(), mine.end(), [&](int a, int b) {
-                const int na = soff[a + 1] - soff[a], nb = soff[b + 1] - soff[b];
-                return na != nb ? na > nb : a < b;
-            });
-            for (int g : mine) {
+            for (int k = pad_off[tile]; k < pad_off[tile + 1]; ++k) {
+                const int g = pad_gid[k];
+                if (g >= 0 && owner[g] == pad_slot[k])
+                    mine.push_back((unsigned long long)(0x7fffffff - (soff[g + 1] - soff[g])) << 32 | (unsigned)g);
+            }
+            std::sort(mine.begin(), mine.end());
+            for (unsigned long long m : mine) {
+                const int g = (int)(m & 0xffffffffu);
                 own_gid.push_back(g);
                 own_ln.push_back((uint16_t)slot_ln[owner[g]]);
             }
@@ -659,7 +652,7 @@ static int build_tiling(tlfea_element_s* h, const double* x, const double* y, co
     if ((st = upload(&tl.lconn, lconn, h->stream))) return st;
     if ((st = upload(&tl.tile_elem, tile_elem, h->stream))) return st;
     std::vector<int> elem_slot((size_t)E);
-    for (int s = 0; s < E; ++s) elem_slot[std::get<2>(key[s])] = s;
+    for (int s = 0; s < E; ++s) elem_slot[order[s]] = s;
     if ((st = upload(&tl.elem_slot, elem_slot, h->stream))) return st;
     if ((st = upload(&tl.bnode_gid, bgid, h->stream))) return st;
     if ((st = upload(&tl.bnode_off, boff, h->stream))) return st;
@@ -1087,6 +1080,61 @@ static int noalloc_scratch(int device, double** out) {
     return TLFEA_OK;
 }
 
+// Error words of the elements alive: one pinned page that every device sees, taken with the
+// process's first element and kept (a pinned allocation takes 2 to 4 ms, more than the rest of a
+// small element's setup), a word per element; past its 1024 words, an allocation per element.  The
+// page is asked for again if it went with its context (cudaDeviceReset).
+struct ErrorPage {
+    static constexpr int WORDS = 1024;
+    std::mutex lock;
+    int* base = nullptr;
+    std::vector<int> free;
+};
+static ErrorPage g_error_page;
+
+static int* pinned_words(int n) {
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, n * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return static_cast<int*>(p);
+}
+
+static int* take_error_word() {
+    ErrorPage& P = g_error_page;
+    std::lock_guard<std::mutex> g(P.lock);
+    cudaPointerAttributes at{};
+    if (P.base && (cudaPointerGetAttributes(&at, P.base) != cudaSuccess || at.type != cudaMemoryTypeHost)) {
+        cudaGetLastError();
+        P.base = nullptr;
+    }
+    if (!P.base) {
+        P.free.clear();
+        if ((P.base = pinned_words(ErrorPage::WORDS)))
+            for (int i = ErrorPage::WORDS; i-- > 0;) P.free.push_back(i);
+    }
+    int* w = nullptr;
+    if (!P.free.empty()) {
+        w = P.base + P.free.back();
+        P.free.pop_back();
+    } else {
+        w = pinned_words(1);
+    }
+    if (w) *w = 0;
+    return w;
+}
+
+// After the element's memory is freed: nothing of it runs any more.
+static void give_error_word(int* w) {
+    ErrorPage& P = g_error_page;
+    std::lock_guard<std::mutex> g(P.lock);
+    if (P.base && w >= P.base && w < P.base + ErrorPage::WORDS)
+        P.free.push_back((int)(w - P.base));
+    else if (cudaFreeHost(w) != cudaSuccess)
+        cudaGetLastError();
+}
+
 // A kernel's bounded wait ran out: report it once and clear the word.
 static int check_device_error(tlfea_element_s* h) {
     // host memory that the kernels see (they write it only then): after the caller's
@@ -1206,12 +1254,10 @@ int tlfea_element_create(int type, int n_elem, int n_nodes, tlfea_element* out) 
     st |= dalloc(&h->d_conn, (size_t)n_elem * h->npe);
     st |= dalloc(&h->f_int, 3 * N) | dalloc(&h->f_ext, 3 * N) | dalloc(&h->f_int32, 3 * N);
     st |= dalloc(&h->detJ, (size_t)n_elem * h->nqp);
-    if (cudaHostAlloc((void**)&h->h_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer((void**)&h->d_err, h->h_err, 0) != cudaSuccess) {
+    h->h_err = take_error_word();
+    if (!h->h_err || cudaHostGetDevicePointer((void**)&h->d_err, h->h_err, 0) != cudaSuccess) {
         set_error("element_create: pinned error word");
         st |= 1;
-    } else {
-        *h->h_err = 0;
     }
     if (st) {
         tlfea_element_destroy(h);
@@ -1234,7 +1280,7 @@ int tlfea_element_destroy(tlfea_element h) {
     dfree(h->X0x); dfree(h->X0y); dfree(h->X0z); dfree(h->u64);
     dfree(h->d_conn); dfree(h->f_int); dfree(h->f_ext); dfree(h->f_int32);
     dfree(h->detJ); dfree(h->Pst);
-    if (h->h_err) cudaFreeHost(h->h_err);
+    if (h->h_err) give_error_word(h->h_err);
     h->h_err = h->d_err = nullptr;
     free_tiling(h->tl);
     dfree(h->inc_off); dfree(h->inc_e); dfree(h->inc_a);
