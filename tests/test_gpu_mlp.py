@@ -140,3 +140,52 @@ def test_training_fits_a_smooth_map_and_is_deterministic():
     assert last < 0.05 * first
     _, last2, p2 = run()
     assert np.array_equal(p1, p2) and last == last2
+
+
+# widths and batches off the tiles of the products (128 x 64) and of the reductions (32 rows);
+# products on 256- and 128-column tiles, whose gradients do not share a launch
+@pytest.mark.parametrize("dims,batch", [([3, 16], 16), ([5, 16, 272, 48], 144), ([20, 80, 336, 32], 1040),
+                                        ([8, 2048, 1296, 64], 2064)])
+def test_gradients_off_the_tiles_match_oracle(dims, batch):
+    """The bars of the square network above: 1e-3 of the loss, 2e-2 of a layer's gradient."""
+    import torch
+
+    net = T.WarmStartMLP(dims, max_batch=(batch + 127) // 128 * 128, seed=4)
+    r = np.random.default_rng(batch)
+    X = r.standard_normal((batch, dims[0])).astype(np.float32)
+    Y = r.standard_normal((batch, dims[-1])).astype(np.float32)
+    dx, dy = torch.tensor(X, device="cuda"), torch.tensor(Y, device="cuda")
+    torch.cuda.synchronize()
+    loss = net.LossGrad(dx.data_ptr(), dy.data_ptr(), batch)
+    loss_ref, g_ref = MO.MLP(dims, net.GetParams(), bf16=True).loss_grad(X, Y)
+    assert abs(loss - loss_ref) / loss_ref < 1e-3
+    (Wg, bg), (Wr, br) = MO.unflatten(net.GetGrads(), dims), MO.unflatten(g_ref, dims)
+    for l in range(len(dims) - 1):
+        assert rel(Wg[l], Wr[l]) < 2e-2 and rel(bg[l], br[l]) < 2e-2
+    net.Destroy()
+
+
+@pytest.mark.parametrize("dims", [[3, 16], [5, 16, 272, 48], [4] + [32] * 9])  # the last: two closing launches
+def test_fused_step_equals_gradients_and_adamw(dims):
+    """TrainStep against LossGrad + AdamWStep from the same weights: the same gradients and the
+    same update, in two kernels whose contractions may differ by an ulp of lr = 1e-3."""
+    import torch
+
+    r = np.random.default_rng(1)
+    dx = torch.tensor(r.standard_normal((144, dims[0])).astype(np.float32), device="cuda")
+    dy = torch.tensor(r.standard_normal((144, dims[-1])).astype(np.float32), device="cuda")
+    torch.cuda.synchronize()
+    out = []
+    for fused in (True, False):
+        net = T.WarmStartMLP(dims, max_batch=256, seed=9)
+        losses = []
+        for _ in range(3):
+            if fused:
+                losses.append(net.TrainStep(dx.data_ptr(), dy.data_ptr(), 144, 1e-3, 0.9, 0.999, 1e-8, 1e-4, True))
+            else:
+                losses.append(net.LossGrad(dx.data_ptr(), dy.data_ptr(), 144))
+                net.AdamWStep(1e-3, 0.9, 0.999, 1e-8, 1e-4)
+        out.append((losses, net.GetParams()))
+        net.Destroy()
+    assert out[0][0][0] == out[1][0][0]
+    assert np.max(np.abs(out[0][1] - out[1][1])) < 1e-6

@@ -136,3 +136,170 @@ def test_zero_load_no_iterations_and_breakdown():
     assert sb.GetLastIterCount() == 100 and sb.GetLastResidual() == 1.0
     del s, s0, sb
     el.Destroy()
+
+
+# ---------------------------------------------------------------- internal force
+# 6 elements; three whole tiles (384); a ragged last tile; more tiles than resident blocks (610)
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-10), ("fp32", 1e-5)])  # the element tests' bars
+@pytest.mark.parametrize("cells,order", [((1, 1, 1), 10), ((8, 4, 2), 10), ((9, 3, 2), 10), ((130, 10, 10), 10),
+                                         ((1, 1, 1), 4), ((8, 4, 2), 4), ((31, 7, 5), 4)])
+def test_internal_force_of_straight_elements(cells, order, prec, tol):
+    import torch
+
+    x, y, z, conn = box(*cells, order)
+    x, y, z = jitter(x, y, z, conn, 0.05 / max(cells[0], 10 * cells[1]))
+    el = make_element(x, y, z, conn, eta=2.0e3, lamd=5.0e2, mass=False)
+    el.SetForcePrecision(prec)
+    xs = perturb(x, y, z, 0.02 / max(cells[0], 10 * cells[1]), 6)
+    el.UpdatePositions(*xs)
+    g, dj = O.dndu_pre(x, y, z, conn)
+    el.ComputeInternalForce()
+    assert rel(el.RetrieveInternalForceToCPU(), O.force(*xs, conn, g, dj, LAM, MU)) < tol
+    v = np.random.default_rng(2).standard_normal(3 * len(x)) * 0.1
+    dv = torch.tensor(v, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    el.ComputeInternalForce(dv.data_ptr())
+    f = el.RetrieveInternalForceToCPU()
+    assert rel(f, O.force(*xs, conn, g, dj, LAM, MU, 2.0e3, 5.0e2, v)) < tol
+    el.ComputeInternalForce(dv.data_ptr())
+    assert np.array_equal(el.RetrieveInternalForceToCPU(), f)
+    el.Destroy()
+
+
+def test_internal_force_beside_orphans_and_of_curved_elements():
+    x, y, z, conn = box(5, 2, 2, 10)
+    r = np.random.default_rng(5)
+    xo, yo, zo = (np.concatenate([v, [7.0, 8.0]]) for v in (x, y, z))  # two nodes without elements
+    edge = np.unique(conn[:, 4:])
+    xc, yc, zc = x.copy(), y.copy(), z.copy()
+    for v in (xc, yc, zc):
+        v[edge] += 1e-3 * r.uniform(-1, 1, edge.size)
+    for p in ((xo, yo, zo), (xc, yc, zc)):
+        el = make_element(*p, conn, mass=False)
+        xs = perturb(*p, 1e-3, 6)
+        el.UpdatePositions(*xs)
+        g, dj = O.dndu_pre(*p, conn)
+        el.ComputeInternalForce()
+        f = el.RetrieveInternalForceToCPU()
+        assert rel(f, O.force(*xs, conn, g, dj, LAM, MU)) < 1e-10
+        assert not f.reshape(-1, 3)[np.setdiff1d(np.arange(len(p[0])), conn)].any()
+        el.Destroy()
+
+
+# ---------------------------------------------------------------- first-order solvers
+# one tile, whole tiles, a ragged last tile; 610 tiles: beyond the resident launch (444 in FP64)
+@pytest.mark.parametrize("kind,cells,order", [
+    ("nesterov", (3, 2, 2), 10), ("nesterov", (8, 4, 2), 10), ("nesterov", (9, 3, 2), 10),
+    ("nesterov", (31, 3, 2), 4), ("nesterov", (130, 10, 10), 10), ("adamw", (9, 3, 2), 10), ("adamw", (31, 3, 2), 4),
+    ("nocoop", (8, 4, 2), 10), ("adamw", (130, 10, 10), 10)])
+def test_first_order_steps_on_straight_elements(kind, cells, order):
+    from .test_gpu_solvers import ADAMW, E_MOD, _oracle_displacement_with_bar
+
+    x, y, z, conn = box(*cells, order)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (10.0, 20.0, -50.0))
+    if kind == "nesterov":
+        params = (1.0e-5, 1e8, 0.0, 0.0, 2, 8, 1.0e-3)
+        s_cls, p = T.SyncedNesterovSolver, T.SyncedNesterovParams(*params)
+    else:
+        a = list(ADAMW)
+        a[0], a[3], a[6], a[7], a[8], a[9], a[10] = 1e-3, 1.0, 0.0, 0.0, 1e4, 2, 8
+        params = tuple(a)
+        s_cls = T.SyncedAdamWSolver if kind == "adamw" else T.SyncedAdamWNocoopSolver
+        p = T.SyncedAdamWParams(*params)
+    el = make_element(x, y, z, conn, fixed=fixed, f_ext=f)
+    s = s_cls(el, el.get_n_constraint())
+    s.Setup()
+    s.SetParameters(p)
+    for _ in range(2):
+        s.Solve()
+    assert s.GetStats()["inner_iters_total"] == 16
+    # both AdamW solvers take the same steps at a fixed count
+    disp, bar = _oracle_displacement_with_bar(x, y, z, conn, E_MOD, fixed, f, "nesterov" if kind == "nesterov" else
+                                              "adamw", params, 2)
+    assert rel(np.stack(el.RetrievePositionToCPU()) - np.stack([x, y, z]), disp) < bar
+    del s
+    el.Destroy()
+
+
+@pytest.mark.parametrize("cells", [(9, 3, 2), (130, 10, 10)])
+def test_first_order_fp32_forces_on_straight_elements(cells):
+    """Element forces in FP32 against the oracle: the solvers' bar for FP32 forces, 1e-4 of the
+    displacement."""
+    from .test_gpu_solvers import E_MOD, _oracle_displacement_with_bar
+
+    x, y, z, conn = box(*cells, 10)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (10.0, 20.0, -50.0))
+    params = (1.0e-5, 1e8, 0.0, 0.0, 2, 8, 1.0e-3)
+    el = make_element(x, y, z, conn, fixed=fixed, f_ext=f)
+    el.SetForcePrecision("fp32")
+    s = T.SyncedNesterovSolver(el, el.get_n_constraint())
+    s.Setup()
+    s.SetParameters(T.SyncedNesterovParams(*params))
+    s.Solve()
+    disp, _ = _oracle_displacement_with_bar(x, y, z, conn, E_MOD, fixed, f, "nesterov", params, 1)
+    assert rel(np.stack(el.RetrievePositionToCPU()) - np.stack([x, y, z]), disp) < 1e-4
+    del s
+    el.Destroy()
+
+
+# ---------------------------------------------------------------- batches
+# the group sizes of the launch (1, 2, 4, 8 sequences a block) and their remainders
+@pytest.mark.parametrize("n,cells,order", [(1, (8, 4, 2), 10), (2, (9, 3, 2), 10), (5, (3, 2, 2), 10),
+                                           (9, (9, 3, 2), 10), (17, (4, 2, 2), 10), (3, (31, 3, 2), 4)])
+def test_sequences_on_straight_elements(n, cells, order):
+    from .test_gpu_dynamics import _batch, _mesh, _oracle_with_bar
+
+    x, y, z, conn, fixed, f, _ = _mesh(cells, order, (10.0, 20.0, -50.0))
+    r = np.random.default_rng(n)
+    E, nu = np.exp(r.uniform(np.log(1e6), np.log(2e7), n)), r.uniform(0.2, 0.4, n)
+    params = (1.0e-6, 1e8, 0.0, 0.0, 2, 8, 1.0e-3)
+    el, b = _batch(x, y, z, conn, fixed, f, E, nu, params)
+    for _ in range(2):
+        b.Step(T.BatchedDynamics.WARM_PREVIOUS)
+    X0 = np.stack([x, y, z])
+    for s in sorted({0, n // 2, n - 1}):
+        disp, vel, bx, bv = _oracle_with_bar(x, y, z, conn, E[s], nu[s], fixed, [f, f], params)
+        assert rel(np.stack(b.RetrievePositions(s)) - X0, disp[1]) < bx
+        assert rel(b.RetrieveVelocity(s), vel[1]) < bv
+    b.Destroy()
+    el.Destroy()
+
+
+# tiles that two or more instances share, instances of many tiles, single instances; on one
+# mesh, groups of several sizes with remainders
+@pytest.mark.parametrize("shared,n,order", [(False, 1, 10), (False, 7, 10), (False, 23, 10), (False, 9, 4),
+                                            (True, 2, 10), (True, 13, 10), (True, 33, 10), (True, 5, 4)])
+def test_batched_operator_and_iterates_on_straight_elements(shared, n, order):
+    """Products against the oracle's matrix; iterates after 20 steps at the batch tests' bar, for
+    quadratic elements (a 48-node mesh of linear ones is at its solution by then, where the
+    oracle's own iterate moves by 1e-8 when its matrix does by 1e-16)."""
+    import torch
+
+    from .test_gpu_batch import _oracle_kbc
+
+    insts = [M.random_beam(300 + (0 if shared else i), nx_range=(2, 14), ny_range=(1, 4), order=order)
+             for i in range(n)]
+    r = np.random.default_rng(n)
+    for d in insts:
+        d.update(E=float(np.exp(r.uniform(np.log(1e6), np.log(1e9)))), nu=float(r.uniform(0.2, 0.45)),
+                 f=d["f"] * r.uniform(0.5, 2.0))
+    b = T.BatchedLinearStaticSolver([(d["x"], d["y"], d["z"], d["conn"]) for d in insts],
+                                    T.TYPE_T10 if order == 10 else T.TYPE_T4, shared=shared)
+    b.SetMaterial([d["E"] for d in insts], [d["nu"] for d in insts])
+    b.SetNodalFixed([d["fixed"] for d in insts])
+    b.SetExternalForce([d["f"] for d in insts])
+    xs = [r.standard_normal(3 * len(d["x"])) for d in insts]
+    xd = torch.tensor(np.concatenate(xs), dtype=torch.float64, device="cuda")
+    yd = torch.empty_like(xd)
+    torch.cuda.synchronize()
+    b.Apply(xd.data_ptr(), yd.data_ptr())
+    b.Solve(1e-300, 20)
+    assert np.all(b.GetResults()[0] == 20)
+    us, y, o = b.RetrieveDisplacement(), yd.cpu().numpy(), 0
+    for k, (d, xv) in enumerate(zip(insts, xs)):
+        off, cols, kv, fb = _oracle_kbc(d)
+        assert rel(y[o:o + xv.size], O.spmv(off, cols, kv, xv)) < 1e-11
+        if order == 10:
+            assert rel(us[k], O.cg(off, cols, kv, fb, 0.0, 20)[0]) < 1e-9
+        o += xv.size
+    b.Destroy()
