@@ -17,10 +17,14 @@ The JSON line carries
   e2e       the same through the public API with host buffers: per step the
             external force and reference positions go host->device and the
             solved positions come back;
-  roofline  the dominant kernel of the step (the CG's matrix-free K p: gather,
-            k_mf_geo, combine);
-  elem_force  the fused element-force kernel (FP32 and FP64) in GB/s of the
-            algorithmic bytes E*(4*NPE + QP*NPE*3*s + QP*s) + N*6*s;
+  roofline  the dominant kernel of the step (the CG's K p on straight-sided
+            elements at the reference configuration: k_lin_tiles), with the
+            per-point product that solves from deformed positions use beside it
+            (gather, k_mf_geo, combine);
+  elem_force  the fused element-force kernels (FP32 and FP64): the gradient stream
+            in GB/s of its algorithmic bytes E*(4*NPE + QP*NPE*3*s + QP*s) + N*6*s,
+            the compact stream, and the default on straight-sided meshes
+            (k_force_straight), each with its own bytes;
   gpu_reference the reference's own CUDA build (its unchanged sources compiled
             for sm_100a, oracle/build_ref.py) on the same workload and GPU: its
             LinearStaticSolver::Solve() and its CalcP + CalcInternalForce;
@@ -29,8 +33,10 @@ The JSON line carries
 --impl reference times the reference's own CUDA build on this workload (the
 reference has no CPU implementation of the path); where that build is absent it
 falls back to the CPU oracle port.
-Inputs are larger than L2 (the matrix-free product's streams: 0.53 GB; K: 1.35 GB;
-the force kernels' gradient streams: 0.29 / 0.58 GB).
+Inputs are larger than L2: an iteration of the solve touches 0.15 GB (geometry 38 MB,
+connectivity 19 MB, three node vectors and the node slots), K is 1.35 GB, the force
+kernels' gradient streams are 0.29 / 0.58 GB.  k_force_straight's inputs in FP32, 80 MB,
+stay in L2 between its repetitions.
 """
 from __future__ import annotations
 
@@ -64,6 +70,7 @@ CG_ITERS_CFG2 = 7071
 SPMV_TRAFFIC_RATIO = 1.026
 FORCE_TRAFFIC_RATIO = {"fp32": 1.118, "fp64": 1.073}
 MF_TRAFFIC_RATIO = 1.121
+LIN_TRAFFIC_RATIO = 1.0
 
 
 def progress(msg):
@@ -170,6 +177,19 @@ def elem_force_bytes_compact(E, N, npe, nqp, s):
     """The compact geometry stream: J^-1 (9 values) and dV per QP instead of the
     3 * NPE gradients."""
     return E * (4 * npe + nqp * 10 * s) + N * 6 * s
+
+
+def elem_force_bytes_straight(E, N, npe, s):
+    """Straight-sided elements: one J^-1 and det J per element; positions and reference
+    positions read in FP64, forces written."""
+    return E * (4 * npe + 10 * s) + N * (6 * 8 + 3 * s)
+
+
+def lin_apply_bytes(E, N, npe):
+    """Algorithmic bytes of one K p at the reference configuration of a straight-sided mesh:
+    per element ten FP64 geometry values and its connectivity and incidence (4 B per node
+    slot); per node p read and q written."""
+    return E * (4 * npe + 10 * 8) + N * 3 * 8 * 2
 
 
 def mf_apply_bytes(E, N, npe, nqp):
@@ -607,17 +627,17 @@ def batched_leg(args, T):
         its.append(itp)
     plain = k / tot
     value = n / (ms / 1e3)
-    # roofline of the batched CG: per iteration an instance streams its compact geometry
-    # (J^-1 and dV per element and QP, FP64) and makes ~14 passes over 3N-vectors (the
-    # matrix-free K p reads p and writes q; p.Kp, u/r update with r.r, p update); summed
-    # over the iterations each instance ran, over the batch's time
+    # roofline of the batched CG: per iteration an instance streams one geometry per element
+    # (ten FP64 values), its connectivity, and makes ~14 passes over 3N-vectors (K p reads p
+    # and writes q; p.Kp, u/r update with r.r, p update); summed over the iterations each
+    # instance ran, over the batch's time
     hbm, _ = peaks()
-    per_iter = np.array([d["conn"].shape[0] * 5 * 10 * 8 + 3 * len(d["x"]) * 8 * 14 for d in insts], np.float64)
+    per_iter = np.array([d["conn"].shape[0] * (10 * 8 + 4 * 10) + 3 * len(d["x"]) * 8 * 14 for d in insts], np.float64)
     moved = float(np.sum(per_iter * np.asarray(it, np.float64)))
     ach = moved / (ms / 1e3) / 1e9
-    roof = {"kernel": "k_bcg_* (whole solve)", "bound": "hbm", "achieved": round(ach, 1), "peak": hbm,
+    roof = {"kernel": "k_bl_* (whole solve)", "bound": "hbm", "achieved": round(ach, 1), "peak": hbm,
             "unit": "GB/s", "frac": round(ach / hbm, 4), "algorithmic_bytes": int(moved),
-            "model": "per instance and iteration: E*5*10*8 (J^-1 + dV stream) + 3N*8*14 (vector passes)"}
+            "model": "per instance and iteration: E*(10*8 + 4*10) + 3N*8*14 (vector passes)"}
     return {"workload": f"{n} uneven TET10 cantilevers, linear static CG to 1e-6 (per-phase kernels, graph chunks)",
             "roofline": roof,
             "elements": counts["elements"], "nodes": counts["nodes"], "dof": 3 * counts["nodes"],
@@ -804,7 +824,7 @@ def config2_more_legs(args, T, cfg):
     for _ in range(3):
         el.ComputeInternalForce()
     ms_f = time_stream(torch, stream, el.ComputeInternalForce, args.kernel_reps)
-    b = elem_force_bytes(conn4.shape[0], len(x4), 4, 1, 8)
+    b = elem_force_bytes_straight(conn4.shape[0], len(x4), 4, 8)
     hbm, _ = peaks()
     t4["elem_force_fp64"] = {"ms": round(ms_f, 4), "achieved_gbs": round(b / (ms_f / 1e3) / 1e9, 1),
                              "frac": round(b / (ms_f / 1e3) / 1e9 / hbm, 4), "algorithmic_bytes": int(b)}
@@ -1252,21 +1272,52 @@ def main():
     e2e = {"value": whole_job_rate(world, args.steps, t_e2e), "unit": "solves/s", "h2d_bytes_per_step": 6 * N * 8,
            "d2h_bytes_per_step": 3 * N * 8}
 
-    # dominant kernel: the matrix-free K p of the CG (tile kernel + shared-node combine
-    # with p.q), timed back to back on the element stream at the last solve's positions
+    # dominant kernel: the CG's K p at the reference configuration, timed back to back on the
+    # element stream (with the copies between Apply's vectors and the CG's node records)
     el.SetBlocking(False)
-    for _ in range(3):
-        solver.Apply(xin.data_ptr(), yout.data_ptr())
-    ms_mf = time_stream(torch, stream, lambda: solver.Apply(xin.data_ptr(), yout.data_ptr()), args.kernel_reps)
+
+    def time_apply(sol):
+        for _ in range(3):
+            sol.Apply(xin.data_ptr(), yout.data_ptr())
+        return time_stream(torch, stream, lambda: sol.Apply(xin.data_ptr(), yout.data_ptr()), args.kernel_reps)
+
+    ms_lin = time_apply(solver)
+    b_lin = lin_apply_bytes(E, N, 10)
+    ach = b_lin / (ms_lin / 1e3) / 1e9
+    roofline = {"kernel": "k_lin_mask + k_lin_tiles + k_lin_collect", "bound": "shared-memory wavefronts and FP64 latency",
+                "achieved": round(ach, 1), "peak": hbm, "unit": "GB/s", "frac": round(ach / hbm, 4),
+                "peak_kind": peak_kind, "algorithmic_bytes": int(b_lin),
+                "format": "linear operator of straight-sided elements: J^-1, det J per element (FP64)",
+                "ms": round(ms_lin, 4), "traffic": int(LIN_TRAFFIC_RATIO * b_lin)}
+    # the product of a solve from deformed positions (the per-point SVK tangent)
+    r = np.random.default_rng(1)
+    el.UpdatePositions(*(v + 1e-4 * r.standard_normal(v.shape) for v in (x, y, z)))
+    deformed = T.LinearStaticSolver(el, cfg["tol"], 1)
+    deformed.Solve()
+    ms_mf = time_apply(deformed)
     b_mf = mf_apply_bytes(E, N, 10, 5)
     ach = b_mf / (ms_mf / 1e3) / 1e9
-    roofline = {"kernel": "k_mf_gather + k_mf_geo + k_mf_combine_dot", "bound": "hbm", "achieved": round(ach, 1), "peak": hbm,
-                "unit": "GB/s", "frac": round(ach / hbm, 4), "peak_kind": peak_kind, "algorithmic_bytes": int(b_mf),
-                "format": "matrix-free SVK tangent: per QP J^-1, dV and the solve's F, S (FP64), p per tile",
-                "ms": round(ms_mf, 4), "traffic": int(MF_TRAFFIC_RATIO * b_mf),
-                "fp64_tflops": round(mf_apply_flops(E, 5) / (ms_mf / 1e3) / 1e12, 2)}
-    # fused element force, FP32 and FP64
+    roofline["deformed_positions"] = {
+        "kernel": "k_mf_gather + k_mf_geo + k_mf_combine_dot", "bound": "hbm", "achieved": round(ach, 1), "peak": hbm,
+        "unit": "GB/s", "frac": round(ach / hbm, 4), "algorithmic_bytes": int(b_mf),
+        "format": "matrix-free SVK tangent: per QP J^-1, dV and the solve's F, S (FP64), p per tile",
+        "ms": round(ms_mf, 4), "traffic": int(MF_TRAFFIC_RATIO * b_mf),
+        "fp64_tflops": round(mf_apply_flops(E, 5) / (ms_mf / 1e3) / 1e12, 2)}
+    del deformed
+    # fused element force, FP32 and FP64: the default on this straight-sided mesh, then the
+    # launch options
     ef = {}
+    for prec, s in (("fp32", 4), ("fp64", 8)):
+        el.SetForcePrecision(prec)
+        for _ in range(3):
+            el.ComputeInternalForce()
+        ms_f = time_stream(torch, stream, el.ComputeInternalForce, args.kernel_reps)
+        b = elem_force_bytes_straight(E, N, 10, s)
+        a = b / (ms_f / 1e3) / 1e9
+        ef["straight_" + prec] = {"kernel": "k_force_straight+k_combine", "achieved": round(a, 1), "peak": hbm,
+                                  "unit": "GB/s", "frac": round(a / hbm, 4), "algorithmic_bytes": int(b),
+                                  "ms": round(ms_f, 4)}
+    el.SetLaunchConfig("tma")
     f_by_prec = {}
     for prec, s in (("fp32", 4), ("fp64", 8)):
         el.SetForcePrecision(prec)
@@ -1326,7 +1377,7 @@ def main():
            "scaling": "weak", "vs_baseline": None, "dtype": "f64", "data": "synthetic",
            "config": {"workload": WORKLOAD, "elements": E, "nodes": N,
                       "dof": 3 * N, "cg_iters_per_solve": iters, "final_rel_residual": resid,
-                      "parallelism": f"replicas{world}", "l2": "inputs larger than L2 (K 1.35 GB)"},
+                      "parallelism": f"replicas{world}", "l2": "inputs larger than L2 (0.15 GB per CG iteration)"},
            "e2e": {k: (round(v, 4) if isinstance(v, float) else v) for k, v in e2e.items()},
            "roofline": roofline, "elem_force": ef, "gpu_launches": int(launches), "clocks": clk.summary(),
            "pcg": pcg, "assembled_operator": assembled}
@@ -1348,7 +1399,7 @@ def main():
             g = gpu_reference_leg(cfg, x, y, z, conn, fixed, f, steps=2, warmup=1)
             g["speedup_value_vs_reference"] = round(out["value"] / g["value"], 3)
             g["speedup_e2e_vs_reference"] = round(out["e2e"]["value"] / g["value"], 3)
-            g["speedup_elem_force_fp64"] = round(g["elem_force_fp64"]["ms"] / ef["fp64"]["ms"], 3)
+            g["speedup_elem_force_fp64"] = round(g["elem_force_fp64"]["ms"] / ef["straight_fp64"]["ms"], 3)
             out["gpu_reference"] = g
     if rank == 0 and world == 1 and not args.no_cpu:
         src = f"this library's CG on this workload in this run ({iters} iterations)"

@@ -167,9 +167,9 @@ template <typename R>
 __device__ __forceinline__ void stage_pos(const TileArgs<R>& A, int gid, double& x, double& y, double& z) {
     if constexpr (sizeof(R) == 4) {
         if (A.u64) {
-            x = A.u64[3 * gid + 0];
-            y = A.u64[3 * gid + 1];
-            z = A.u64[3 * gid + 2];
+            x = A.u64[4 * (size_t)gid + 0];
+            y = A.u64[4 * (size_t)gid + 1];
+            z = A.u64[4 * (size_t)gid + 2];
         } else {
             x = A.x64[gid] - A.X0x[gid];
             y = A.y64[gid] - A.X0y[gid];
@@ -914,8 +914,9 @@ struct tlfea_element_s {
     double *x = nullptr, *y = nullptr, *z = nullptr;
     double *xj = nullptr, *yj = nullptr, *zj = nullptr;
     double *X0x = nullptr, *X0y = nullptr, *X0z = nullptr;
-    double* u64 = nullptr;  // interleaved x - X0 for the FP32 force (refreshed when positions change)
-    bool u_dirty = true;
+    // node records, 4 per node: 1 = x (FP64 force), 2 = x - X0 (FP32), 0 = stale
+    double* u64 = nullptr;
+    int node_content = 0;
     // the tile-ordered node record (Tiling::sx/sy/sz): 0 = stale, 1 = FP64 positions,
     // 2 = displacements x - X0 (FP32 mode); stale again whenever the positions change
     int stage_content = 0;
@@ -959,7 +960,7 @@ struct tlfea_element_s {
     int* d_err = nullptr;  // the same word as the kernels see it
     // grid of the persistent force pipeline per (FP32?, damping?), 0 = not yet sized
     int pipe_grid[4] = {0, 0, 0, 0};
-    int straight_grid[4] = {0, 0, 0, 0};  // the same of the straight-sided force kernel
+    int straight_grid[8] = {};  // the same of the straight-sided force kernel
     // launch configuration (tlfea_element_set_launch_config): force kernel 0 = gradient stream,
     // 1 = one tile per block, 2 = persistent pipeline, 3 = compact stream; -1 (until the caller
     // chooses) = the straight-sided kernel where the mesh allows it, else 0; cap on the
@@ -971,7 +972,7 @@ struct tlfea_element_s {
 // The positions changed: the records derived from them (FP32 mode's displacement u64,
 // the tile-ordered node record) are rebuilt before the next force evaluation.
 inline void positions_changed(tlfea_element_s* h) {
-    h->u_dirty = true;
+    h->node_content = 0;
     h->stage_content = 0;
 }
 
@@ -979,7 +980,7 @@ namespace tlfea {
 // Implemented in element.cu, used by the solvers.
 int element_build_pattern(tlfea_element_s* h);
 int element_force(tlfea_element_s* h, const double* d_v, bool fp32);
-int element_refresh_u64(tlfea_element_s* h);
+int element_refresh_nodes(tlfea_element_s* h, bool displacements);
 // Rebuild the tile-ordered node record (FP64 positions, or FP32 mode displacements) if stale.
 int element_refresh_record(tlfea_element_s* h, bool fp32);
 

@@ -84,6 +84,7 @@ template <typename R>
 struct SForceArgs {
     SForceTables<R> T;
     const double *x, *y, *z, *X0x, *X0y, *X0z;
+    const double* nodes;  // records of x, or of x - X0 (FP32)
     const double* v;  // interleaved velocities (DAMP)
     R* f_out;
     R* partial;
@@ -91,15 +92,17 @@ struct SForceArgs {
     SvkRule rule;
 };
 
-// The internal force, positions gathered from node order (FP32: displacements, differenced in
-// FP64), so no tile-ordered copy of them has to be rebuilt first; interior nodes written
-// directly, shared nodes as per-tile partials for k_combine.  At 480,000 elements, with the
-// positions rewritten before each call, a call takes 144 us in FP64 against 184 (gradient
-// stream: 137 the kernel, 12 the copy); 15,360 bytes of geometry per tile against 163,840.
-template <typename R, int NPE, bool DAMP>
+// The internal force; REC: node values from records (a 256-bit load a node, FP32: displacements),
+// else gathered from the position arrays (FP32: differenced from X0 in FP64), so that nothing has
+// to be rebuilt first (the rule stands at the launch); interior nodes written directly, shared
+// nodes as per-tile partials for k_combine.  At 480,000 elements, with the positions rewritten
+// before each call, a call takes 93 us in FP64 against 161 for the gradient stream and the copy it
+// stages from, 78 in FP32 against 118: 15,360 bytes of geometry per tile against 163,840.  What is
+// left is shared-memory wavefronts (node values out, forces in, forces summed) and latency.
+template <typename R, int NPE, bool DAMP, bool REC>
 __global__ void __launch_bounds__(TILE_ELEMS, sizeof(R) == 4 ? (DAMP ? 3 : 4) : (DAMP ? 2 : 3)) k_force_straight(SForceArgs<R> A) {
-    constexpr int TE = TILE_ELEMS, NB = 3;
-    constexpr bool DISP = sizeof(R) == 4;
+    constexpr int TE = TILE_ELEMS, NB = NPE == 10 ? 3 : 1;  // node values in flight per thread
+    constexpr bool DISP = sizeof(R) == 4 && !REC;
     extern __shared__ __align__(128) unsigned char smem[];
     const int t = threadIdx.x;
     const SForceTables<R>& T = A.T;
@@ -119,9 +122,13 @@ __global__ void __launch_bounds__(TILE_ELEMS, sizeof(R) == 4 ? (DAMP ? 3 : 4) : 
 #pragma unroll
         for (int j = 0; j < NB; ++j) {
             const int g = T.pad_gid[pb + min(t + j * TE, n - 1)];
-            pv[j][0] = A.x[g];
-            pv[j][1] = A.y[g];
-            pv[j][2] = A.z[g];
+            if constexpr (REC) {
+                ld_node(A.nodes + 4 * (size_t)g, pv[j]);
+            } else {
+                pv[j][0] = A.x[g];
+                pv[j][1] = A.y[g];
+                pv[j][2] = A.z[g];
+            }
             if constexpr (DISP) {
                 p0[j][0] = A.X0x[g];
                 p0[j][1] = A.X0y[g];
@@ -130,6 +137,7 @@ __global__ void __launch_bounds__(TILE_ELEMS, sizeof(R) == 4 ? (DAMP ? 3 : 4) : 
         }
     };
     sf_geometry(T, tile, ji, det);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     gather(tile, nl);
     for (int it = 0; tile < T.n_tiles; ++it) {
         if (!mbar_wait(bar0 + 8 * (it & 1), (it >> 1) & 1)) atomicExch(T.err, 3);
@@ -150,7 +158,12 @@ __global__ void __launch_bounds__(TILE_ELEMS, sizeof(R) == 4 ? (DAMP ? 3 : 4) : 
             const int pb = T.pad_off[tile];
             for (int ln = t; ln < nl; ln += TE) {
                 const int g = T.pad_gid[pb + ln];
-                if (ln >= NB * TE) {  // larger tiles
+                if (REC && ln >= NB * TE) {  // larger tiles
+                    double p[3];
+                    ld_node(A.nodes + 4 * (size_t)g, p);
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) xs[3 * ln + d] = p[d];
+                } else if (ln >= NB * TE) {
                     xs[3 * ln + 0] = A.x[g] - (DISP ? A.X0x[g] : 0.0);
                     xs[3 * ln + 1] = A.y[g] - (DISP ? A.X0y[g] : 0.0);
                     xs[3 * ln + 2] = A.z[g] - (DISP ? A.X0z[g] : 0.0);
@@ -219,7 +232,7 @@ struct SeqForceArgs {
 // sequence of units (item, sequence), an item a tile and a group of sequences.
 template <typename R, int NPE, typename Run>
 __device__ __forceinline__ void seq_force_tiles(const SeqForceArgs<R>& A, unsigned char* smem, Run running) {
-    constexpr int TE = TILE_ELEMS, NB = 3;
+    constexpr int TE = TILE_ELEMS, NB = NPE == 10 ? 3 : 1;  // node values in flight per thread
     const int t = threadIdx.x;
     const SForceTables<R>& T = A.T;
     const SForceLayout<R, NPE> L(T.max_local, true);
