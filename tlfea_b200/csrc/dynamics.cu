@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(DYN_NODE_THREADS) k_dyn_grad(DynArgs D) {
 // update, so the tiles gather two records per node instead of nine scattered values) and the
 // tile sums in node slots.  The node kernels issue every load before their first store: with
 // the two interleaved the compiler has to keep their order, and each store waits for a round
-// trip (at 16 sequences of 88,641 nodes 149 us for the two kernels, 149 before).
+// trip (at 16 sequences of 88,641 nodes the two take 104 us back to back, 149 with them mixed).
 __device__ __forceinline__ void dyn_record(const DynArgs& D, size_t node, const double xp[3], const double vp[3],
                                            const double y[3]) {
     st_node(D.x4 + 4 * node, xp[0] + D.dt * y[0], xp[1] + D.dt * y[1], xp[2] + D.dt * y[2]);
@@ -340,9 +340,10 @@ __global__ void __launch_bounds__(TILE_ELEMS, NPE == 10 ? 3 : 4) k_dyn_force_str
     seq_force_tiles<double, NPE>(A, smem, [&](int s) { return __ldcg(D.done + s) == DYN_RUNNING; });
 }
 
-// As k_dyn_grad, DYN_GRAD_NODES nodes per thread: a block that ends pays the reduction's fence
-// and ticket, so a sequence has few blocks.
-constexpr int DYN_GRAD_NODES = 4;
+// As k_dyn_grad, up to DYN_GRAD_NODES nodes per thread: a block that ends pays the reduction's
+// fence and ticket, so a sequence has few blocks; below DYN_GRAD_FILL blocks (4 per SM) of one
+// node a thread the chip is not full and a thread's nodes would only queue.
+constexpr int DYN_GRAD_NODES = 4, DYN_GRAD_FILL = 592;
 __global__ void __launch_bounds__(DYN_NODE_THREADS) k_dyn_grad_straight(DynArgs D) {
     __shared__ double red_sh[32];
     __shared__ bool last;
@@ -938,7 +939,8 @@ int tlfea_dynbatch_create(tlfea_element mesh, int n_seq, tlfea_dynbatch* out) {
     D.slots = b->slots;
     D.node_soff = el->tl.node_soff;
     D.n_slots = el->tl.n_local_total;
-    D.grad_blocks = (bps + DYN_GRAD_NODES - 1) / DYN_GRAD_NODES;
+    const int per_thread = std::min(DYN_GRAD_NODES, std::max(1, bps * b->B / DYN_GRAD_FILL));
+    D.grad_blocks = (bps + per_thread - 1) / per_thread;
     cudaMemsetAsync(b->mom, 0, B * sizeof(int), stream);
     const dim3 grid(bps, n_seq);
     k_dyn_reset_state<<<grid, DYN_NODE_THREADS, 0, stream>>>(D, b->vhist, el->X0x, el->X0y, el->X0z);
