@@ -1,6 +1,8 @@
 // first_order.cu -- SyncedNesterovSolver, SyncedAdamWSolver and
 // SyncedAdamWNocoopSolver (SyncedNesterov.cu:97-414, SyncedAdamW.cu:99-425,
-// SyncedAdamWNocoop.cu:97-458) as one persistent cooperative kernel per Solve().
+// SyncedAdamWNocoop.cu:97-458) as one persistent cooperative kernel per Solve(), as one kernel
+// per phase in CUDA-graph chunks (from 200,000 nodes), and on straight-edged SVK meshes as
+// fo_resident.cuh's one launch or, for Nesterov beyond its size, as the k_fos_* phases.
 //
 // Differences from the reference, none of which changes the iteration:
 //   * every phase is grid-strided, so any mesh size runs (the reference
@@ -1513,7 +1515,10 @@ int first_order_steps(tlfea_solver_s* s, int steps, const StepLoad* load, int* i
     const int n_steps = std::max(1, steps);
     st = TLFEA_OK;
     // the straight-sided paths (explicit launch modes keep the general kernels): the resident
-    // solve where every tile fits, else Nesterov's per-phase launches
+    // solve where every tile fits, else Nesterov's per-phase launches.  Nesterov takes them from
+    // three tiles a SM on, where a tile's block has 128 threads for its nodes too: 60 iterations
+    // at 36,000 elements (282 tiles) 1.41 ms resident against 1.63, at 48,000 (375) 1.98 against
+    // 1.67, at 60,000 2.05 in FP64 by phases against 3.78 for the general persistent launch.
     const size_t straight_smem = el->npe == 10 ? SForceLayout<double, 10>(el->tl.max_local_pad, true).total
                                                : SForceLayout<double, 4>(el->tl.max_local_pad, true).total;
     const bool straight = s->fo_mode == 0 && mass && !damp && el->tl.straight && el->tl.n_orphans == 0 &&
@@ -1523,6 +1528,7 @@ int first_order_steps(tlfea_solver_s* s, int steps, const StepLoad* load, int* i
         st = fp32 ? (el->npe == 10 ? resident_column<float, 10>(s, &column) : resident_column<float, 4>(s, &column))
                   : (el->npe == 10 ? resident_column<double, 10>(s, &column) : resident_column<double, 4>(s, &column));
         if (st) return st;
+        if (s->kind == KIND_NESTEROV && column == 0) column = -1;
         if (column >= 0 || s->kind == KIND_NESTEROV) {
             if ((st = fos_alloc(s))) return st;
             return straight_steps(s, S, n_steps, load, inner_iters, fp32, column);
