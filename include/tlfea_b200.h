@@ -176,10 +176,12 @@ int tlfea_element_compute_internal_force(tlfea_element h, const double* d_v);
 int tlfea_element_set_force_precision(tlfea_element h, int precision);
 /* Launch configuration of the fused force kernel (new; the autotuner's knob):
  * force_kernel 0 = one tile per block with bulk-copy double-buffered QP
- * slices of the gradient stream (default), 1 = one tile per block with direct
- * loads, 2 = persistent producer/consumer pipeline, 3 = as 0 on the compact
- * geometry stream (J^-1 and dV per QP, gradients formed in registers);
- * grid_limit caps the persistent grid (0 = all resident blocks). */
+ * slices of the gradient stream, 1 = one tile per block with direct loads, 2 =
+ * persistent producer/consumer pipeline, 3 = as 0 on the compact geometry stream
+ * (J^-1 and dV per QP, gradients formed in registers); grid_limit caps the
+ * persistent grid (0 = all resident blocks).  An element that was never given a
+ * configuration takes one J^-1 per element where the mesh allows it (SVK,
+ * mid-edge nodes at their edges' midpoints), else kernel 0. */
 int tlfea_element_set_launch_config(tlfea_element h, int force_kernel, int grid_limit);
 
 /* Allocation-free internal force.  No counterpart in the reference.
@@ -267,8 +269,10 @@ int tlfea_linear_static_set_preconditioner(tlfea_solver s, int kind);
  * solve, 15 doubles per element and QP), never assembled (K is assembled on demand, at the
  * positions of the last solve, for tlfea_linear_static_retrieve_k); 1 = the assembled K of
  * the reference (3x3 node blocks); 0 (default) = matrix-free where it applies from 100,000
- * elements, assembled otherwise.  Both are the same operator: the solutions and iteration
- * counts agree to rounding. */
+ * elements, assembled otherwise.  With 0 and 2 a solve from the reference configuration of a
+ * TET10 mesh with straight edges (SVK, no damping, no preconditioner, more than 128 elements)
+ * applies the linear operator of those elements, at any size, in one launch up to 75,776
+ * elements.  All are the same operator: the solutions and iteration counts agree to rounding. */
 int tlfea_linear_static_set_operator(tlfea_solver s, int mode);
 /* GetLastIterCount / GetLastResidual (LinearStaticSolver.cuh:68-72). */
 int tlfea_linear_static_last(tlfea_solver s, int* iters, double* rel_residual);
@@ -294,7 +298,9 @@ int tlfea_solver_set_stop_rule(tlfea_solver s, double rel_tol);
  * device, chunks of iterations replayed as CUDA graphs until the solve ends; 1 = the
  * whole Solve() in one persistent cooperative launch; 0 (default) = per-phase from
  * 200,000 nodes, persistent below.  The iterations are the same; with fixed iteration
- * counts so are the trajectories, bit for bit. */
+ * counts so are the trajectories of 1 and 2, bit for bit.  With 0, an undamped SVK solve on a
+ * mesh with straight edges without the stop rule sums its forces in another order (one J^-1
+ * per element): the same iterations to rounding. */
 int tlfea_solver_set_mode(tlfea_solver s, int mode);
 
 /* New, no reference counterpart: n_steps implicit steps of a first-order solver

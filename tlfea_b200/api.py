@@ -178,7 +178,9 @@ class _TetData(ElementBase):
     def SetLaunchConfig(self, force_kernel="tma", grid_limit: int = 0):
         """New: the fused force kernel -- "tma" (gradient stream, bulk-copy double
         buffered), "direct", "pipeline" (persistent producer/consumer) or
-        "compact" (J^-1 stream, gradients formed in registers)."""
+        "compact" (J^-1 stream, gradients formed in registers).  Without this call an SVK
+        element whose edges are straight is evaluated from one J^-1 per element, any other
+        by "tma"."""
         k = self.FORCE_KERNELS[force_kernel] if isinstance(force_kernel, str) else int(force_kernel)
         capi.call("tlfea_element_set_launch_config", self._handle(), k, int(grid_limit))
 
@@ -405,7 +407,8 @@ class _FirstOrder(SolverBase):
         """New: "phased" -- one kernel per phase, the loop state on the device, chunks of
         iterations replayed as CUDA graphs -- or "persistent" (the whole Solve() in one
         cooperative launch); "auto" (the default) takes the per-phase launches from
-        200,000 nodes."""
+        200,000 nodes, and on straight-edged SVK meshes kernels of their own (one J^-1 per
+        element, one launch per Solve() while every tile is resident)."""
         capi.call("tlfea_solver_set_mode", self._h, {"auto": 0, "persistent": 1, "phased": 2}[mode])
 
     def RunSteps(self, n_steps: int, f_var=None, amp: float = 1.0, omega: float = 0.0, phase: float = 0.0,
@@ -477,7 +480,8 @@ class LinearStaticSolver(SolverBase):
     def SetOperator(self, mode: str = "auto"):
         """New: "matrix-free" (TET10, SVK, no damping, no preconditioner), "assembled"
         (the reference's assembled K), or "auto" (the default: matrix-free from 100,000
-        elements where it applies)."""
+        elements where it applies).  Solves from the reference configuration of a straight-edged
+        TET10 mesh apply its linear operator unless "assembled" is asked for."""
         capi.call("tlfea_linear_static_set_operator", self._h, {"auto": 0, "assembled": 1, "matrix-free": 2}[mode])
 
     def _last(self):
