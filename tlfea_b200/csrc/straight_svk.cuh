@@ -120,10 +120,9 @@ __device__ __forceinline__ void svk_element(const R (&ji)[9], R det, R lam, R mu
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                T[i][j] = a0 * P[i][j];   // the centroid's share of sb and (4 / 4) of every moment
-                sb[i][j] = T[i][j];
+                T[i][j] = R(0);
+                sb[i][j] = a0 * P[i][j];
             }
-        const R c1 = R(4) * a1 * ra, c2 = R(4) * a1 * rb;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
 #pragma unroll
@@ -138,17 +137,22 @@ __device__ __forceinline__ void svk_element(const R (&ji)[9], R det, R lam, R mu
             for (int i = 0; i < 3; ++i)
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    T[i][j] += c2 * P[i][j];
-                    sb[i][j] += a1 * P[i][j];
-                    B[q][i][j] = c1 * P[i][j];
+                    T[i][j] += P[i][j];
+                    B[q][i][j] = P[i][j];
                 }
         }
+        // sb = sum_q w_q P_q det J; B_v = sum_q w_q (4 L_v - 1) P_q det J, which the centroid is
+        // not part of (formed as 4 sum_q w_q L_v P_q - sb it cancels)
+        const R d1 = R(4) * a1 * ra, d2 = R(rule.w1 * (4.0 * rule.b - 1.0)) * det;
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
+        for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
+            for (int j = 0; j < 3; ++j) {
+                sb[i][j] += a1 * T[i][j];
+                T[i][j] *= d2;
 #pragma unroll
-                for (int j = 0; j < 3; ++j) B[q][i][j] += T[i][j];  // 4 sum_q w_q L_v P_q det J
+                for (int q = 0; q < 4; ++q) B[q][i][j] = T[i][j] + d1 * B[q][i][j];
+            }
     } else {
         svk_p<R, DAMP>(B[0], Bd[0], lam, mu, eta, lamd, sb);
         const R a0 = R(rule.w0) * det;
@@ -212,15 +216,18 @@ __device__ __forceinline__ void svk_element(const R (&ji)[9], R det, R lam, R mu
         }
         if constexpr (NPE == 10) {
 #pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int m = 0; m < 3; ++m) {
+                    f[i] += B[i][c][m] * gl[i][m];
+                    B[i][c][m] += sb[c][m];  // 4 sum_q w_q L_v P_q det J
+                }
+#pragma unroll
             for (int k = 0; k < 6; ++k) {
                 const int i = edge_i(k), j = edge_j(k);
 #pragma unroll
                 for (int m = 0; m < 3; ++m) f[4 + k] += B[i][c][m] * gl[j][m] + B[j][c][m] * gl[i][m];
             }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int m = 0; m < 3; ++m) f[i] += (B[i][c][m] - sb[c][m]) * gl[i][m];
         } else {
 #pragma unroll
             for (int i = 0; i < 4; ++i)
