@@ -22,16 +22,17 @@ template <typename R, int NPE, typename X>
 __device__ __forceinline__ void vertex_f(const R (&ji)[9], X x, R (&V)[NPE == 10 ? 4 : 1][3][3]) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
+        // FP64 up to the vertex gradients: their coefficients of 3 and 4 would amplify FP32 rounding
         const double x0 = x(0, c);
-        R d[NPE], G[NPE == 10 ? 4 : 1][3];
-        d[0] = R(0);
+        double d[NPE], G[NPE == 10 ? 4 : 1][3];
+        d[0] = 0.0;
 #pragma unroll
-        for (int a = 1; a < NPE; ++a) d[a] = R(x(a, c) - x0);
-        vertex_gradients<R, NPE>(d, G);
+        for (int a = 1; a < NPE; ++a) d[a] = x(a, c) - x0;
+        vertex_gradients<double, NPE>(d, G);
 #pragma unroll
         for (int v = 0; v < (NPE == 10 ? 4 : 1); ++v)
 #pragma unroll
-            for (int j = 0; j < 3; ++j) V[v][c][j] = G[v][0] * ji[j] + G[v][1] * ji[3 + j] + G[v][2] * ji[6 + j];
+            for (int j = 0; j < 3; ++j) V[v][c][j] = R(G[v][0]) * ji[j] + R(G[v][1]) * ji[3 + j] + R(G[v][2]) * ji[6 + j];
     }
 }
 
