@@ -272,7 +272,9 @@ int tlfea_linear_static_set_preconditioner(tlfea_solver s, int kind);
  * elements, assembled otherwise.  With 0 and 2 a solve from the reference configuration of a
  * TET10 mesh with straight edges (SVK, no damping, no preconditioner, more than 128 elements)
  * applies the linear operator of those elements, at any size, in one launch up to 75,776
- * elements.  All are the same operator: the solutions and iteration counts agree to rounding. */
+ * elements, unless max_iter lies between 81 and 999 (iterates of a stopped solve amplify the
+ * operators' rounding there).  All are the same operator: converged solutions and iteration
+ * counts agree to rounding. */
 int tlfea_linear_static_set_operator(tlfea_solver s, int mode);
 /* GetLastIterCount / GetLastResidual (LinearStaticSolver.cuh:68-72). */
 int tlfea_linear_static_last(tlfea_solver s, int* iters, double* rel_residual);

@@ -7,6 +7,8 @@ geometry of a straight element is its corners', whose distance from the per-poin
 rounding of the coordinates, 1e-16 |x| / h.  With h >= 1/200 of the beam that is under 1e-13,
 times a few tens of additions: 1e-11 for products of random vectors.  Converged solves differ
 by the tolerance 1e-10 times the beam's condition: 1e-7."""
+from pathlib import Path
+
 import numpy as np
 import pytest
 import scipy.sparse as sp
@@ -95,6 +97,45 @@ def test_resident_and_phased_forms_agree_at_a_fixed_count(cells):
         el.ResetPositions()
         del s
     assert rel(out[0], out[1]) < 1e-9
+    el.Destroy()
+
+
+# the smallest and the largest such budget, between them the one that showed the difference; 80 and
+# 1000 lie outside: the linear operator, whose iterates agree to 1e-13 of the positions (80) and, where
+# the solve converges, to the tolerance
+@pytest.mark.parametrize("budget", [80, 81, 100, 999, 1000])
+def test_stopped_solves_return_the_iterates_of_the_assembled_operator(budget):
+    x, y, z, conn = box(24, 4, 4, 10)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (0.0, 3.0, -100.0))
+    x, y, z = jitter(x, y, z, conn, 0.002)
+    el = make_element(x, y, z, conn, fixed=fixed, f_ext=f, mass=False)
+    out = []
+    for operator in ("auto", "assembled"):
+        s = T.LinearStaticSolver(el, 1e-10, budget)
+        s.SetOperator(operator)
+        s.Solve()
+        assert s.GetLastIterCount() == budget
+        out.append(np.stack(el.RetrievePositionToCPU()))
+        el.ResetPositions()
+        del s
+    assert np.array_equal(out[0], out[1]) == (81 <= budget <= 999)
+    if budget == 80:
+        assert rel(out[0], out[1]) < 1e-9
+    el.Destroy()
+
+
+def test_stopped_solve_of_a_large_mesh_returns_the_recorded_iterate():
+    """150 iterations at 108,192 elements, every 499th node, as the per-point operator gave them on a B200:
+    rounding in another order moves this iterate by 2e-8."""
+    x, y, z, conn = box(92, 14, 14, 10)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (0.0, 3.0, -100.0))
+    x, y, z = jitter(x, y, z, conn, 7e-4, 1)
+    el = make_element(x, y, z, conn, fixed=fixed, f_ext=f, mass=False)
+    s = T.LinearStaticSolver(el, 1e-10, 150)
+    s.Solve()
+    want = np.load(Path(__file__).parent / "golden" / "stopped_cg_t10.npz")["positions"]
+    assert rel(np.stack(el.RetrievePositionToCPU())[:, ::499], want) < 1e-9
+    del s
     el.Destroy()
 
 

@@ -481,7 +481,8 @@ class LinearStaticSolver(SolverBase):
         """New: "matrix-free" (TET10, SVK, no damping, no preconditioner), "assembled"
         (the reference's assembled K), or "auto" (the default: matrix-free from 100,000
         elements where it applies).  Solves from the reference configuration of a straight-edged
-        TET10 mesh apply its linear operator unless "assembled" is asked for."""
+        TET10 mesh apply its linear operator unless "assembled" is asked for or max_iter lies
+        between 81 and 999 (a solve stopped there returns what the other operators give)."""
         capi.call("tlfea_linear_static_set_operator", self._h, {"auto": 0, "assembled": 1, "matrix-free": 2}[mode])
 
     def _last(self):
