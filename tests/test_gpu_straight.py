@@ -262,6 +262,60 @@ def test_first_order_steps_on_straight_elements(kind, cells, order):
     el.Destroy()
 
 
+@pytest.mark.parametrize("point", [(0.25, 0.25, 0.25), (0.1, 0.2, 0.3), (0.0, 0.0, 1.0)])
+@pytest.mark.parametrize("prec,tol", [("fp64", 1e-10), ("fp32", 1e-5)])
+def test_mass_of_linear_elements_follows_the_point(point, prec, tol):
+    """One quadrature point anywhere in the element: Nesterov, AdamW and a batch of sequences against the
+    persistent kernel, which takes the shape functions at the point (the solvers' and the forces' bars)."""
+    x, y, z, conn = box(31, 3, 2, 4)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (10.0, 20.0, -50.0))
+    nesterov = T.SyncedNesterovParams(1.0e-5, 1e8, 0.0, 0.0, 2, 8, 1.0e-3)
+    adamw = T.SyncedAdamWParams(2e-4, 0.9, 0.999, 1.0, 1e-4, 0.995, 0.0, 0.0, 1e4, 2, 8, 1e-3, 10)
+
+    def element():
+        el = T.GPU_FEAT4_Data(conn.shape[0], len(x))
+        el.Initialize()
+        el.SetNodalFixed(fixed)
+        el.SetExternalForce(f)
+        el.Setup(*(np.array([v]) for v in point), np.array([1.0 / 6.0]), x, y, z, conn)
+        el.SetDensity(1000.0)
+        el.SetDamping(0.0, 0.0)
+        el.SetSVK(1e7, 0.3)
+        el.CalcDnDuPre()
+        el.CalcMassMatrix()
+        el.CalcConstraintData()
+        el.ConvertToCSR_ConstraintJacT()
+        el.SetForcePrecision(prec)
+        return el
+
+    def moved(cls, params, mode):
+        el = element()
+        s = cls(el, el.get_n_constraint())
+        s.Setup()
+        s.SetParameters(params)
+        s.SetMode(mode)
+        for _ in range(2):
+            s.Solve()
+        out = np.stack(el.RetrievePositionToCPU()) - np.stack([x, y, z])
+        del s
+        el.Destroy()
+        return out
+
+    ref = moved(T.SyncedNesterovSolver, nesterov, "persistent")
+    assert rel(moved(T.SyncedNesterovSolver, nesterov, "auto"), ref) < tol
+    assert rel(moved(T.SyncedAdamWSolver, adamw, "auto"), moved(T.SyncedAdamWSolver, adamw, "persistent")) < tol
+    if prec == "fp64":  # (sequences have FP64 forces)
+        el = element()
+        b = T.BatchedDynamics(el, 2)
+        b.SetMaterial(np.array([1e7, 1e7]), np.array([0.3, 0.3]))
+        b.SetParameters(nesterov, 0.0)
+        for _ in range(2):
+            b.Step(T.BatchedDynamics.WARM_PREVIOUS)
+        assert rel(np.stack(b.RetrievePositions(1)) - np.stack([x, y, z]), ref) < tol
+        b.Destroy()
+        el.Destroy()
+
+
 @pytest.mark.parametrize("cells", [(9, 3, 2), (130, 10, 10)])
 def test_first_order_fp32_forces_on_straight_elements(cells):
     """Element forces in FP32 against the oracle: the solvers' bar for FP32 forces, 1e-4 of the

@@ -222,7 +222,8 @@ inline LinRule lin_rule(const tlfea_element_s* h) {
     return r;
 }
 
-// Whether the element's rule has the symmetric form the straight-sided arithmetic assumes.
+// Whether the element's rule has the form the straight-sided arithmetic assumes: for TET4 any
+// point will do (svk_element takes its mass from the point itself).
 inline bool rule_is_symmetric(const tlfea_element_s* h) {
     if (h->npe != 10) return true;
     const double tol = 4e-16;

@@ -7,13 +7,15 @@
 namespace tlfea {
 
 // The rule and its mass moments for the nonlinear element: point 0 the centroid (weight w0),
-// points 1..4 L = (a, b, b, b) and its permutations (weight w1); TET4: w0 its one weight.
-// Mass moments m = sum_q w_q N_a N_b, per unit rho det J, of the pairs (vertex, itself),
+// points 1..4 L = (a, b, b, b) and its permutations (weight w1); TET4: w0 and L its one point,
+// anywhere (the force does not depend on it, the mass does).
+// TET10's mass moments m = sum_q w_q N_a N_b, per unit rho det J, of the pairs (vertex, itself),
 // (vertex, other vertex), (vertex, its edge), (vertex, edge not at it), (edge, itself),
 // (edge, edge sharing a vertex), (edge, opposite edge).
 struct SvkRule {
     double a, b, w0, w1;
     double vv, vw, ve, vf, ee, ea, eo;
+    double L[4];
 };
 
 // Rows of F (FP64, from positions) or H = F - I (FP32, from displacements) at the vertices:
@@ -206,10 +208,11 @@ __device__ __forceinline__ void svk_element(const R (&ji)[9], R det, R lam, R mu
 #pragma unroll
                 for (int a = 0; a < 4; ++a) {
                     m[a] = R(w(a, c));
-                    sv += m[a];
+                    sv += R(rule.L[a]) * m[a];
                 }
+                sv *= R(rule.w0) * det;
 #pragma unroll
-                for (int a = 0; a < 4; ++a) f[a] = R(rule.vw) * det * sv + R(rule.vv - rule.vw) * det * m[a];
+                for (int a = 0; a < 4; ++a) f[a] = R(rule.L[a]) * sv;
             }
         } else {
 #pragma unroll
@@ -246,8 +249,7 @@ inline SvkRule svk_rule(const tlfea_element_s* h) {
     const QpBary q = qp_bary(h);
     r.w0 = h->qw[0];
     if (h->npe != 10) {
-        r.vv = r.w0 * q.L[0][0] * q.L[0][0];
-        r.vw = r.w0 * q.L[0][0] * q.L[0][1];
+        for (int k = 0; k < 4; ++k) r.L[k] = q.L[0][k];
         return r;
     }
     r.a = q.L[1][0];
