@@ -316,6 +316,52 @@ def test_mass_of_linear_elements_follows_the_point(point, prec, tol):
         el.Destroy()
 
 
+# 9 tiles resident, 610 in launches whose graphs are kept from solve to solve
+@pytest.mark.parametrize("cells", [(9, 3, 2), (130, 10, 10)])
+def test_density_changed_between_solves(cells):
+    """The second solve from rest equals a fresh solver's at the new density, bit for bit."""
+    x, y, z, conn = box(*cells, 10)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (10.0, 20.0, -50.0))
+    out = []
+    for first in (1000.0, 3000.0):
+        el = make_element(x, y, z, conn, rho=first, fixed=fixed, f_ext=f)
+        s = T.SyncedNesterovSolver(el, el.get_n_constraint())
+        s.SetParameters(T.SyncedNesterovParams(1.0e-5, 1e8, 0.0, 0.0, 2, 8, 1.0e-3))
+        for rho in ((first, 3000.0) if first != 3000.0 else (3000.0,)):
+            el.SetDensity(rho)
+            el.CalcMassMatrix()
+            el.ResetPositions()
+            s.Setup()
+            s.Solve()
+        out.append(np.stack(el.RetrievePositionToCPU()))
+        del s
+        el.Destroy()
+    assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("damped", [False, True])
+def test_density_and_damping_changed_between_steps_of_sequences(damped):
+    x, y, z, conn = box(9, 3, 2, 10)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (10.0, 20.0, -50.0))
+    last = (3000.0, 2.0e3 if damped else 0.0)
+    out = []
+    for first in ((1000.0, 1.0e3 if damped else 0.0), last):
+        el = make_element(x, y, z, conn, rho=first[0], fixed=fixed, f_ext=f, eta=first[1])
+        b = T.BatchedDynamics(el, 3)
+        b.SetMaterial(np.array([1e7, 3e6, 2e7]), np.array([0.3, 0.25, 0.35]))
+        b.SetParameters(T.SyncedNesterovParams(1.0e-6, 1e8, 0.0, 0.0, 2, 8, 1.0e-3), 0.0)
+        for rho, eta in ((first, last) if first != last else (last,)):
+            el.SetDensity(rho)
+            el.SetDamping(eta, 0.0)
+            el.CalcMassMatrix()
+            b.Reset()
+            b.Step()
+        out.append([np.stack(b.RetrievePositions(s)) for s in range(3)])
+        b.Destroy()
+        el.Destroy()
+    assert np.array_equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("cells", [(9, 3, 2), (130, 10, 10)])
 def test_first_order_fp32_forces_on_straight_elements(cells):
     """Element forces in FP32 against the oracle: the solvers' bar for FP32 forces, 1e-4 of the

@@ -591,6 +591,7 @@ struct tlfea_dynbatch_s {
     int chunk = 8;
     cudaGraphExec_t graph = nullptr;
     bool graph_straight = false;  // the force kernel of the captured graph
+    double graph_el[3] = {};      // density, damping: what it bakes in of the element
     int beta_n = -1;
 };
 
@@ -742,15 +743,17 @@ int enqueue_iteration(tlfea_dynbatch_s* b, cudaStream_t stream) {
     return TLFEA_OK;
 }
 
-// A CUDA graph of `chunk` inner iterations, built on first use after the parameters last
-// changed (the kernels' arguments are baked into it).
+// A CUDA graph of `chunk` inner iterations, built on first use after the parameters, or the
+// element's density or damping, last changed (the kernels' arguments are baked into it).
 int ensure_graph(tlfea_dynbatch_s* b) {
     const bool straight = use_straight(b);
-    if (b->graph && b->graph_straight != straight) {
+    const double now[3] = {b->el->rho, b->el->eta_d, b->el->lambda_d};
+    if (b->graph && (b->graph_straight != straight || !std::equal(now, now + 3, b->graph_el))) {
         cudaGraphExecDestroy(b->graph);
         b->graph = nullptr;
     }
     b->graph_straight = straight;
+    std::copy(now, now + 3, b->graph_el);
     b->D.mass_scale = b->el->rho / b->np.time_step;
     if (b->graph) return TLFEA_OK;
     cudaStream_t stream = b->el->stream;

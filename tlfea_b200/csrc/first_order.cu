@@ -1053,11 +1053,13 @@ static int run_phased_straight(tlfea_solver_s* s, const FOArgs& S, cudaStream_t 
     FOCtl* C = static_cast<FOCtl*>(s->fo_ctl);
     const SeqForceArgs<R> A = fos_force_args<R>(s);
     const FOStraight Q{s->fo_x4, s->fo_w4, s->fo_slots, el->tl.node_soff, el->rho / S.dt};
-    std::vector<unsigned char> key(sizeof(int) + sizeof(S) + sizeof(A));
+    static_assert(sizeof(FOStraight) == 5 * 8, "no padding: the key compares its bytes");
+    std::vector<unsigned char> key(sizeof(int) + sizeof(S) + sizeof(A) + sizeof(Q));
     const int variant = 64 | (sizeof(R) == 4 ? 1 : 0) | (NPE == 10 ? 2 : 0);
     memcpy(key.data(), &variant, sizeof(int));
     memcpy(key.data() + sizeof(int), &S, sizeof(S));
     memcpy(key.data() + sizeof(int) + sizeof(S), &A, sizeof(A));
+    memcpy(key.data() + sizeof(int) + sizeof(S) + sizeof(A), &Q, sizeof(Q));
     const int gn = std::max(1, std::min(s->max_blocks / 4, (S.N + FO_NODE_THREADS - 1) / FO_NODE_THREADS));
     if (key != s->fo_graph_key) {
         first_order_drop_graphs(s);
