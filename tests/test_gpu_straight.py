@@ -14,6 +14,7 @@ import pytest
 import scipy.sparse as sp
 
 import tlfea_b200 as T
+from tlfea_b200 import _capi as capi
 from oracle import oracle as O
 from tlfea_b200 import mesh as M
 
@@ -443,4 +444,87 @@ def test_batched_operator_and_iterates_on_straight_elements(shared, n, order):
         if order == 10:
             assert rel(us[k], O.cg(off, cols, kv, fb, 0.0, 20)[0]) < 1e-9
         o += xv.size
+    b.Destroy()
+
+
+# ---------------------------------------------------------------- waits that run out
+def late(fn, *args):
+    """The call reports the error word of an expired wait, once."""
+    with pytest.raises(T.TLFEAError, match="BUDGET_EXCEEDED"):
+        fn(*args)
+
+
+# static solves: resident (9 tiles), in launches per phase (610 tiles), on the assembled K; explicit steps
+@pytest.mark.parametrize("cells,operator", [((9, 3, 2), "auto"), ((130, 10, 10), "auto"), ((9, 3, 2), "assembled")])
+def test_static_solves_report_an_expired_wait(cells, operator):
+    import torch
+
+    x, y, z, conn = box(*cells, 10)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (0.0, 3.0, -100.0))
+    el = make_element(x, y, z, conn, fixed=fixed, f_ext=f, mass=False)
+    s = T.LinearStaticSolver(el, 1e-10, 25)
+    s.SetOperator(operator)
+    capi.call("tlfea_test_expire_wait", el._handle())
+    late(s.Solve)
+    assert np.array_equal(np.stack(el.RetrievePositionToCPU()), np.stack([x, y, z]))
+    s.Solve()
+    assert s.GetLastIterCount() == 25
+    if operator == "auto":
+        v = torch.zeros(3 * len(x), dtype=torch.float64, device="cuda")
+        w = torch.empty_like(v)
+        torch.cuda.synchronize()
+        capi.call("tlfea_test_expire_wait", el._handle())
+        late(s.Apply, v.data_ptr(), w.data_ptr())
+        s.Apply(v.data_ptr(), w.data_ptr())
+    del s
+    el.Destroy()
+
+
+@pytest.mark.parametrize("cells", [(9, 3, 2), (130, 10, 10)])
+def test_steps_report_an_expired_wait(cells):
+    x, y, z, conn = box(*cells, 10)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (10.0, 20.0, -50.0))
+    params = T.SyncedNesterovParams(1.0e-6, 1e8, 0.0, 0.0, 1, 8, 1.0e-3)
+    el = make_element(x, y, z, conn, fixed=fixed, f_ext=f)
+    s = T.SyncedNesterovSolver(el, el.get_n_constraint())
+    s.Setup()
+    s.SetParameters(params)
+    capi.call("tlfea_test_expire_wait", el._handle())
+    late(s.Solve)
+    s.Solve()
+    capi.call("tlfea_test_expire_wait", el._handle())
+    late(s.RunSteps, 2)
+    b = T.BatchedDynamics(el, 2)
+    b.SetMaterial(np.array([1e7, 5e6]), np.array([0.3, 0.3]))
+    b.SetParameters(params, 0.0)
+    capi.call("tlfea_test_expire_wait", el._handle())
+    late(b.Step)
+    b.Step()
+    b.Destroy()
+    del s
+    el.Destroy()
+
+
+@pytest.mark.parametrize("mode,prec", [("phased", "fp64"), ("phased", "fp32"), ("persistent", "fp64"),
+                                       ("persistent", "fp32")])
+@pytest.mark.parametrize("shared", [False, True])
+def test_batches_report_an_expired_wait(shared, mode, prec):
+    import torch
+
+    d = M.random_beam(300, nx_range=(6, 14), ny_range=(2, 4), order=10)
+    b = T.BatchedLinearStaticSolver([(d["x"], d["y"], d["z"], d["conn"])] * 3, T.TYPE_T10, shared=shared)
+    b.SetMaterial([1e7] * 3, [0.3] * 3)
+    b.SetNodalFixed([d["fixed"]] * 3)
+    b.SetExternalForce([d["f"]] * 3)
+    b.SetMode(mode)
+    b.SetPrecision(prec)
+    capi.call("tlfea_test_expire_batch_wait", b._h)
+    late(b.Solve, 1e-6, 2000)
+    b.Solve(1e-6, 2000)
+    assert not b.GetResults()[2].any()
+    v = torch.zeros(3 * b.n_nodes, dtype=torch.float64, device="cuda")
+    w = torch.empty_like(v)
+    torch.cuda.synchronize()
+    capi.call("tlfea_test_expire_batch_wait", b._h)
+    late(b.Apply, v.data_ptr(), w.data_ptr())
     b.Destroy()

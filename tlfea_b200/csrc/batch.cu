@@ -1353,6 +1353,8 @@ static int blin_phased(tlfea_batch_s* b, double tol, int max_iter, bool warm, cu
         TLFEA_LAUNCHED(3 * chunk + 1);
         TLFEA_CUDA(cudaMemcpyAsync(ctl, b->n_done, 2 * sizeof(int), cudaMemcpyDeviceToHost, st));
         TLFEA_CUDA(cudaStreamSynchronize(st));
+        const int late = element_check_error(b->el);
+        if (late) return late;
         if (ctl[0] >= b->n_inst || ctl[1] >= max_iter) break;
     }
     k_bl_finish<R><<<(b->n_inst + 127) / 128, 128, 0, st>>>(A);
@@ -1920,7 +1922,7 @@ int tlfea_batch_solve(tlfea_batch b, double tol, int max_iter) {
                                 : bcg_run(b, false, 0, tol, max_iter, b->warm, st)))
             return s;
         TLFEA_CUDA(cudaStreamSynchronize(st));
-        return TLFEA_OK;
+        return element_check_error(b->el);
     }
     // FP32 element work, FP64 verdict: iterative refinement on the correction
     // equation.  Each pass evaluates the true residual r = f - K u with the FP64
@@ -1948,6 +1950,7 @@ int tlfea_batch_solve(tlfea_batch b, double tol, int max_iter) {
         int nd = 0;
         TLFEA_CUDA(cudaMemcpyAsync(&nd, b->n_done, sizeof(int), cudaMemcpyDeviceToHost, st));
         TLFEA_CUDA(cudaStreamSynchronize(st));
+        if ((s = element_check_error(b->el))) return s;
         if (nd >= b->n_inst || pass == MAX_PASSES) break;
         // u (the FP64 kernel's copy of the evaluation point) is the accumulated solution
         TLFEA_CUDA(cudaMemcpyAsync(b->uacc, b->u, n3 * sizeof(double), cudaMemcpyDeviceToDevice, st));
@@ -1966,6 +1969,13 @@ int tlfea_batch_solve(tlfea_batch b, double tol, int max_iter) {
     }
     TLFEA_CUDA(cudaStreamSynchronize(st));
     b->refined = true;
+    return TLFEA_OK;
+}
+
+// Not in the header: the batch's error word as a kernel sets it whose bounded wait ran out (tests).
+int tlfea_test_expire_batch_wait(tlfea_batch b) {
+    CHECK_BATCH(b);
+    *b->el->h_err = 3;
     return TLFEA_OK;
 }
 
@@ -2025,7 +2035,7 @@ int tlfea_batch_apply(tlfea_batch b, const double* d_x, double* d_y) {
 #undef TLFEA_BLIN_APPLY
         if (s) return s;
         TLFEA_CUDA(cudaStreamSynchronize(st));
-        return TLFEA_OK;
+        return element_check_error(b->el);
     }
     if ((s = batch_dispatch_grid(b, 0, &grid, true))) return s;
     auto go = [&](auto tag, const void* fn, size_t smem) -> int {

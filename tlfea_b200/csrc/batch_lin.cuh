@@ -93,7 +93,8 @@ __device__ __forceinline__ void bl_init_barriers(uint32_t bar) {
 }
 
 // K p over the tiles of the instances that are running in iteration `it` (skip = false: of
-// all).  `loads` counts the table loads of this block since bl_init_barriers.  The work of a
+// all).  `loads` counts the table loads of this block since bl_init_barriers; -1 from the first
+// table on that did not land: the block does no more products.  The work of a
 // block is a sequence of units (item, instance); the next unit's p (and, where the tile
 // changes, its tables and geometry) are in flight while the current one is computed.
 template <typename R, int NPE, bool SH>
@@ -162,7 +163,7 @@ __device__ __forceinline__ void bl_tiles(const BLinArgs<R>& A, int it, bool skip
     };
     int item = blockIdx.x, inst = 0;
     seek(item, inst);
-    if (item >= n_items) return;
+    if (item >= n_items || loads < 0) return;
     int tile = item % A.n_tiles;
     int nl = A.node_off[tile + 1] - A.node_off[tile];
     if (t == 0) {
@@ -174,8 +175,8 @@ __device__ __forceinline__ void bl_tiles(const BLinArgs<R>& A, int it, bool skip
     bool fresh = true;  // this unit's tables are still on their way
     while (item < n_items) {
         const int load = loads;
-        if (fresh && !(mbar_wait(bar0 + 8 * (load & 1), (load >> 1) & 1) && mbar_wait(bar0 + 16, load & 1)))
-            atomicExch(A.err, 3);
+        const bool landed =
+            !fresh || (mbar_wait(bar0 + 8 * (load & 1), (load >> 1) & 1) && mbar_wait(bar0 + 16, load & 1));
         const unsigned char* tab = smem + L.tab + (load & 1) * L.tab_bytes;
         const uint16_t* incs = reinterpret_cast<const uint16_t*>(tab + L.inc);
         const uint16_t* lcs = reinterpret_cast<const uint16_t*>(smem + L.lconn);
@@ -206,7 +207,13 @@ __device__ __forceinline__ void bl_tiles(const BLinArgs<R>& A, int it, bool skip
         const bool more = item2 < n_items;
         const int tile2 = more ? item2 % A.n_tiles : tile;
         const bool swap = more && item2 != item;
-        __syncthreads();  // p staged; the other table buffer's readers are past it
+        // p staged; the other table buffer's readers are past it
+        if (!__syncthreads_and(landed)) {
+            tables_late(A.err, bar0 + 8 * (load & 1), (load >> 1) & 1);
+            mbar_wait(bar0 + 16, load & 1);
+            loads = -1;
+            return;
+        }
         if (swap && t == 0) issue(tile2, load + 1);
         {
             int lc[NPE];
@@ -480,6 +487,13 @@ __device__ __forceinline__ void bl_finish(const BLinArgs<R>& A) {
     }
 }
 
+// Products are missing: every instance counts as ended (called where n_done may grow; the host
+// reads the error word).
+template <typename R>
+__device__ __forceinline__ void bl_end_if_late(const BLinArgs<R>& A, int loads) {
+    if (loads < 0 && threadIdx.x == 0) atomicMax(A.n_done, A.n_inst);
+}
+
 // ---- one launch per phase (mode 0).  Iteration j of a captured chunk is *base + j; a phase
 // past the cap, or that finds every instance done, returns.  n_done only grows in the phases
 // after their own test of it matters (an instance that ends in the direction phase still gets
@@ -499,6 +513,7 @@ __global__ void __launch_bounds__(TILE_ELEMS, 4) k_bl_tiles(BLinArgs<R> A, const
     bl_init_barriers(smem_u32(smem + BLinLayout<R, NPE>(A.max_local).bar));
     int loads = 0;
     bl_tiles<R, NPE, SH>(A, it, skip != 0, smem, loads);
+    if (skip) bl_end_if_late(A, loads);
 }
 template <typename R>
 __global__ void __launch_bounds__(TILE_ELEMS) k_bl_start(BLinArgs<R> A, int warm) {
@@ -573,6 +588,7 @@ __global__ void __launch_bounds__(TILE_ELEMS, 4) k_bl_cg(BLinArgs<R> A, double t
     bl_residual(A, warm);
     grid.sync();
     bl_init(A, tol);
+    bl_end_if_late(A, loads);
     grid.sync();
     for (int it = 0; it < max_iter; ++it) {
         if (__ldcg(A.n_done) >= A.n_inst) break;  // uniform: read after a grid barrier, grows before one
@@ -581,6 +597,7 @@ __global__ void __launch_bounds__(TILE_ELEMS, 4) k_bl_cg(BLinArgs<R> A, double t
         bl_update(A, it);
         grid.sync();
         bl_direction(A, it, tol, max_iter);
+        bl_end_if_late(A, loads);
         grid.sync();
     }
     bl_finish(A);

@@ -1101,6 +1101,7 @@ int tlfea_dynbatch_step(tlfea_dynbatch b, int warm_start, const double* d_v_gues
             TLFEA_LAUNCHED(3 * b->chunk);
             TLFEA_CUDA(cudaMemcpyAsync(b->h_counters, b->counters, sizeof(int), cudaMemcpyDeviceToHost, stream));
             TLFEA_CUDA(cudaStreamSynchronize(stream));
+            if ((st = element_check_error(el))) return st;
             if (b->h_counters[0] >= b->B) break;
         }
         k_dyn_outer<<<grid, DYN_NODE_THREADS, 0, stream>>>(b->D, b->outer_done, el->fixed, (int)el->h_fixed.size(),

@@ -1160,13 +1160,13 @@ static void give_error_word(int* w) {
 }
 
 // A kernel's bounded wait ran out: report it once and clear the word.
-static int check_device_error(tlfea_element_s* h) {
+int element_check_error(tlfea_element_s* h) {
     // host memory that the kernels see (they write it only then): after the caller's
     // synchronisation this is a plain read, where a copy back cost a force call 8 us
     const int e = *static_cast<volatile int*>(h->h_err);
     if (e) {
         *h->h_err = 0;
-        set_error("a pipeline wait in the force kernel ran out (code " + std::to_string(e) + ")");
+        set_error("a bounded wait in a kernel ran out (code " + std::to_string(e) + ")");
         return TLFEA_BUDGET_EXCEEDED;
     }
     return TLFEA_OK;
@@ -1227,7 +1227,7 @@ using namespace tlfea;
     do {                                                           \
         if ((h)->blocking) {                                       \
             TLFEA_CUDA(cudaStreamSynchronize((h)->stream));        \
-            int st_err_ = check_device_error(h);                   \
+            int st_err_ = element_check_error(h);                   \
             if (st_err_) return st_err_;                           \
         }                                                          \
     } while (0)
@@ -1323,6 +1323,13 @@ int tlfea_element_set_stream(tlfea_element h, void* stream) {
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
     h->own_stream = false;
     h->stream = (cudaStream_t)stream;
+    return TLFEA_OK;
+}
+
+// Not in the header: the error word as a kernel sets it whose bounded wait ran out (tests).
+int tlfea_test_expire_wait(tlfea_element h) {
+    CHECK_HANDLE(h);
+    *h->h_err = 3;
     return TLFEA_OK;
 }
 

@@ -981,6 +981,9 @@ namespace tlfea {
 int element_build_pattern(tlfea_element_s* h);
 int element_force(tlfea_element_s* h, const double* d_v, bool fp32);
 int element_refresh_nodes(tlfea_element_s* h, bool displacements);
+// TLFEA_BUDGET_EXCEEDED if a kernel's bounded wait ran out (reported once); after a synchronisation
+// with the element's stream, a plain read of host memory.
+int element_check_error(tlfea_element_s* h);
 // Rebuild the tile-ordered node record (FP64 positions, or FP32 mode displacements) if stale.
 int element_refresh_record(tlfea_element_s* h, bool fp32);
 

@@ -844,13 +844,14 @@ __global__ void __launch_bounds__(FO_NODE_THREADS) k_fos_outer_start(FOArgs S, F
 
 template <typename R, int NPE>
 __global__ void __launch_bounds__(TILE_ELEMS, NPE != 10 || sizeof(R) == 4 ? 4 : 3)
-    k_fos_force(SeqForceArgs<R> A, const FOCtl* C) {
+    k_fos_force(SeqForceArgs<R> A, FOCtl* C) {
     extern __shared__ __align__(128) unsigned char smem[];
     asm volatile("griddepcontrol.launch_dependents;");
     sf_init_barriers(smem_u32(smem + SForceLayout<R, NPE>(A.T.max_local, true).bar));
     asm volatile("griddepcontrol.wait;" ::: "memory");
     if (__ldcg(&C->mode) != FO_INNER) return;
-    seq_force_tiles<R, NPE>(A, smem, [](int) { return true; });
+    // forces are missing: the loop ends without moving the positions (the host reads the error word)
+    if (!seq_force_tiles<R, NPE>(A, smem, [](int) { return true; }) && threadIdx.x == 0) C->mode = FO_DONE;
 }
 
 template <typename R>
@@ -1079,7 +1080,7 @@ static int run_phased_straight(tlfea_solver_s* s, const FOArgs& S, cudaStream_t 
             for (int j = 0; j < parts[k] && e == cudaSuccess; ++j) {
                 e = launch_next(k_fos_outer_start<R>, go, FO_NODE_THREADS, 0, st, S, Q, C);
                 for (int n = 0; n < FOS_INNER && e == cudaSuccess; ++n) {
-                    e = launch_next(force, gf, TILE_ELEMS, smem, st, A, (const FOCtl*)C);
+                    e = launch_next(force, gf, TILE_ELEMS, smem, st, A, C);
                     if (e == cudaSuccess) e = launch_next(k_fos_node<R>, gn, FO_NODE_THREADS, 0, st, S, Q, C);
                 }
                 if (e == cudaSuccess) e = launch_next(k_fos_outer, go, FO_NODE_THREADS, 0, st, S, C);
@@ -1113,6 +1114,8 @@ static int run_phased_straight(tlfea_solver_s* s, const FOArgs& S, cudaStream_t 
         int mode = 0;
         TLFEA_CUDA(cudaMemcpyAsync(&mode, &C->mode, sizeof(int), cudaMemcpyDeviceToHost, st));
         TLFEA_CUDA(cudaStreamSynchronize(st));
+        const int late = element_check_error(el);
+        if (late) return late;
         if (mode == FO_DONE) break;
         if (parts > max_parts) {
             set_error("first-order solve: the per-phase loop did not finish within its iteration bounds");
@@ -1390,6 +1393,7 @@ static int straight_steps(tlfea_solver_s* s, const FOArgs& S0, int n_steps, cons
         set_error(std::string("first-order solve: ") + cudaGetErrorString(e != cudaSuccess ? e : es));
         return TLFEA_CUDA_ERROR;
     }
+    if ((st = element_check_error(el))) return st;
     if (bar[1]) {
         set_error("first-order solve: a wait between its blocks ran out");
         return TLFEA_BUDGET_EXCEEDED;

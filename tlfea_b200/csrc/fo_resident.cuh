@@ -100,7 +100,11 @@ __global__ void __launch_bounds__(BT, BT >= 384 ? 1 : (BT >= 192 ? 2 : (sizeof(R
         bulk_g2s(smem_u32(gid), T.pad_gid + pb, bytes, bar0 + 8);
     }
     bool fine = mbar_wait(bar0, 0);
-    fine = mbar_wait(bar0 + 8, 0) && fine;
+    fine = __syncthreads_and(mbar_wait(bar0 + 8, 0) && fine);
+    if (!fine) {  // (the block leaves below; its copies get one more wait)
+        mbar_wait(bar0, 0);
+        mbar_wait(bar0 + 8, 0);
+    }
     const int nl = T.node_off[tile + 1] - T.node_off[tile];
     const int ob = Q.own_off[tile], no = Q.own_off[tile + 1] - ob;
     const int* own = Q.own_gid + ob;
@@ -375,7 +379,10 @@ __global__ void __launch_bounds__(BT, BT >= 384 ? 1 : (BT >= 192 ? 2 : (sizeof(R
             outer_flag = 1;
         }
     }
-    if (!fine && t == 0) *Q.fail = 1;
+    if (!fine) {  // a bounded wait ran out: the positions stay
+        if (t == 0) *Q.fail = 1;
+        return;
+    }
     // final positions x = x_prev + dt v, the force of the last evaluation
     for (int o = t; o < no; o += BT) {
         const int i = own[o];

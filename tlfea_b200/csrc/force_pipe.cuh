@@ -54,6 +54,14 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     return false;
 }
 
+// A table that has not landed when its bounded wait ends: the block records it, gives its copies
+// one more such wait and leaves (the decision is the block's, taken at its next barrier; nothing
+// of the table is read before).
+__device__ __forceinline__ void tables_late(int* err, uint32_t bar, uint32_t parity) {
+    if (threadIdx.x == 0) atomicExch(err, 3);
+    mbar_wait(bar, parity);
+}
+
 // 1-D bulk copy global -> shared, completion counted on `bar` (16-byte aligned
 // addresses, size a multiple of 16).
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {

@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(TILE_ELEMS, sizeof(R) == 4 ? (DAMP ? 3 : 4) : 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     gather(tile, nl);
     for (int it = 0; tile < T.n_tiles; ++it) {
-        if (!mbar_wait(bar0 + 8 * (it & 1), (it >> 1) & 1)) atomicExch(T.err, 3);
+        const bool landed = mbar_wait(bar0 + 8 * (it & 1), (it >> 1) & 1);
         const unsigned char* tab = smem + L.tab + (it & 1) * L.tab_bytes;
         const uint16_t* incs = reinterpret_cast<const uint16_t*>(tab + L.inc);
         const uint16_t* lcs = reinterpret_cast<const uint16_t*>(tab + L.lconn);
@@ -174,7 +174,11 @@ __global__ void __launch_bounds__(TILE_ELEMS, sizeof(R) == 4 ? (DAMP ? 3 : 4) : 
                 }
             }
         }
-        __syncthreads();  // values staged; the other table buffer's readers are past it
+        // values staged; the other table buffer's readers are past it
+        if (!__syncthreads_and(landed)) {
+            tables_late(T.err, bar0 + 8 * (it & 1), (it >> 1) & 1);
+            return;
+        }
         const int next = tile + gridDim.x;
         if (t == 0 && next < T.n_tiles) sf_issue<R, NPE>(T, L, smem, next, it + 1);
         {
@@ -229,9 +233,10 @@ struct SeqForceArgs {
 };
 
 // Forces and the mass term over the tiles and the running sequences.  A block's work is a
-// sequence of units (item, sequence), an item a tile and a group of sequences.
+// sequence of units (item, sequence), an item a tile and a group of sequences.  False (in every
+// thread) if a table did not land.
 template <typename R, int NPE, typename Run>
-__device__ __forceinline__ void seq_force_tiles(const SeqForceArgs<R>& A, unsigned char* smem, Run running) {
+__device__ __forceinline__ bool seq_force_tiles(const SeqForceArgs<R>& A, unsigned char* smem, Run running) {
     constexpr int TE = TILE_ELEMS, NB = NPE == 10 ? 3 : 1;  // node values in flight per thread
     const int t = threadIdx.x;
     const SForceTables<R>& T = A.T;
@@ -265,7 +270,7 @@ __device__ __forceinline__ void seq_force_tiles(const SeqForceArgs<R>& A, unsign
     };
     int item = blockIdx.x, seq = 0, load = 0;
     seek(item, seq);
-    if (item >= n_items) return;
+    if (item >= n_items) return true;
     int tile = item / groups;
     int nl = T.node_off[tile + 1] - T.node_off[tile];
     if (t == 0) sf_issue<R, NPE>(T, L, smem, tile, 0);
@@ -273,7 +278,7 @@ __device__ __forceinline__ void seq_force_tiles(const SeqForceArgs<R>& A, unsign
     gather(tile, seq, nl);
     bool fresh = true;
     while (item < n_items) {
-        if (fresh && !mbar_wait(bar0 + 8 * (load & 1), (load >> 1) & 1)) atomicExch(T.err, 3);
+        const bool landed = !fresh || mbar_wait(bar0 + 8 * (load & 1), (load >> 1) & 1);
         const unsigned char* tab = smem + L.tab + (load & 1) * L.tab_bytes;
         const uint16_t* incs = reinterpret_cast<const uint16_t*>(tab + L.inc);
         const uint16_t* lcs = reinterpret_cast<const uint16_t*>(tab + L.lconn);
@@ -305,7 +310,11 @@ __device__ __forceinline__ void seq_force_tiles(const SeqForceArgs<R>& A, unsign
         const bool more = item2 < n_items, swap = more && item2 != item;
         const int tile2 = more ? item2 / groups : tile;
         const R lam = A.lam_s ? R(__ldg(A.lam_s + seq)) : A.lambda, mu = A.lam_s ? R(__ldg(A.mu_s + seq)) : A.mu;
-        __syncthreads();  // values staged; the other table buffer's readers are past it
+        // values staged; the other table buffer's readers are past it
+        if (!__syncthreads_and(landed)) {
+            tables_late(T.err, bar0 + 8 * (load & 1), (load >> 1) & 1);
+            return false;
+        }
         if (swap && t == 0) sf_issue<R, NPE>(T, L, smem, tile2, load + 1);
         {
             int lc[NPE];
@@ -339,6 +348,7 @@ __device__ __forceinline__ void seq_force_tiles(const SeqForceArgs<R>& A, unsign
         seq = seq2;
         tile = tile2;
     }
+    return true;
 }
 
 // A node's slots [b, e) summed in tile order, two in flight.

@@ -233,7 +233,8 @@ __global__ void __launch_bounds__(BT, 512 / BT) k_lin_cg(LinArgs A) {
     const int* own_gid = A.own_gid + ob;
     const uint16_t* own_ln = A.own_ln + ob;
     __syncthreads();  // barrier initialised
-    bool fine = mbar_wait(bar, 0);
+    bool fine = __syncthreads_and(mbar_wait(bar, 0));
+    if (!fine) mbar_wait(bar, 0);  // (the block leaves below; its copies get one more wait)
     for (int k = t; k < 3 * nl; k += BT) ps[k] = 0.0;
     // owned nodes: r = f, u = 0
     double s = 0.0;
@@ -419,7 +420,7 @@ __global__ void __launch_bounds__(TILE_ELEMS, 4) k_lin_tiles(LinArgs A, int* err
     int it = 0;
     for (int tile = blockIdx.x; tile < A.n_tiles; tile += gridDim.x, ++it) {
         const unsigned char* tab = smem + L.tab + (it & 1) * L.tab_bytes;
-        if (!mbar_wait(bar0 + 8 * (it & 1), (it >> 1) & 1)) atomicExch(err, 3);
+        const bool landed = mbar_wait(bar0 + 8 * (it & 1), (it >> 1) & 1);
         if (done) return;  // (the copy in flight has landed)
         const uint16_t* incs = reinterpret_cast<const uint16_t*>(tab + L.inc);
         const uint16_t* lcs = reinterpret_cast<const uint16_t*>(tab + L.lconn);
@@ -438,7 +439,15 @@ __global__ void __launch_bounds__(TILE_ELEMS, 4) k_lin_tiles(LinArgs A, int* err
 #pragma unroll
             for (int d = 0; d < 3; ++d) ps[3 * ln + d] = pv[0][d];
         }
-        __syncthreads();  // p staged; the other table buffer's readers are past it
+        // p staged; the other table buffer's readers are past it
+        if (!__syncthreads_and(landed)) {
+            if (t == 0) {
+                ctl->status = 3;
+                ctl->done = 1;  // ends the solve: this launch sets no alpha
+            }
+            tables_late(err, bar0 + 8 * (it & 1), (it >> 1) & 1);
+            return;
+        }
         const int next = tile + gridDim.x;
         if (t == 0 && next < A.n_tiles) {
             lin_issue_tables<NPE, true>(A, next, smem + L.tab + ((it + 1) & 1) * L.tab_bytes, L,

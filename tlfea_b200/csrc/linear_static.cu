@@ -717,6 +717,7 @@ static int assemble_k(tlfea_solver_s* s, const double* x, const double* y, const
 // The result of a solve and UpdatePositions.
 static int finish_solve(tlfea_solver_s* s, const CgCtl& h) {
     tlfea_element_s* el = s->el;
+    if (int st = element_check_error(el)) return st;  // (the stream is drained: h was read)
     if (h.status == 1) {
         set_error("LinearStaticSolver CG: non-positive p*Kp detected; aborting.");
         // the reference leaves last_iter_count = max_iter and residual = 1 on breakdown
@@ -936,6 +937,7 @@ static int lin_solve(tlfea_solver_s* s, bool* solved) {
         TLFEA_LAUNCHED(3LL * LIN_CHUNK[k]);
         launched += LIN_CHUNK[k];
     }
+    if ((rc = element_check_error(el))) return rc;
     if (h.status == 3 || (resident && !h.done)) {
         set_error("LinearStaticSolver CG: a wait between its blocks ran out");
         return TLFEA_BUDGET_EXCEEDED;
@@ -1063,8 +1065,9 @@ int linear_static_apply(tlfea_solver_s* s, const double* d_x, double* d_y) {
         TLFEA_LAUNCHED(1);
         k_lin_collect<<<(el->N + 255) / 256, 256, 0, st>>>(A, d_x, d_y);
         TLFEA_CHECK_LAUNCH();
-        if (el->blocking) TLFEA_CUDA(cudaStreamSynchronize(st));
-        return TLFEA_OK;
+        if (!el->blocking) return TLFEA_OK;
+        TLFEA_CUDA(cudaStreamSynchronize(st));
+        return element_check_error(el);
     }
     if (s->mf_last) {
         // matrix-free, at the positions of the last solve (its tangent stream); the
@@ -1073,8 +1076,9 @@ int linear_static_apply(tlfea_solver_s* s, const double* d_x, double* d_y) {
         TLFEA_CUDA(cudaMemsetAsync(s->ctl_apply, 0, sizeof(CgCtl), el->stream));
         if (launch_mf_apply(s, el->stream, d_x, d_y, s->ctl_apply)) return TLFEA_CUDA_ERROR;
         TLFEA_LAUNCHED(3);
-        if (el->blocking) TLFEA_CUDA(cudaStreamSynchronize(el->stream));
-        return TLFEA_OK;
+        if (!el->blocking) return TLFEA_OK;
+        TLFEA_CUDA(cudaStreamSynchronize(el->stream));
+        return element_check_error(el);
     }
     k_cg_spmv_dot<<<cg_grid(s), 256, 0, el->stream>>>(el->N, el->pat_off, el->pat_col, s->K, d_x, d_y, s->cg_part,
                                                       s->ctl_apply);
