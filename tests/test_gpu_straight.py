@@ -82,6 +82,48 @@ def test_linear_solve_on_the_linear_operator(cells, order):
     el.Destroy()
 
 
+@pytest.mark.parametrize("change", ["material", "mooney", "damping", "reference", "fixed"])
+def test_operator_of_the_last_solve_outlives_changes_to_the_element(change):
+    """Apply and the stiffness matrix are the last solve's, whatever the element was given since."""
+    import torch
+
+    x, y, z, conn = box(9, 3, 2, 10)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (1.0, 5.0, -20.0))
+    x, y, z = jitter(x, y, z, conn, 0.002)
+    off, cols, kv, _ = oracle_k(x, y, z, conn, f, fixed)
+    el = make_element(x, y, z, conn, fixed=fixed, f_ext=f, mass=False)
+    s = T.LinearStaticSolver(el, 1e-10, 20000)
+    s.Solve()
+    if change == "material":
+        el.SetSVK(3e6, 0.2)
+    elif change == "mooney":
+        el.SetMooneyRivlin(1e6, 2e5, 5e7)
+    elif change == "damping":
+        el.SetDamping(10.0, 5.0)
+    elif change == "reference":
+        el.UpdatePositions(1.1 * x, y, z)
+        el.CalcDnDuPre()
+        det = el.RetrieveDetJToCPU()
+    else:
+        el.UpdateNodalFixed(fixed[:3])
+    xv = torch.tensor(np.random.default_rng(2).standard_normal(f.size), dtype=torch.float64, device="cuda")
+    yv = torch.empty_like(xv)
+    torch.cuda.synchronize()
+    s.Apply(xv.data_ptr(), yv.data_ptr())
+    torch.cuda.synchronize()
+    K = sp.csr_matrix((kv, cols, off), shape=(f.size, f.size))
+    assert rel(yv.cpu().numpy(), K @ xv.cpu().numpy()) < 1e-11
+    o2, c2, v2 = s.RetrieveStiffnessCSRToCPU()
+    assert np.array_equal(o2, off) and np.array_equal(c2, cols) and rel(v2, kv) < 1e-11
+    if change == "reference":  # and the element's geometry is the new one
+        assert np.array_equal(el.RetrieveDetJToCPU(), det)
+        el.ResetPositions()
+        el.ComputeInternalForce()
+        assert np.linalg.norm(el.RetrieveInternalForceToCPU()) < 1e-6
+    del s
+    el.Destroy()
+
+
 # 592 resident tiles of 128 elements: 75,776 elements; on either side of it
 @pytest.mark.parametrize("cells", [(120, 10, 10), (130, 10, 10)])
 def test_resident_and_phased_forms_agree_at_a_fixed_count(cells):

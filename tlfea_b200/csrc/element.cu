@@ -1037,6 +1037,24 @@ int element_refresh_nodes(tlfea_element_s* h, bool displacements) {
     return TLFEA_OK;
 }
 
+// The per-point geometry (gradients, weights, J^-1, det J) of the mesh at the given positions.
+int element_geometry_at(tlfea_element_s* h, const double* x, const double* y, const double* z) {
+    QuadParams qp;
+    memcpy(qp.qx, h->qx, sizeof(qp.qx));
+    memcpy(qp.qy, h->qy, sizeof(qp.qy));
+    memcpy(qp.qz, h->qz, sizeof(qp.qz));
+    memcpy(qp.qw, h->qw, sizeof(qp.qw));
+    const int n_slots = h->tl.n_tiles * TILE_ELEMS;
+    const long long nt = (long long)n_slots * h->nqp;
+    const unsigned blocks = (unsigned)((nt + 127) / 128);
+    Tiling& tl = h->tl;
+    auto kern = h->npe == 10 ? k_dndu_pre<10, 5> : k_dndu_pre<4, 1>;
+    kern<<<blocks, 128, 0, h->stream>>>(n_slots, h->E, tl.tile_elem, h->d_conn, x, y, z, qp, tl.grad64, tl.grad32,
+                                        tl.dv64, tl.dv32, h->detJ, tl.ji64, tl.ji32);
+    TLFEA_CHECK_LAUNCH();
+    return TLFEA_OK;
+}
+
 // f_int (FP64) or f_int32 (FP32) = internal force at the current positions.
 // Asynchronous on h->stream (the solvers call it inside their loops).
 int element_force(tlfea_element_s* h, const double* d_v, bool fp32) {
@@ -1549,24 +1567,10 @@ int tlfea_element_update_constraint_targets(tlfea_element h, const double* x, co
 int tlfea_element_calc_dndu_pre(tlfea_element h) {
     CHECK_HANDLE(h);
     REQUIRE_SETUP(h);
-    QuadParams qp;
-    memcpy(qp.qx, h->qx, sizeof(qp.qx));
-    memcpy(qp.qy, h->qy, sizeof(qp.qy));
-    memcpy(qp.qz, h->qz, sizeof(qp.qz));
-    memcpy(qp.qw, h->qw, sizeof(qp.qw));
-    const int n_slots = h->tl.n_tiles * TILE_ELEMS;
-    const long long nt = (long long)n_slots * h->nqp;
-    const unsigned blocks = (unsigned)((nt + 127) / 128);
     Tiling& tl = h->tl;
-    if (h->npe == 10)
-        k_dndu_pre<10, 5><<<blocks, 128, 0, h->stream>>>(n_slots, h->E, tl.tile_elem, h->d_conn, h->x, h->y, h->z, qp,
-                                                        tl.grad64, tl.grad32, tl.dv64, tl.dv32, h->detJ,
-                                                        tl.ji64, tl.ji32);
-    else
-        k_dndu_pre<4, 1><<<blocks, 128, 0, h->stream>>>(n_slots, h->E, tl.tile_elem, h->d_conn, h->x, h->y, h->z, qp,
-                                                       tl.grad64, tl.grad32, tl.dv64, tl.dv32, h->detJ,
-                                                        tl.ji64, tl.ji32);
-    TLFEA_CHECK_LAUNCH();
+    const int n_slots = tl.n_tiles * TILE_ELEMS;
+    if (int st = element_geometry_at(h, h->x, h->y, h->z)) return st;
+    h->geometry_version++;
     const size_t nb = (size_t)h->N * sizeof(double);
     TLFEA_CUDA(cudaMemcpyAsync(h->X0x, h->x, nb, cudaMemcpyDeviceToDevice, h->stream));
     TLFEA_CUDA(cudaMemcpyAsync(h->X0y, h->y, nb, cudaMemcpyDeviceToDevice, h->stream));

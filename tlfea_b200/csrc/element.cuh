@@ -960,6 +960,7 @@ struct tlfea_element_s {
     int* d_err = nullptr;  // the same word as the kernels see it
     // grid of the persistent force pipeline per (FP32?, damping?), 0 = not yet sized
     int pipe_grid[4] = {0, 0, 0, 0};
+    long long geometry_version = 0;  // CalcDnDuPre calls
     int straight_grid[8] = {};  // the same of the straight-sided force kernel
     // launch configuration (tlfea_element_set_launch_config): force kernel 0 = gradient stream,
     // 1 = one tile per block, 2 = persistent pipeline, 3 = compact stream; -1 (until the caller
@@ -981,6 +982,7 @@ namespace tlfea {
 int element_build_pattern(tlfea_element_s* h);
 int element_force(tlfea_element_s* h, const double* d_v, bool fp32);
 int element_refresh_nodes(tlfea_element_s* h, bool displacements);
+int element_geometry_at(tlfea_element_s* h, const double* x, const double* y, const double* z);
 // TLFEA_BUDGET_EXCEEDED if a kernel's bounded wait ran out (reported once); after a synchronisation
 // with the element's stream, a plain read of host memory.
 int element_check_error(tlfea_element_s* h);

@@ -536,8 +536,8 @@ static MfArgs mf_args(tlfea_solver_s* s, const double* p, double* q, CgCtl* ctl)
     M.prec = s->mf_prec;
     M.pfix = s->mf_pfix;
     M.tile_dot = s->mf_part;
-    M.lambda = el->lambda;
-    M.mu = el->mu;
+    M.lambda = s->op.lambda;
+    M.mu = s->op.mu;
     M.qb = qp_bary(el);
     M.ctl = ctl;
     return M;
@@ -643,6 +643,8 @@ static int build_cg_graph(tlfea_solver_s* s, int iters) {
     s->cg_graph_iters = iters;
     s->cg_graph_precond = s->precond;
     s->cg_graph_mf = use_matrix_free(s) ? 1 : 0;
+    s->cg_graph_lame[0] = s->op.lambda;
+    s->cg_graph_lame[1] = s->op.mu;
     return TLFEA_OK;
 }
 
@@ -698,15 +700,16 @@ static int assemble_k(tlfea_solver_s* s, const double* x, const double* y, const
     tlfea_element_s* el = s->el;
     cudaStream_t stream = el->stream;
     const int N = el->N;
-    const bool mr = (el->material == TLFEA_MATERIAL_MOONEY_RIVLIN);
+    const tlfea_solver_s::Operator& op = s->op;
+    const bool mr = (op.material == TLFEA_MATERIAL_MOONEY_RIVLIN);
     auto kern = (el->npe == 10) ? (mr ? k_stiffness_rows<10, 5, true> : k_stiffness_rows<10, 5, false>)
                                 : (mr ? k_stiffness_rows<4, 1, true> : k_stiffness_rows<4, 1, false>);
     kern<<<(N + 127) / 128, 128, 0, stream>>>(N, el->E, el->d_conn, x, y, z, el->tl.elem_slot, el->tl.grad64,
                                                el->tl.dv64, el->inc_off, el->inc_e, el->inc_a, el->pat_off,
-                                               el->pat_col, s->K, el->lambda, el->mu, el->eta_d, el->lambda_d, 1.0,
-                                               el->mu10, el->mu01, el->kappa);
+                                               el->pat_col, s->K, op.lambda, op.mu, op.eta_d, op.lambda_d, 1.0,
+                                               op.mu10, op.mu01, op.kappa);
     TLFEA_CHECK_LAUNCH();
-    if (el->n_constraint > 0) {
+    if (op.fixed) {
         k_apply_bcs<<<(N + 255) / 256, 256, 0, stream>>>(N, el->pat_off, el->pat_col, s->is_fixed, s->K, s->f);
         TLFEA_CHECK_LAUNCH();
     }
@@ -793,8 +796,8 @@ static LinArgs lin_args(tlfea_solver_s* s, CgCtl* ctl) {
     A.r = s->r;
     A.slots = s->lin_slots;
     A.part = s->lin_part;
-    A.lambda = el->lambda;
-    A.mu = el->mu;
+    A.lambda = s->op.lambda;
+    A.mu = s->op.mu;
     A.tol = s->tol;
     A.max_iter = s->max_iter;
     A.rule = lin_rule(el);
@@ -960,6 +963,8 @@ int linear_static_solve(tlfea_solver_s* s) {
     if (st) return st;
     cudaStream_t stream = el->stream;
     const int N = el->N, n3 = 3 * N;
+    s->op = {el->material, el->lambda, el->mu,    el->eta_d,            el->lambda_d,
+             el->mu10,     el->mu01,   el->kappa, el->n_constraint > 0, el->geometry_version};
     // the right-hand side and the Dirichlet DOFs
     TLFEA_CUDA(cudaMemcpyAsync(s->f, el->f_ext, sizeof(double) * n3, cudaMemcpyDeviceToDevice, stream));
     TLFEA_CUDA(cudaMemsetAsync(s->is_fixed, 0, n3, stream));
@@ -1032,7 +1037,8 @@ int linear_static_solve(tlfea_solver_s* s) {
         TLFEA_CUDA(cudaStreamSynchronize(stream));
         if (h.done || launched >= s->max_iter) break;
         if (!s->cg_graph || s->cg_graph_iters != chunk || s->cg_graph_precond != s->precond ||
-            s->cg_graph_mf != (mf ? 1 : 0)) {
+            s->cg_graph_mf != (mf ? 1 : 0) || s->cg_graph_lame[0] != s->op.lambda ||
+            s->cg_graph_lame[1] != s->op.mu) {
             if ((st = build_cg_graph(s, chunk))) return st;
         }
         TLFEA_CUDA(cudaGraphLaunch(s->cg_graph, stream));
@@ -1041,6 +1047,21 @@ int linear_static_solve(tlfea_solver_s* s) {
         if (chunk < 64) chunk *= 2;
     }
     return finish_solve(s, h);
+}
+
+// K of the last solve, which did not assemble it, at that solve's positions and material.  A solve
+// on the linear operator ran at its reference configuration: if the element has another one by now,
+// the geometry at the solve's positions is formed for the assembly and the present one again after
+// it, and the products go by K from then on.
+static int assemble_last(tlfea_solver_s* s) {
+    tlfea_element_s* el = s->el;
+    const bool other = s->lin_last && s->op.geometry != el->geometry_version;
+    int st = prepare_k(s);
+    if (!st && other) st = element_geometry_at(el, s->xk, s->yk, s->zk);
+    if (!st) st = assemble_k(s, s->xk, s->yk, s->zk);
+    if (!st && other) st = element_geometry_at(el, el->X0x, el->X0y, el->X0z);
+    if (!st && other) s->lin_last = false;
+    return st;
 }
 
 int linear_static_apply(tlfea_solver_s* s, const double* d_x, double* d_y) {
@@ -1053,6 +1074,10 @@ int linear_static_apply(tlfea_solver_s* s, const double* d_x, double* d_y) {
         int st = dalloc(&s->ctl_apply, 1);
         if (st) return st;
         TLFEA_CUDA(cudaMemsetAsync(s->ctl_apply, 0, sizeof(CgCtl), el->stream));
+    }
+    if (s->lin_last && s->op.geometry != el->geometry_version) {
+        int st = assemble_last(s);
+        if (st) return st;
     }
     if (s->lin_last) {
         cudaStream_t st = el->stream;
@@ -1091,10 +1116,7 @@ int linear_static_retrieve_k(tlfea_solver_s* s, long long* nnz, int* offsets, in
     tlfea_element_s* el = s->el;
     TLFEA_CUDA(cudaStreamSynchronize(el->stream));
     if (!s->k_built && (s->mf_last || s->lin_last)) {
-        // the last solve did not assemble K: do it at its positions now
-        int st = prepare_k(s);
-        if (st) return st;
-        st = assemble_k(s, s->xk, s->yk, s->zk);
+        int st = assemble_last(s);
         if (st) return st;
         TLFEA_CUDA(cudaStreamSynchronize(el->stream));
     }

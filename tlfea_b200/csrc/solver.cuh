@@ -88,7 +88,16 @@ struct tlfea_solver_s {
     double* mf_prec = nullptr;     // p in the node record's tile order (3 per padded slot)
     uint16_t* mf_pfix = nullptr;   // fixed-DOF flags per padded slot
     double* mf_tan = nullptr;      // F and S per element QP at the last solve's positions
-    double *xk = nullptr, *yk = nullptr, *zk = nullptr;  // positions of the last matrix-free solve
+    double *xk = nullptr, *yk = nullptr, *zk = nullptr;  // positions of the last solve without K
+    // the operator of the last solve, for Apply and for K on demand: the element's material,
+    // whether it had fixed nodes, its geometry
+    struct Operator {
+        int material;
+        double lambda, mu, eta_d, lambda_d, mu10, mu01, kappa;
+        bool fixed;
+        long long geometry;
+    } op{};
+    double cg_graph_lame[2] = {0, 0};  // the material the captured graph was built for
     bool lin_last = false;       // the last solve ran on the linear operator (lin_cg.cuh)
     double* lin_slots = nullptr;  // 4 per node slot
     double* lin_p = nullptr;      // 4 per node: p, or the resident solve's r
