@@ -426,6 +426,35 @@ def test_first_order_fp32_forces_on_straight_elements(cells):
     el.Destroy()
 
 
+def test_fp32_forces_in_the_solver_are_no_further_off_than_per_point():
+    """60 Nesterov iterations with FP32 forces against the FP64 solver on the per-point kernels: the mean
+    distance over four meshes is no larger than the per-point FP32 kernels'."""
+    err = {"auto": [], "persistent": []}
+    for seed in range(4):
+        x, y, z, conn = box(20, 4, 4, 10)
+        fixed, f, _ = M.cantilever_loads(x, y, z, (50.0, 0.0, 0.0))
+        x, y, z = jitter(x, y, z, conn, 0.0025, seed)
+
+        def run(mode, prec):
+            el = make_element(x, y, z, conn, fixed=fixed, f_ext=f)
+            el.SetForcePrecision(prec)
+            s = T.SyncedNesterovSolver(el, el.get_n_constraint())
+            s.Setup()
+            s.SetParameters(T.SyncedNesterovParams(5.0e-5, 1e8, 0.0, 0.0, 1, 60, 1.0e-3))
+            s.SetMode(mode)
+            s.Solve()
+            out = np.stack(el.RetrievePositionToCPU()) - np.stack([x, y, z])
+            del s
+            el.Destroy()
+            return out
+
+        exact = run("persistent", "fp64")
+        assert np.linalg.norm(exact) < 1e-2 * np.linalg.norm(np.stack([x, y, z]))  # a stable step size
+        for mode, e in err.items():
+            e.append(rel(run(mode, "fp32"), exact))
+    assert np.mean(err["auto"]) <= np.mean(err["persistent"]), err
+
+
 # ---------------------------------------------------------------- batches
 # the group sizes of the launch (1, 2, 4, 8 sequences a block) and their remainders
 @pytest.mark.parametrize("n,cells,order", [(1, (8, 4, 2), 10), (2, (9, 3, 2), 10), (5, (3, 2, 2), 10),
