@@ -599,3 +599,20 @@ def test_batches_report_an_expired_wait(shared, mode, prec):
     capi.call("tlfea_test_expire_batch_wait", b._h)
     late(b.Apply, v.data_ptr(), w.data_ptr())
     b.Destroy()
+
+
+def test_elements_beyond_the_shared_page_have_words_of_their_own():
+    """512 elements share a page of host words; the ones after it, and one in it, report for themselves."""
+    x, y, z, conn = box(1, 1, 1, 4)
+    crowd = [T.GPU_FEAT4_Data(conn.shape[0], len(x)) for _ in range(511)]
+    for el in crowd:
+        el.Initialize()
+    els = [make_element(x, y, z, conn, mass=False) for _ in range(3)]
+    for k in range(3):
+        capi.call("tlfea_test_expire_wait", els[k]._handle())
+        for j in range(3):
+            if j == k:
+                late(els[j].ComputeInternalForce)
+            els[j].ComputeInternalForce()
+    for el in crowd + els:
+        el.Destroy()

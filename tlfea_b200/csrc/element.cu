@@ -2,9 +2,9 @@
 // mass CSR and constraints behind the C ABI (include/tlfea_b200.h).
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <fstream>
-#include <mutex>
 #include <mutex>
 #include <numeric>
 #include <vector>
@@ -1122,14 +1122,16 @@ static int noalloc_scratch(int device, double** out) {
     return TLFEA_OK;
 }
 
-// Error words of the elements alive: one pinned page that every device sees, taken with the
-// process's first element and kept (a pinned allocation takes 2 to 4 ms, more than the rest of a
-// small element's setup), a word per element; past its 1024 words, an allocation per element.  The
-// page is asked for again if it went with its context (cudaDeviceReset).
+// Host words of the elements alive, which every device sees: an element's error word and the flag
+// of its straight-sided geometry.  One page, pinned with the process's first element and kept
+// (pinning it takes 0.3 ms, a pinned allocation of the runtime's 1.2 to 2.1); past its 512 elements,
+// an allocation per element.  The page is pinned again if that went with its context
+// (cudaDeviceReset).
 struct ErrorPage {
-    static constexpr int WORDS = 1024;
+    static constexpr int ELEMENTS = 512, WORDS = 2 * ELEMENTS;
     std::mutex lock;
-    int* base = nullptr;
+    int* base = nullptr;  // pinned
+    int* page = nullptr;
     std::vector<int> free;
 };
 static ErrorPage g_error_page;
@@ -1153,17 +1155,25 @@ static int* take_error_word() {
     }
     if (!P.base) {
         P.free.clear();
-        if ((P.base = pinned_words(ErrorPage::WORDS)))
-            for (int i = ErrorPage::WORDS; i-- > 0;) P.free.push_back(i);
+        constexpr size_t bytes = ErrorPage::WORDS * sizeof(int);
+        if (!P.page) P.page = static_cast<int*>(std::aligned_alloc(4096, bytes));
+        if (P.page && cudaHostRegister(P.page, bytes, cudaHostRegisterMapped | cudaHostRegisterPortable) == cudaSuccess) {
+            P.base = P.page;
+        } else {
+            cudaGetLastError();
+            P.base = pinned_words(ErrorPage::WORDS);
+        }
+        if (P.base)
+            for (int i = ErrorPage::ELEMENTS; i-- > 0;) P.free.push_back(2 * i);
     }
     int* w = nullptr;
     if (!P.free.empty()) {
         w = P.base + P.free.back();
         P.free.pop_back();
     } else {
-        w = pinned_words(1);
+        w = pinned_words(2);
     }
-    if (w) *w = 0;
+    if (w) w[0] = w[1] = 0;
     return w;
 }
 
@@ -1577,35 +1587,19 @@ int tlfea_element_calc_dndu_pre(tlfea_element h) {
     TLFEA_CUDA(cudaMemcpyAsync(h->X0z, h->z, nb, cudaMemcpyDeviceToDevice, h->stream));
     // straight-sided meshes: the one-Jacobian geometry beside the per-point streams
     tl.straight = false;
-    const bool rule_ok = rule_is_symmetric(h);
-    int curved = 1;
-    if (rule_ok) {
-        int* d_curved = nullptr;
-        int st = dalloc(&d_curved, 1);
-        if (st) return st;
-        cudaError_t ec = cudaMemsetAsync(d_curved, 0, sizeof(int), h->stream);
-        const unsigned gb = (unsigned)((n_slots + 127) / 128);
-        if (h->npe == 10)
-            k_straight_geo<10><<<gb, 128, 0, h->stream>>>(n_slots, h->E, tl.tile_elem, h->d_conn, h->x, h->y, h->z,
-                                                         tl.geo64, tl.geo32, d_curved);
-        else
-            k_straight_geo<4><<<gb, 128, 0, h->stream>>>(n_slots, h->E, tl.tile_elem, h->d_conn, h->x, h->y, h->z,
-                                                        tl.geo64, tl.geo32, d_curved);
-        if (ec == cudaSuccess) ec = cudaGetLastError();
-        TLFEA_LAUNCHED(1);
-        if (ec == cudaSuccess)
-            ec = cudaMemcpyAsync(&curved, d_curved, sizeof(int), cudaMemcpyDeviceToHost, h->stream);
-        if (ec == cudaSuccess) ec = cudaStreamSynchronize(h->stream);
-        dfree(d_curved);
-        if (ec != cudaSuccess) {
-            set_error(std::string("calc_dndu_pre: ") + cudaGetErrorString(ec));
-            return TLFEA_CUDA_ERROR;
-        }
+    volatile int* curved = h->h_err + 1;
+    *curved = 1;
+    if (rule_is_symmetric(h)) {
+        *curved = 0;  // (nothing that sets it is in flight: this call synchronises)
+        auto geo = h->npe == 10 ? k_straight_geo<10> : k_straight_geo<4>;
+        geo<<<(unsigned)((n_slots + 127) / 128), 128, 0, h->stream>>>(n_slots, h->E, tl.tile_elem, h->d_conn, h->x, h->y,
+                                                                      h->z, tl.geo64, tl.geo32, h->d_err + 1);
+        TLFEA_CHECK_LAUNCH();
     }
-    tl.straight = (curved == 0);
     positions_changed(h);
     h->precomputed = true;
     SYNC(h);
+    tl.straight = *curved == 0;
     return TLFEA_OK;
 }
 

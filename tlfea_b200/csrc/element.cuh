@@ -956,8 +956,8 @@ struct tlfea_element_s {
     double* j_val = nullptr;
 
     // error word set by kernels whose bounded waits ran out (checked at sync points)
-    int* h_err = nullptr;  // pinned
-    int* d_err = nullptr;  // the same word as the kernels see it
+    int* h_err = nullptr;  // pinned, two words: the second, CalcDnDuPre's flag of a curved mesh
+    int* d_err = nullptr;  // the same words as the kernels see them
     // grid of the persistent force pipeline per (FP32?, damping?), 0 = not yet sized
     int pipe_grid[4] = {0, 0, 0, 0};
     long long geometry_version = 0;  // CalcDnDuPre calls
