@@ -179,8 +179,8 @@ int tlfea_element_set_force_precision(tlfea_element h, int precision);
  * slices of the gradient stream, 1 = one tile per block with direct loads, 2 =
  * persistent producer/consumer pipeline, 3 = as 0 on the compact geometry stream
  * (J^-1 and dV per QP, gradients formed in registers); grid_limit caps the
- * persistent grid (0 = all resident blocks).  An element that was never given a
- * configuration takes one J^-1 per element where the mesh allows it (SVK,
+ * persistent grid (0 = all resident blocks).  -1, the configuration of an element
+ * that was never given one: one J^-1 per element where the mesh allows it (SVK,
  * mid-edge nodes at their edges' midpoints), else kernel 0. */
 int tlfea_element_set_launch_config(tlfea_element h, int force_kernel, int grid_limit);
 

@@ -250,6 +250,26 @@ def test_internal_force_of_straight_elements(cells, order, prec, tol):
     el.Destroy()
 
 
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_default_force_kernel_can_be_chosen_again(prec):
+    x, y, z, conn = box(9, 3, 2, 10)
+    el = make_element(x, y, z, conn, mass=False)
+    el.SetForcePrecision(prec)
+    el.UpdatePositions(*perturb(x, y, z, 1e-3, 6))
+    el.ComputeInternalForce()
+    first = el.RetrieveInternalForceToCPU()
+    out = []
+    for kernel in ("tma", "auto"):
+        el.SetLaunchConfig(kernel)
+        el.ComputeInternalForce()
+        out.append(el.RetrieveInternalForceToCPU())
+    assert np.array_equal(out[1], first) and not np.array_equal(out[0], first)
+    for bad in (-2, 4):
+        with pytest.raises(T.TLFEAError):
+            el.SetLaunchConfig(bad)
+    el.Destroy()
+
+
 def test_internal_force_beside_orphans_and_of_curved_elements():
     x, y, z, conn = box(5, 2, 2, 10)
     r = np.random.default_rng(5)
