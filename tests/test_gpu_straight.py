@@ -538,6 +538,36 @@ def test_batched_operator_and_iterates_on_straight_elements(shared, n, order):
     b.Destroy()
 
 
+def test_batches_on_straight_elements_hold_one_set_of_buffers():
+    """Against the same batch on a curved mesh, which runs the general kernels: a shared batch takes no more
+    memory; sequences take less than 96 bytes a node more, which two records of 32 and at least one slot of 32
+    a node would be beside the general buffers."""
+    import torch
+
+    x, y, z, conn = box(40, 8, 8, 10)
+    yc = y.copy()
+    edge = np.unique(conn[:, 4:])
+    yc[edge] += 1e-4 * np.random.default_rng(5).uniform(-1, 1, edge.size)
+    n = 64 * len(x)
+
+    def used(create):
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        b = create()
+        took = free - torch.cuda.mem_get_info()[0]
+        b.Destroy()
+        return took
+
+    shared, sequences = [], []
+    for ys in (y, yc):
+        el = make_element(x, ys, z, conn)
+        shared.append(used(lambda: T.BatchedLinearStaticSolver([(x, ys, z, conn)] * 64, T.TYPE_T10, shared=True)))
+        sequences.append(used(lambda: T.BatchedDynamics(el, 64)))
+        el.Destroy()
+    assert shared[0] <= shared[1]
+    assert sequences[0] - sequences[1] < 96 * n
+
+
 # ---------------------------------------------------------------- waits that run out
 def late(fn, *args):
     """The call reports the error word of an expired wait, once."""

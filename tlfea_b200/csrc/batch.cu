@@ -1482,6 +1482,51 @@ static std::vector<unsigned char> untouched_nodes(const tlfea_batch_s* b) {
     return fx;
 }
 
+// The state of the straight-sided phases (batch_lin.cuh), b->lin; where the mesh does not allow
+// them, or they do not fit (they take 80 bytes a node, the general phases 48 and, on a shared mesh,
+// 36 a shared node and tile), the general phases serve.
+static int batch_alloc_lin(tlfea_batch_s* b) {
+    const int n_inst = b->n_inst;
+    const Tiling& tl = b->el->tl;
+    const long long lin_slots = tl.n_local_total * (b->shared ? n_inst : 1);
+    if (!tl.straight || BLinLayout<double, 10>(tl.max_local_pad).total > 200 * 1024 || lin_slots >= (1LL << 31))
+        return TLFEA_OK;
+    std::vector<int> tp, ip((size_t)n_inst + 1, 0), ni;
+    size_t pairs = 0;
+    if (b->shared) {
+        for (int i = 0; i <= n_inst; ++i) ip[i] = i * tl.n_tiles;
+        pairs = (size_t)n_inst * tl.n_tiles;
+    } else {
+        std::vector<int> ti(2 * (size_t)tl.n_tiles);
+        TLFEA_CUDA(cudaMemcpy(ti.data(), b->tile_inst, ti.size() * sizeof(int), cudaMemcpyDeviceToHost));
+        tp.resize((size_t)tl.n_tiles);
+        for (int t = 0; t < tl.n_tiles; ++t) {
+            tp[t] = (int)pairs;
+            pairs += (size_t)(ti[2 * t + 1] - ti[2 * t] + 1);
+            for (int i = ti[2 * t]; i <= ti[2 * t + 1]; ++i) ip[(size_t)i + 1]++;
+        }
+        for (int i = 0; i < n_inst; ++i) ip[(size_t)i + 1] += ip[i];
+        ni.resize((size_t)b->N);
+        for (int i = 0; i < n_inst; ++i)
+            for (int n = b->node_off[i]; n < b->node_off[i + 1]; ++n) ni[n] = i;
+    }
+    if (dalloc(&b->lin_p, 4 * (size_t)b->N) || dalloc(&b->lin_slots, 4 * (size_t)lin_slots) ||
+        dalloc(&b->lin_pair, pairs) || dalloc(&b->stamp, (size_t)n_inst) || dalloc(&b->tile_pair, tp.size()) ||
+        dalloc(&b->inst_pair, ip.size()) || dalloc(&b->node_inst, ni.size())) {
+        cudaGetLastError();
+        for (double** p : {&b->lin_p, &b->lin_slots, &b->lin_pair}) dfree(*p);
+        for (int** p : {&b->stamp, &b->tile_pair, &b->inst_pair, &b->node_inst}) dfree(*p);
+        return TLFEA_OK;
+    }
+    TLFEA_CUDA(cudaMemcpy(b->inst_pair, ip.data(), ip.size() * sizeof(int), cudaMemcpyHostToDevice));
+    if (!b->shared) {
+        TLFEA_CUDA(cudaMemcpy(b->tile_pair, tp.data(), tp.size() * sizeof(int), cudaMemcpyHostToDevice));
+        TLFEA_CUDA(cudaMemcpy(b->node_inst, ni.data(), ni.size() * sizeof(int), cudaMemcpyHostToDevice));
+    }
+    b->lin = true;
+    return TLFEA_OK;
+}
+
 // Solver state of a batch whose element (tiling, gradients) is set up.
 static int batch_alloc_state(tlfea_batch_s* b) {
     const int n_inst = b->n_inst;
@@ -1490,53 +1535,20 @@ static int batch_alloc_state(tlfea_batch_s* b) {
     int st;
     if ((st = dalloc(&b->lam, nmat)) || (st = dalloc(&b->mu, nmat)) || (st = dalloc(&b->lam32, nmat)) ||
         (st = dalloc(&b->mu32, nmat)) || (st = dalloc(&b->fixed, (size_t)b->N)) || (st = dalloc(&b->u, n3)) ||
-        (st = dalloc(&b->r, n3)) || (st = dalloc(&b->p, n3)) || (st = dalloc(&b->q, n3)) ||
-        (st = dalloc(&b->f, n3)) || (st = dalloc(&b->u0, n3)) || (st = dalloc(&b->rr, 2 * (size_t)n_inst)) ||
-        (st = dalloc(&b->fnorm, (size_t)n_inst)) || (st = dalloc(&b->rel, (size_t)n_inst)) ||
+        (st = dalloc(&b->r, n3)) || (st = dalloc(&b->f, n3)) || (st = dalloc(&b->u0, n3)) ||
+        (st = dalloc(&b->rr, 2 * (size_t)n_inst)) || (st = dalloc(&b->fnorm, (size_t)n_inst)) || (st = dalloc(&b->rel, (size_t)n_inst)) ||
         (st = dalloc(&b->iters, (size_t)n_inst)) || (st = dalloc(&b->status, (size_t)n_inst)) ||
         (st = dalloc(&b->done, (size_t)n_inst)) || (st = dalloc(&b->n_done, 2)) ||
         (st = dalloc(&b->alpha, (size_t)n_inst)) || (st = dalloc(&b->beta, (size_t)n_inst)) ||
         (st = dalloc(&b->flag, (size_t)n_inst)) || (st = dalloc(&b->ticket, (size_t)n_inst)))
         return st;
-    if (b->shared) {
+    if ((st = batch_alloc_lin(b))) return st;
+    if (!b->lin && ((st = dalloc(&b->p, n3)) || (st = dalloc(&b->q, n3)))) return st;
+    if (!b->lin && b->shared) {
         const size_t np = 3 * (size_t)n_inst * (size_t)std::max(b->el->tl.n_pslots, 1);
         if ((st = dalloc(&b->part64, np)) || (st = dalloc(&b->part32, np))) return st;
     }
     cudaStream_t s = b->el->stream;
-    const Tiling& tl = b->el->tl;
-    const long long lin_slots = tl.n_local_total * (b->shared ? n_inst : 1);
-    if (tl.straight && BLinLayout<double, 10>(tl.max_local_pad).total <= 200 * 1024 && lin_slots < (1LL << 31)) {
-        std::vector<int> tp, ip((size_t)n_inst + 1, 0), ni;
-        size_t pairs = 0;
-        if (b->shared) {
-            for (int i = 0; i <= n_inst; ++i) ip[i] = i * tl.n_tiles;
-            pairs = (size_t)n_inst * tl.n_tiles;
-        } else {
-            std::vector<int> ti(2 * (size_t)tl.n_tiles);
-            TLFEA_CUDA(cudaMemcpy(ti.data(), b->tile_inst, ti.size() * sizeof(int), cudaMemcpyDeviceToHost));
-            tp.resize((size_t)tl.n_tiles);
-            for (int t = 0; t < tl.n_tiles; ++t) {
-                tp[t] = (int)pairs;
-                pairs += (size_t)(ti[2 * t + 1] - ti[2 * t] + 1);
-                for (int i = ti[2 * t]; i <= ti[2 * t + 1]; ++i) ip[(size_t)i + 1]++;
-            }
-            for (int i = 0; i < n_inst; ++i) ip[(size_t)i + 1] += ip[i];
-            ni.resize((size_t)b->N);
-            for (int i = 0; i < n_inst; ++i)
-                for (int n = b->node_off[i]; n < b->node_off[i + 1]; ++n) ni[n] = i;
-        }
-        if ((st = dalloc(&b->lin_p, 4 * (size_t)b->N)) || (st = dalloc(&b->lin_slots, 4 * (size_t)lin_slots)) ||
-            (st = dalloc(&b->lin_pair, pairs)) || (st = dalloc(&b->stamp, (size_t)n_inst)) ||
-            (st = dalloc(&b->tile_pair, tp.size())) || (st = dalloc(&b->inst_pair, ip.size())) ||
-            (st = dalloc(&b->node_inst, ni.size())))
-            return st;
-        TLFEA_CUDA(cudaMemcpy(b->inst_pair, ip.data(), ip.size() * sizeof(int), cudaMemcpyHostToDevice));
-        if (!b->shared) {
-            TLFEA_CUDA(cudaMemcpy(b->tile_pair, tp.data(), tp.size() * sizeof(int), cudaMemcpyHostToDevice));
-            TLFEA_CUDA(cudaMemcpy(b->node_inst, ni.data(), ni.size() * sizeof(int), cudaMemcpyHostToDevice));
-        }
-        b->lin = true;
-    }
     const std::vector<unsigned char> fx = untouched_nodes(b);
     TLFEA_CUDA(cudaMemcpyAsync(b->fixed, fx.data(), (size_t)b->N, cudaMemcpyHostToDevice, s));
     TLFEA_CUDA(cudaMemsetAsync(b->f, 0, n3 * sizeof(double), s));

@@ -658,6 +658,34 @@ bool use_straight(const tlfea_dynbatch_s* b) {
     return b->straight && b->el->tl.straight && b->el->eta_d == 0.0 && b->el->lambda_d == 0.0;
 }
 
+// The buffers of the force kernels that run now, the general or the straight-sided ones (a batch
+// holds both only after its damping changed).  Where the straight-sided ones, 110 bytes a node and
+// sequence, do not fit, the general kernels, 41, serve.
+int alloc_force(tlfea_dynbatch_s* b) {
+    const size_t N = b->el->N, B = b->B;
+    const Tiling& tl = b->el->tl;
+    if (use_straight(b) && !b->slots &&
+        (dalloc(&b->x4, 4 * B * N) || dalloc(&b->w4, 4 * B * N) || dalloc(&b->slots, 4 * B * (size_t)tl.n_local_total))) {
+        cudaGetLastError();
+        dfree(b->x4);
+        dfree(b->w4);
+        dfree(b->slots);
+        b->straight = false;
+    }
+    if (!use_straight(b) && !b->f) {
+        if (dalloc(&b->f, 3 * B * N) || dalloc(&b->partial, 3 * B * (size_t)std::max(tl.n_pslots, 1))) {
+            dfree(b->f);
+            return TLFEA_CUDA_ERROR;
+        }
+    }
+    b->D.x4 = b->x4;
+    b->D.w4 = b->w4;
+    b->D.slots = b->slots;
+    b->D.f = b->f;
+    b->D.partial = b->partial;
+    return TLFEA_OK;
+}
+
 template <typename... P, typename... Q>
 int launch_next(void (*kern)(P...), dim3 grid, int block, size_t smem, cudaStream_t st, Q... args) {
     cudaLaunchAttribute attr[1];
@@ -746,6 +774,7 @@ int enqueue_iteration(tlfea_dynbatch_s* b, cudaStream_t stream) {
 // A CUDA graph of `chunk` inner iterations, built on first use after the parameters, or the
 // element's density or damping, last changed (the kernels' arguments are baked into it).
 int ensure_graph(tlfea_dynbatch_s* b) {
+    if (const int rc = alloc_force(b)) return rc;
     const bool straight = use_straight(b);
     const double now[3] = {b->el->rho, b->el->eta_d, b->el->lambda_d};
     if (b->graph && (b->graph_straight != straight || !std::equal(now, now + 3, b->graph_el))) {
@@ -873,8 +902,7 @@ int tlfea_dynbatch_create(tlfea_element mesh, int n_seq, tlfea_dynbatch* out) {
     st |= dalloc(&b->x, B * N) | dalloc(&b->y, B * N) | dalloc(&b->z, B * N);
     st |= dalloc(&b->xp, B * N) | dalloc(&b->yp, B * N) | dalloc(&b->zp, B * N);
     st |= dalloc(&b->vg, B * n3) | dalloc(&b->vp, B * n3) | dalloc(&b->vk, B * n3) | dalloc(&b->g, B * n3);
-    st |= dalloc(&b->f, B * n3) | dalloc(&b->vhist, B * n3);
-    st |= dalloc(&b->partial, B * 3 * (size_t)std::max(el->tl.n_pslots, 1));
+    st |= dalloc(&b->vhist, B * n3);
     st |= dalloc(&b->lam, B * nc) | dalloc(&b->lam_s, B) | dalloc(&b->mu_s, B) | dalloc(&b->alpha_s, B);
     st |= dalloc(&b->done, B) | dalloc(&b->inner, B) | dalloc(&b->inner_total, B) | dalloc(&b->rule_met, B);
     st |= dalloc(&b->status, B) | dalloc(&b->outer_done, B) | dalloc(&b->rel, B);
@@ -885,9 +913,7 @@ int tlfea_dynbatch_create(tlfea_element mesh, int n_seq, tlfea_dynbatch* out) {
     if (el->n_constraint == 0) st |= dalloc(&b->zero_off, n3 + 1);
     const size_t straight_need = el->npe == 10 ? straight_smem<10>(el) : straight_smem<4>(el);
     b->straight = el->tl.straight && straight_need <= 200 * 1024;
-    if (b->straight)
-        st |= dalloc(&b->x4, 4 * B * N) | dalloc(&b->w4, 4 * B * N) |
-              dalloc(&b->slots, 4 * B * (size_t)el->tl.n_local_total);
+    if (!st) st = alloc_force(b);
     if (!st && cudaMallocHost((void**)&b->h_counters, sizeof(int)) != cudaSuccess) st = TLFEA_CUDA_ERROR;
     if (st) {
         dyn_free(b);
@@ -927,7 +953,7 @@ int tlfea_dynbatch_create(tlfea_element mesh, int n_seq, tlfea_dynbatch* out) {
     D.f_ext = el->f_ext;
     D.fext_norm = b->fext_norm;
     D.x = b->x; D.y = b->y; D.z = b->z; D.xp = b->xp; D.yp = b->yp; D.zp = b->zp;
-    D.vg = b->vg; D.vp = b->vp; D.vk = b->vk; D.g = b->g; D.f = b->f; D.partial = b->partial; D.lam = b->lam;
+    D.vg = b->vg; D.vp = b->vp; D.vk = b->vk; D.g = b->g; D.lam = b->lam;
     D.nc = (int)nc;
     D.lam_s = b->lam_s;
     D.mu_s = b->mu_s;
@@ -937,9 +963,6 @@ int tlfea_dynbatch_create(tlfea_element mesh, int n_seq, tlfea_dynbatch* out) {
     D.mom = b->mom;
     D.red2 = b->red2;
     D.restart = 0;
-    D.x4 = b->x4;
-    D.w4 = b->w4;
-    D.slots = b->slots;
     D.node_soff = el->tl.node_soff;
     D.n_slots = el->tl.n_local_total;
     const int per_thread = std::min(DYN_GRAD_NODES, std::max(1, bps * b->B / DYN_GRAD_FILL));

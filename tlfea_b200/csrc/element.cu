@@ -639,8 +639,6 @@ static int build_tiling(tlfea_element_s* h, const double* x, const double* y, co
     if ((st = upload(&tl.own_off, own_off, h->stream))) return st;
     if ((st = upload(&tl.own_gid, own_gid, h->stream))) return st;
     if ((st = upload(&tl.own_ln, own_ln, h->stream))) return st;
-    const size_t ngeo = (size_t)n_tiles * 10 * TE;
-    if ((st = dalloc(&tl.geo64, ngeo)) || (st = dalloc(&tl.geo32, ngeo))) return st;
     tl.straight = false;
     if ((st = dalloc(&tl.sx, (size_t)tl.n_pad)) || (st = dalloc(&tl.sy, (size_t)tl.n_pad)) ||
         (st = dalloc(&tl.sz, (size_t)tl.n_pad)))
@@ -1585,11 +1583,14 @@ int tlfea_element_calc_dndu_pre(tlfea_element h) {
     TLFEA_CUDA(cudaMemcpyAsync(h->X0x, h->x, nb, cudaMemcpyDeviceToDevice, h->stream));
     TLFEA_CUDA(cudaMemcpyAsync(h->X0y, h->y, nb, cudaMemcpyDeviceToDevice, h->stream));
     TLFEA_CUDA(cudaMemcpyAsync(h->X0z, h->z, nb, cudaMemcpyDeviceToDevice, h->stream));
-    // straight-sided meshes: the one-Jacobian geometry beside the per-point streams
+    // straight-sided meshes: the one-Jacobian geometry beside the per-point streams (where there is
+    // no memory for it the mesh counts as curved)
     tl.straight = false;
     volatile int* curved = h->h_err + 1;
     *curved = 1;
-    if (rule_is_symmetric(h)) {
+    const bool first = !tl.geo64;
+    if (rule_is_symmetric(h) &&
+        (!first || !(dalloc(&tl.geo64, 10 * (size_t)n_slots) || dalloc(&tl.geo32, 10 * (size_t)n_slots)))) {
         *curved = 0;  // (nothing that sets it is in flight: this call synchronises)
         auto geo = h->npe == 10 ? k_straight_geo<10> : k_straight_geo<4>;
         geo<<<(unsigned)((n_slots + 127) / 128), 128, 0, h->stream>>>(n_slots, h->E, tl.tile_elem, h->d_conn, h->x, h->y,
@@ -1600,6 +1601,11 @@ int tlfea_element_calc_dndu_pre(tlfea_element h) {
     h->precomputed = true;
     SYNC(h);
     tl.straight = *curved == 0;
+    if (first && !tl.straight) {  // no kernel or captured graph has seen these
+        cudaGetLastError();
+        dfree(tl.geo64);
+        dfree(tl.geo32);
+    }
     return TLFEA_OK;
 }
 

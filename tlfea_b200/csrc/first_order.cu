@@ -1026,9 +1026,15 @@ static cudaError_t launch_next(void (*kern)(P...), int grid, int block, size_t s
 static int fos_alloc(tlfea_solver_s* s) {
     if (s->fo_slots) return TLFEA_OK;
     const size_t N = s->el->N;
-    int st = dalloc(&s->fo_x4, 4 * N) | dalloc(&s->fo_w4, 4 * N) | dalloc(&s->fo_bar, 2);
-    if (!st) st = dalloc(&s->fo_slots, 4 * (size_t)s->el->tl.n_local_total);
-    return st ? TLFEA_CUDA_ERROR : TLFEA_OK;
+    if (dalloc(&s->fo_x4, 4 * N) || dalloc(&s->fo_w4, 4 * N) || dalloc(&s->fo_bar, 2) ||
+        dalloc(&s->fo_slots, 4 * (size_t)s->el->tl.n_local_total)) {
+        cudaGetLastError();
+        dfree(s->fo_x4);
+        dfree(s->fo_w4);
+        dfree(s->fo_bar);
+        return TLFEA_CUDA_ERROR;
+    }
+    return TLFEA_OK;
 }
 
 template <typename R>
@@ -1535,10 +1541,8 @@ int first_order_steps(tlfea_solver_s* s, int steps, const StepLoad* load, int* i
                   : (el->npe == 10 ? resident_column<double, 10>(s, &column) : resident_column<double, 4>(s, &column));
         if (st) return st;
         if (s->kind == KIND_NESTEROV && column == 0) column = -1;
-        if (column >= 0 || s->kind == KIND_NESTEROV) {
-            if ((st = fos_alloc(s))) return st;
+        if ((column >= 0 || s->kind == KIND_NESTEROV) && !fos_alloc(s))  // (what does not fit goes below)
             return straight_steps(s, S, n_steps, load, inner_iters, fp32, column);
-        }
     }
     // per-phase launches by default from FO_PHASED_MIN_NODES nodes: below it the host
     // round trip of each chunk outweighs the persistent kernel's latency (the 100x10x10

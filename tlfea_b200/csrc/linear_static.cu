@@ -890,9 +890,13 @@ static int lin_solve(tlfea_solver_s* s, bool* solved) {
     if (lin_smem(s, 2) > STRAIGHT_MAX_SMEM) return TLFEA_OK;  // a tile touches too many nodes: the other operators
     int rc;
     const size_t np = std::max<size_t>(2 * (size_t)el->tl.n_tiles, (size_t)lin_node_blocks(s));
-    if (!s->lin_slots && (rc = dalloc(&s->lin_slots, 4 * (size_t)el->tl.n_local_total))) return rc;
-    if (!s->lin_p && (rc = dalloc(&s->lin_p, 4 * (size_t)N))) return rc;
-    if (!s->lin_part && (rc = dalloc(&s->lin_part, np))) return rc;
+    if ((!s->lin_slots && dalloc(&s->lin_slots, 4 * (size_t)el->tl.n_local_total)) ||
+        (!s->lin_p && dalloc(&s->lin_p, 4 * (size_t)N)) || (!s->lin_part && dalloc(&s->lin_part, np))) {
+        cudaGetLastError();  // does not fit: the other operators
+        dfree(s->lin_slots);
+        dfree(s->lin_p);
+        return TLFEA_OK;
+    }
     TLFEA_CUDA(allow_tile_smem(lin_tiles_kernel()));
     if (s->lin_threads < 0) {  // the widest blocks of which every tile is resident, 0 = none
         int sms = 0, per_sm = 0, threads_fit = 0;
