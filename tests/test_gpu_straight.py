@@ -538,6 +538,26 @@ def test_batched_operator_and_iterates_on_straight_elements(shared, n, order):
     b.Destroy()
 
 
+@pytest.mark.parametrize("shared", [False, True])
+@pytest.mark.parametrize("left", [1, 2, 3])  # of 33: up to a sixteenth the node phases run on the resident blocks
+def test_instances_left_of_a_batch_iterate_as_in_a_full_one(shared, left):
+    """The others have no load and are done at once; the iterates are the same bit for bit."""
+    insts = [M.random_beam(300 + (0 if shared else i), nx_range=(6, 14), ny_range=(2, 3)) for i in range(33)]
+    b = T.BatchedLinearStaticSolver([(d["x"], d["y"], d["z"], d["conn"]) for d in insts], T.TYPE_T10, shared=shared)
+    b.SetMaterial([1e7 * (1 + 0.1 * i) for i in range(33)], [0.3] * 33)
+    b.SetNodalFixed([d["fixed"] for d in insts])
+    running = [0, 17, 32][:left]
+    out = []
+    for who in (range(33), running):
+        b.SetExternalForce([d["f"] if i in who else 0 * d["f"] for i, d in enumerate(insts)])
+        b.Solve(1e-300, 100)
+        assert [b.GetResults()[0][i] for i in running] == [100] * left
+        u = b.RetrieveDisplacement()
+        out.append([u[i] for i in running])
+    assert all(np.array_equal(p, q) for p, q in zip(*out))
+    b.Destroy()
+
+
 def test_batches_on_straight_elements_hold_one_set_of_buffers():
     """Against the same batch on a curved mesh, which runs the general kernels: a shared batch takes no more
     memory; sequences take less than 96 bytes a node more, which two records of 32 and at least one slot of 32

@@ -85,6 +85,7 @@ struct tlfea_batch_s {
         int precision, max_iter, iters;
         double tol;
         cudaGraphExec_t exec;
+        bool few = false;  // node phases on resident blocks (straight-sided batches)
     };
     std::vector<PhaseGraph> phase_graphs;
     // FP32 element work: iterations summed over the refinement passes
@@ -1310,7 +1311,19 @@ static int blin_phased(tlfea_batch_s* b, double tol, int max_iter, bool warm, cu
         const int rc = blin_tile_grid<R, NPE, SH>(b, &tile_grid);
         if (rc) return rc;
     }
-    const int chunk_grid = b->n_chunks;  // one block per chunk
+    const int chunk_grid = b->n_chunks;
+    // The node phases have a block per chunk, or, once a sixteenth of the instances or fewer run, the
+    // resident blocks: 512 instances of 40x8x8 on one mesh 1,807 us an iteration against 1,816 with
+    // all running, 329 / 283 with 64, 177 / 102 with eight, 146 / 37 with one; 512 uneven beams 834 /
+    // 944, 152 / 157, 78 / 65, 75 / 61.
+    int resident_grid[2] = {0, 0};  // update, direction
+    {
+        int sms = 0;
+        TLFEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->el->device));
+        TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident_grid[0], k_bl_update<R>, TILE_ELEMS, 0));
+        TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident_grid[1], k_bl_direction<R>, TILE_ELEMS, 0));
+        for (int& g : resident_grid) g = std::max(1, std::min(chunk_grid, g * sms));
+    }
     int* base = b->n_done + 1;
     TLFEA_CUDA(cudaMemsetAsync(b->n_done, 0, 2 * sizeof(int), st));
     k_bl_start<R><<<chunk_grid, TILE_ELEMS, 0, st>>>(A, w);
@@ -1322,18 +1335,22 @@ static int blin_phased(tlfea_batch_s* b, double tol, int max_iter, bool warm, cu
     const int prec = sizeof(R) == 4 ? TLFEA_PRECISION_FP32 : TLFEA_PRECISION_FP64;
     int ctl[2] = {0, 0};
     for (int chunk = 16; max_iter > 0; chunk = 64) {
+        const bool few = chunk > 16 && 16LL * (b->n_inst - ctl[0]) <= b->n_inst;  // (known after the first chunk)
+        const int update_grid = few ? resident_grid[0] : chunk_grid;
+        const int direction_grid = few ? resident_grid[1] : chunk_grid;
         cudaGraphExec_t ge = nullptr;
         for (auto& g : b->phase_graphs)
-            if (g.precision == prec && g.tol == tol && g.max_iter == max_iter && g.iters == chunk) ge = g.exec;
+            if (g.precision == prec && g.tol == tol && g.max_iter == max_iter && g.iters == chunk && g.few == few)
+                ge = g.exec;
         if (!ge) {
             cudaGraph_t g = nullptr;
             TLFEA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
             cudaError_t e = cudaSuccess;
             for (int j = 0; j < chunk && e == cudaSuccess; ++j) {
                 e = launch_next(tiles, tile_grid, smem, st, A, (const int*)base, j, 1, max_iter);
-                if (e == cudaSuccess) e = launch_next(k_bl_update<R>, chunk_grid, 0, st, A, (const int*)base, j, max_iter);
+                if (e == cudaSuccess) e = launch_next(k_bl_update<R>, update_grid, 0, st, A, (const int*)base, j, max_iter);
                 if (e == cudaSuccess)
-                    e = launch_next(k_bl_direction<R>, chunk_grid, 0, st, A, (const int*)base, j, tol, max_iter);
+                    e = launch_next(k_bl_direction<R>, direction_grid, 0, st, A, (const int*)base, j, tol, max_iter);
             }
             if (e == cudaSuccess) {
                 k_bl_advance<<<1, 1, 0, st>>>(base, chunk);
@@ -1347,7 +1364,7 @@ static int blin_phased(tlfea_batch_s* b, double tol, int max_iter, bool warm, cu
                 set_error("batch_solve: capture of the iteration chunk failed");
                 return TLFEA_CUDA_ERROR;
             }
-            b->phase_graphs.push_back({prec, max_iter, chunk, tol, ge});
+            b->phase_graphs.push_back({prec, max_iter, chunk, tol, ge, few});
         }
         TLFEA_CUDA(cudaGraphLaunch(ge, st));
         TLFEA_LAUNCHED(3 * chunk + 1);

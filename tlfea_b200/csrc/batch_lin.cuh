@@ -112,10 +112,13 @@ __device__ __forceinline__ void bl_tiles(const BLinArgs<R>& A, int it, bool skip
     // the first unit at or after (item, inst); item = n_items: none
     auto seek = [&](int& item, int& inst) {
         for (; item < n_items; item += gridDim.x) {
-            if constexpr (SH) {
-                const int g0 = (item / A.n_tiles) * A.group, g1 = min(g0 + A.group, A.n_inst);
-                for (inst = max(inst, g0); inst < g1; ++inst)
-                    if (running(inst)) return;
+            if constexpr (SH) {  // a lane per instance of the group (up to eight): one round trip
+                const int g0 = (item / A.n_tiles) * A.group, b = g0 + (t & 31);
+                const bool run = (t & 31) < A.group && b >= inst && b < A.n_inst && running(b);
+                if (const unsigned m = __ballot_sync(0xffffffffu, run)) {
+                    inst = g0 + __ffs(m) - 1;
+                    return;
+                }
                 inst = 0;
             } else {
                 for (int b = A.tile_inst[2 * item]; b <= A.tile_inst[2 * item + 1]; ++b)
@@ -375,14 +378,28 @@ __device__ __forceinline__ void bl_init(const BLinArgs<R>& A, double tol) {
     }
 }
 
+// f(c, b) for the block's chunks c whose instance b runs in iteration `it`.  A lane looks at a
+// chunk: a large batch of which few instances are left would spend its time on blocks and round
+// trips that find nothing to do.
+template <typename R, typename F>
+__device__ __forceinline__ void bl_running_chunks(const BLinArgs<R>& A, int it, F f) {
+    for (long long c0 = blockIdx.x; c0 < A.n_chunks; c0 += 32LL * gridDim.x) {
+        const long long c = c0 + (long long)(threadIdx.x & 31) * gridDim.x;
+        const int b = c < A.n_chunks ? A.chunk_inst[c] : 0;
+        unsigned m = __ballot_sync(0xffffffffu, c < A.n_chunks && __ldcg(A.stamp + b) > it);
+        for (; m; m &= m - 1) {  // uniform over the block: a stamp set in this phase is above `it`
+            const int k = __ffs(m) - 1;
+            f((int)(c0 + (long long)k * gridDim.x), __shfl_sync(0xffffffffu, b, k));
+        }
+    }
+}
+
 // alpha, r -= alpha q, r.r per chunk.
 template <typename R>
 __device__ __forceinline__ void bl_update(const BLinArgs<R>& A, int it) {
     const int t = threadIdx.x;
     const double* rr_old = A.rr + (size_t)(it & 1) * A.n_inst;
-    for (int c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
-        const int b = A.chunk_inst[c];
-        if (__ldcg(A.stamp + b) <= it) continue;  // uniform over the block, as every branch on b
+    bl_running_chunks(A, it, [&](int c, int b) {
         const bool first = t == 0 && c == A.inst_chunk[b];
         const double pq = bl_fold(A.pair, A.inst_pair[b], A.inst_pair[b + 1]);
         if (!(pq > 0.0)) {  // non-positive p.Kp: the reference aborts this solve
@@ -392,7 +409,7 @@ __device__ __forceinline__ void bl_update(const BLinArgs<R>& A, int it) {
                 A.stamp[b] = it + 1;
                 atomicAdd(A.n_done, 1);
             }
-            continue;
+            return;
         }
         const double alpha = __ldcg(rr_old + b) / pq;
         if (first) A.alpha[b] = alpha;
@@ -423,7 +440,7 @@ __device__ __forceinline__ void bl_update(const BLinArgs<R>& A, int it) {
         }
         s = bl_block_sum(s);
         if (t == 0) A.cpb[c] = s;
-    }
+    });
 }
 
 // The stop test and beta, u += alpha p, p = r + beta p.
@@ -431,9 +448,8 @@ template <typename R>
 __device__ __forceinline__ void bl_direction(const BLinArgs<R>& A, int it, double tol, int max_iter) {
     const int t = threadIdx.x;
     const double* rr_old = A.rr + (size_t)(it & 1) * A.n_inst;
-    for (int c = blockIdx.x; c < A.n_chunks; c += gridDim.x) {
-        const int b = A.chunk_inst[c];
-        if (__ldcg(A.stamp + b) <= it || __ldcg(A.flag + b) == 2) continue;
+    bl_running_chunks(A, it, [&](int c, int b) {
+        if (__ldcg(A.flag + b) == 2) return;
         const double alpha = __ldcg(A.alpha + b);
         const double rrn = bl_fold(A.cpb, A.inst_chunk[b], A.inst_chunk[b + 1]);
         const double rel = sqrt(rrn) / __ldcg(A.fnorm + b);
@@ -474,7 +490,7 @@ __device__ __forceinline__ void bl_direction(const BLinArgs<R>& A, int it, doubl
                             rv[j][2] + beta * pv[j][2]);
             }
         }
-    }
+    });
 }
 
 // Instances still running at the iteration cap end with status 2; the done flags.
