@@ -1,5 +1,5 @@
 """The straight-sided element paths against the oracle, at the sizes where their tiles and
-launches change: less than one tile, exactly one, a ragged last tile, the resident launch's
+launches change: tiles whole and ragged, each block width of the resident launches, their
 limit and beyond it; and the meshes that must not take them.
 
 Bars: forces and products are sums of products of the same data in another order; the
@@ -44,9 +44,11 @@ def oracle_k(x, y, z, conn, f, fixed):
     return off, cols, kv, fb
 
 
-@pytest.mark.parametrize("cells,order", [((3, 1, 1), 10), ((4, 2, 2), 10), ((9, 3, 2), 10), ((23, 5, 4), 10),
-                                         ((3, 1, 1), 4), ((31, 7, 5), 4)])
-def test_linear_solve_on_the_linear_operator(cells, order):
+# the linear operator from two tiles of quadratic elements on: two with a ragged end (252 elements), three whole
+# ones (384), three and 22 with ragged ends; one tile and linear elements keep the assembled K
+@pytest.mark.parametrize("cells,order", [((3, 1, 1), 10), ((4, 2, 2), 10), ((7, 3, 2), 10), ((8, 4, 2), 10),
+                                         ((9, 3, 2), 10), ((23, 5, 4), 10), ((3, 1, 1), 4), ((31, 7, 5), 4)])
+def test_linear_solve_from_the_reference_configuration(cells, order):
     import torch
 
     x, y, z, conn = box(*cells, order)
@@ -124,8 +126,9 @@ def test_operator_of_the_last_solve_outlives_changes_to_the_element(change):
     el.Destroy()
 
 
-# 592 resident tiles of 128 elements: 75,776 elements; on either side of it
-@pytest.mark.parametrize("cells", [(120, 10, 10), (130, 10, 10)])
+# the resident solve's blocks of 512 (a tile per SM), 256 (two) and 128 threads: 24, 197, 282, 563 tiles; beyond
+# its 592 tiles
+@pytest.mark.parametrize("cells", [(16, 8, 4), (42, 10, 10), (60, 10, 10), (120, 10, 10), (130, 10, 10)])
 def test_resident_and_phased_forms_agree_at_a_fixed_count(cells):
     x, y, z, conn = box(*cells, 10)
     fixed, f, _ = M.cantilever_loads(x, y, z, (0.0, 3.0, -100.0))
@@ -182,7 +185,26 @@ def test_stopped_solve_of_a_large_mesh_returns_the_recorded_iterate():
     el.Destroy()
 
 
-def test_curved_and_degenerate_meshes_keep_the_general_path():
+def test_phased_solve_converges_to_the_assembled_solution():
+    """Beyond the resident limit (610 tiles), at the bar of converged solves."""
+    x, y, z, conn = box(130, 10, 10, 10)
+    fixed, f, _ = M.cantilever_loads(x, y, z, (1.0, 3.0, -100.0))
+    x, y, z = jitter(x, y, z, conn, 7e-4)
+    el = make_element(x, y, z, conn, fixed=fixed, f_ext=f, mass=False)
+    out = []
+    for operator in ("auto", "assembled"):
+        s = T.LinearStaticSolver(el, 1e-10, 20000)
+        s.SetOperator(operator)
+        s.Solve()
+        assert s.GetLastResidual() < 1e-10 and s.GetLastIterCount() < 20000
+        out.append(np.stack(el.RetrievePositionToCPU()) - np.stack([x, y, z]))
+        el.ResetPositions()
+        del s
+    assert rel(out[0], out[1]) < 1e-7
+    el.Destroy()
+
+
+def test_curved_meshes_keep_the_general_path():
     x, y, z, conn = box(6, 2, 2, 10)
     fixed, f, _ = M.cantilever_loads(x, y, z, (0.0, 0.0, -20.0))
     r = np.random.default_rng(5)
@@ -250,6 +272,113 @@ def test_internal_force_of_straight_elements(cells, order, prec, tol):
     el.Destroy()
 
 
+def with_a_flat_element(x, y, z, conn):
+    """One more element, of no volume: four corners of a cell's face, mid-edge nodes at the midpoints."""
+    order = conn.shape[1]
+    face = [int(np.argmin(np.abs(x - a) + np.abs(y - b) + np.abs(z))) for a, b in
+            ((0.0, 0.0), (x.max(), 0.0), (x.max(), y.max()), (0.0, y.max()))]
+    new, xs = list(face), [x, y, z]
+    if order == 10:
+        for a, b in ((0, 1), (1, 2), (0, 2), (0, 3), (1, 3), (2, 3)):
+            new.append(len(xs[0]))
+            xs = [np.append(v, 0.5 * (v[face[a]] + v[face[b]])) for v in xs]
+    return (*xs, np.concatenate([conn, np.array([new], conn.dtype)]))
+
+
+@pytest.mark.parametrize("order", [10, 4])
+def test_degenerate_element_keeps_the_general_path(order):
+    """The default is the gradient stream's result bit for bit, and the oracle's."""
+    x, y, z, conn = with_a_flat_element(*box(9, 3, 2, order))
+    el = make_element(x, y, z, conn, mass=False)
+    xs = perturb(x, y, z, 1e-3, 6)
+    el.UpdatePositions(*xs)
+    el.ComputeInternalForce()
+    f = el.RetrieveInternalForceToCPU()
+    el.SetLaunchConfig("tma")
+    el.ComputeInternalForce()
+    assert np.array_equal(f, el.RetrieveInternalForceToCPU())
+    g, dj = O.dndu_pre(x, y, z, conn)
+    assert rel(f, O.force(*xs, conn, g, dj, LAM, MU)) < 1e-10
+    el.Destroy()
+
+
+@pytest.mark.parametrize("ulps,straight", [(0, True), (3, True), (6, False), (1e6, False)])
+def test_straight_sided_up_to_four_units_in_the_last_place(ulps, straight):
+    """One mid-edge node moved by units in the last place of its element's coordinates, which lie in
+    [0.5, 1): 2.2e-16 times the largest of them a unit."""
+    x, y, z, conn = box(9, 3, 2, 10)
+    x = 0.5 + 0.5 * x * (1 - 2 ** -30)
+    e = len(conn) - 1
+    big = x[conn[e]].max()
+    for k, (a, b) in enumerate(((0, 1), (1, 2), (0, 2), (0, 3), (1, 3), (2, 3))):
+        x[conn[:, 4 + k]] = 0.5 * (x[conn[:, a]] + x[conn[:, b]])
+    x[conn[e, 4]] += ulps * 2.220446049250313e-16 * big
+    el = make_element(x, y, z, conn, mass=False)
+    xs = perturb(x, y, z, 1e-3, 6)
+    el.UpdatePositions(*xs)
+    el.ComputeInternalForce()
+    f = el.RetrieveInternalForceToCPU()
+    el.SetLaunchConfig("tma")
+    el.ComputeInternalForce()
+    assert np.array_equal(f, el.RetrieveInternalForceToCPU()) == (not straight)
+    g, dj = O.dndu_pre(x, y, z, conn)
+    assert rel(f, O.force(*xs, conn, g, dj, LAM, MU)) < 1e-10
+    el.Destroy()
+
+
+def test_points_in_another_order_keep_the_general_path():
+    """The rule with its points permuted: the same sums, by the per-point kernels."""
+    from tlfea_b200 import quadrature as Q
+
+    x, y, z, conn = box(9, 3, 2, 10)
+    el = T.GPU_FEAT10_Data(conn.shape[0], len(x))
+    el.Initialize()
+    order = [3, 1, 0, 4, 2]
+    el.Setup(*(np.ascontiguousarray(v[order]) for v in Q.t10()), x, y, z, conn)
+    el.SetDensity(1000.0)
+    el.SetDamping(0.0, 0.0)
+    el.SetSVK(1e7, 0.3)
+    el.CalcDnDuPre()
+    xs = perturb(x, y, z, 1e-3, 6)
+    el.UpdatePositions(*xs)
+    el.ComputeInternalForce()
+    f = el.RetrieveInternalForceToCPU()
+    el.SetLaunchConfig("tma")
+    el.ComputeInternalForce()
+    assert np.array_equal(f, el.RetrieveInternalForceToCPU())
+    g, dj = O.dndu_pre(x, y, z, conn)
+    assert rel(f, O.force(*xs, conn, g, dj, LAM, MU)) < 1e-10
+    el.Destroy()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+@pytest.mark.parametrize("prec", ["fp64", "fp32"])
+def test_non_finite_positions_stay_in_their_elements(bad, prec):
+    """The force is not finite at the nodes of the elements that hold the node, as from the gradient stream;
+    a first-order solve from there reports it."""
+    x, y, z, conn = box(9, 3, 2, 10)
+    fixed, f_ext, _ = M.cantilever_loads(x, y, z, (10.0, 20.0, -50.0))
+    el = make_element(x, y, z, conn, fixed=fixed, f_ext=f_ext)
+    el.SetForcePrecision(prec)
+    xs = perturb(x, y, z, 1e-3, 6)
+    xs[1][conn[100, 5]] = bad
+    el.UpdatePositions(*xs)
+    finite = []
+    for kernel in ("auto", "tma"):
+        el.SetLaunchConfig(kernel)
+        el.ComputeInternalForce()
+        finite.append(np.isfinite(el.RetrieveInternalForceToCPU().reshape(-1, 3)).all(1))
+    near = np.unique(conn[(conn == conn[100, 5]).any(1)])
+    assert not finite[0][near].any() and np.array_equal(finite[0], finite[1])
+    s = T.SyncedNesterovSolver(el, el.get_n_constraint())
+    s.Setup()
+    s.SetParameters(T.SyncedNesterovParams(1.0e-5, 1e8, 0.0, 0.0, 1, 8, 1.0e-3))
+    with pytest.raises(T.TLFEAError, match="NONFINITE"):
+        s.Solve()
+    del s
+    el.Destroy()
+
+
 @pytest.mark.parametrize("prec", ["fp64", "fp32"])
 def test_default_force_kernel_can_be_chosen_again(prec):
     x, y, z, conn = box(9, 3, 2, 10)
@@ -291,11 +420,14 @@ def test_internal_force_beside_orphans_and_of_curved_elements():
 
 
 # ---------------------------------------------------------------- first-order solvers
-# one tile, whole tiles, a ragged last tile; 610 tiles: beyond the resident launch (444 in FP64)
+# one tile, whole tiles, a ragged last tile; 197 and 352 tiles: the resident launch's blocks of 192 threads (two
+# tiles an SM) and of 128 (AdamW; Nesterov's phases); 610: beyond it (444 in FP64)
 @pytest.mark.parametrize("kind,cells,order", [
     ("nesterov", (3, 2, 2), 10), ("nesterov", (8, 4, 2), 10), ("nesterov", (9, 3, 2), 10),
     ("nesterov", (31, 3, 2), 4), ("nesterov", (130, 10, 10), 10), ("adamw", (9, 3, 2), 10), ("adamw", (31, 3, 2), 4),
-    ("nocoop", (8, 4, 2), 10), ("adamw", (130, 10, 10), 10)])
+    ("nocoop", (8, 4, 2), 10), ("adamw", (130, 10, 10), 10), ("nesterov", (42, 10, 10), 10),
+    ("nesterov", (75, 10, 10), 10), ("adamw", (42, 10, 10), 10), ("adamw", (75, 10, 10), 10),
+    ("nocoop", (42, 10, 10), 10), ("nocoop", (75, 10, 10), 10), ("nesterov", (42, 10, 10), 4), ("adamw", (75, 10, 10), 4)])
 def test_first_order_steps_on_straight_elements(kind, cells, order):
     from .test_gpu_solvers import ADAMW, E_MOD, _oracle_displacement_with_bar
 
@@ -425,22 +557,28 @@ def test_density_and_damping_changed_between_steps_of_sequences(damped):
     assert np.array_equal(out[0], out[1])
 
 
-@pytest.mark.parametrize("cells", [(9, 3, 2), (130, 10, 10)])
-def test_first_order_fp32_forces_on_straight_elements(cells):
+# the resident launch in FP32: blocks of 512, 256 and 128 threads (up to 592 tiles); beyond it
+@pytest.mark.parametrize("kind,cells", [("nesterov", (9, 3, 2)), ("nesterov", (42, 10, 10)), ("nesterov", (130, 10, 10)),
+                                        ("adamw", (42, 10, 10)), ("adamw", (110, 10, 10))])
+def test_first_order_fp32_forces_on_straight_elements(kind, cells):
     """Element forces in FP32 against the oracle: the solvers' bar for FP32 forces, 1e-4 of the
     displacement."""
-    from .test_gpu_solvers import E_MOD, _oracle_displacement_with_bar
+    from .test_gpu_solvers import ADAMW, E_MOD, _oracle_displacement_with_bar
 
     x, y, z, conn = box(*cells, 10)
     fixed, f, _ = M.cantilever_loads(x, y, z, (10.0, 20.0, -50.0))
     params = (1.0e-5, 1e8, 0.0, 0.0, 2, 8, 1.0e-3)
+    if kind == "adamw":
+        a = list(ADAMW)
+        a[0], a[3], a[6], a[7], a[8], a[9], a[10] = 1e-3, 1.0, 0.0, 0.0, 1e4, 2, 8
+        params = tuple(a)
     el = make_element(x, y, z, conn, fixed=fixed, f_ext=f)
     el.SetForcePrecision("fp32")
-    s = T.SyncedNesterovSolver(el, el.get_n_constraint())
+    s = (T.SyncedNesterovSolver if kind == "nesterov" else T.SyncedAdamWSolver)(el, el.get_n_constraint())
     s.Setup()
-    s.SetParameters(T.SyncedNesterovParams(*params))
+    s.SetParameters((T.SyncedNesterovParams if kind == "nesterov" else T.SyncedAdamWParams)(*params))
     s.Solve()
-    disp, _ = _oracle_displacement_with_bar(x, y, z, conn, E_MOD, fixed, f, "nesterov", params, 1)
+    disp, _ = _oracle_displacement_with_bar(x, y, z, conn, E_MOD, fixed, f, kind, params, 1)
     assert rel(np.stack(el.RetrievePositionToCPU()) - np.stack([x, y, z]), disp) < 1e-4
     del s
     el.Destroy()
