@@ -91,6 +91,7 @@ struct tlfea_batch_s {
     // FP32 element work: iterations summed over the refinement passes
     // straight-sided meshes (batch_lin.cuh)
     bool lin = false;
+    int sms = 1;
     double *lin_p = nullptr, *lin_slots = nullptr, *lin_pair = nullptr;
     int *stamp = nullptr, *tile_pair = nullptr, *inst_pair = nullptr, *node_inst = nullptr;
     std::vector<int> iters_total;
@@ -982,11 +983,11 @@ template <typename R>
 static size_t general_smem(const tlfea_batch_s* b);
 
 // Instances that share a pass of a tile's tables (shared mesh): up to eight, as long as every
-// resident block (about 600) still gets some four passes; a small batch gives each block one.
+// resident block (four per SM) still gets four passes; a small batch gives each block one.
 static int blin_group(const tlfea_batch_s* b) {
     if (!b->shared) return 1;
     const long long units = (long long)b->el->tl.n_tiles * b->n_inst;
-    return (int)std::max(1LL, std::min<long long>(std::min(b->n_inst, 8), units / 2400));
+    return (int)std::max(1LL, std::min<long long>(std::min(b->n_inst, 8), units / (4LL * 4 * b->sms)));
 }
 
 template <typename R>
@@ -1063,7 +1064,7 @@ static size_t batch_smem(const tlfea_batch_s* b) {
     return general_smem<R>(b);
 }
 
-// Shared memory of the per-point tile routine (curved meshes, and Apply).
+// Shared memory of the per-point tile routine (curved meshes).
 template <typename R>
 static size_t general_smem(const tlfea_batch_s* b) {
     const size_t ml = (size_t)b->el->tl.max_local;
@@ -1317,13 +1318,9 @@ static int blin_phased(tlfea_batch_s* b, double tol, int max_iter, bool warm, cu
     // all running, 329 / 283 with 64, 177 / 102 with eight, 146 / 37 with one; 512 uneven beams 834 /
     // 944, 152 / 157, 78 / 65, 75 / 61.
     int resident_grid[2] = {0, 0};  // update, direction
-    {
-        int sms = 0;
-        TLFEA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->el->device));
-        TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident_grid[0], k_bl_update<R>, TILE_ELEMS, 0));
-        TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident_grid[1], k_bl_direction<R>, TILE_ELEMS, 0));
-        for (int& g : resident_grid) g = std::max(1, std::min(chunk_grid, g * sms));
-    }
+    TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident_grid[0], k_bl_update<R>, TILE_ELEMS, 0));
+    TLFEA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident_grid[1], k_bl_direction<R>, TILE_ELEMS, 0));
+    for (int& g : resident_grid) g = std::max(1, std::min(chunk_grid, g * b->sms));
     int* base = b->n_done + 1;
     TLFEA_CUDA(cudaMemsetAsync(b->n_done, 0, 2 * sizeof(int), st));
     k_bl_start<R><<<chunk_grid, TILE_ELEMS, 0, st>>>(A, w);
@@ -1506,6 +1503,7 @@ static int batch_alloc_lin(tlfea_batch_s* b) {
     const int n_inst = b->n_inst;
     const Tiling& tl = b->el->tl;
     const long long lin_slots = tl.n_local_total * (b->shared ? n_inst : 1);
+    TLFEA_CUDA(cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, b->el->device));
     if (!tl.straight || BLinLayout<double, 10>(tl.max_local_pad).total > 200 * 1024 || lin_slots >= (1LL << 31))
         return TLFEA_OK;
     std::vector<int> tp, ip((size_t)n_inst + 1, 0), ni;

@@ -341,9 +341,9 @@ __global__ void __launch_bounds__(TILE_ELEMS, NPE == 10 ? 3 : 4) k_dyn_force_str
 }
 
 // As k_dyn_grad, up to DYN_GRAD_NODES nodes per thread: a block that ends pays the reduction's
-// fence and ticket, so a sequence has few blocks; below DYN_GRAD_FILL blocks (4 per SM) of one
+// fence and ticket, so a sequence has few blocks; below DYN_GRAD_FILL blocks per SM of one
 // node a thread the chip is not full and a thread's nodes would only queue.
-constexpr int DYN_GRAD_NODES = 4, DYN_GRAD_FILL = 592;
+constexpr int DYN_GRAD_NODES = 4, DYN_GRAD_FILL = 4;
 __global__ void __launch_bounds__(DYN_NODE_THREADS) k_dyn_grad_straight(DynArgs D) {
     __shared__ double red_sh[32];
     __shared__ bool last;
@@ -965,7 +965,9 @@ int tlfea_dynbatch_create(tlfea_element mesh, int n_seq, tlfea_dynbatch* out) {
     D.restart = 0;
     D.node_soff = el->tl.node_soff;
     D.n_slots = el->tl.n_local_total;
-    const int per_thread = std::min(DYN_GRAD_NODES, std::max(1, bps * b->B / DYN_GRAD_FILL));
+    int sms = 1;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, el->device);
+    const int per_thread = std::min(DYN_GRAD_NODES, std::max(1, bps * b->B / (DYN_GRAD_FILL * std::max(sms, 1))));
     D.grad_blocks = (bps + per_thread - 1) / per_thread;
     cudaMemsetAsync(b->mom, 0, B * sizeof(int), stream);
     const dim3 grid(bps, n_seq);

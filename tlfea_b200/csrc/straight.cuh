@@ -173,7 +173,7 @@ __device__ __forceinline__ void st_node(double* p, double a, double b, double c)
 }
 
 // Sum of the tile's element forces at one node: entries [beg, end) of its incidence list, in
-// that order, eight loads in flight at a time (a corner node has up to 24).
+// that order, NK = 6 loads in flight at a time (a corner node has up to 24).
 template <typename R>
 __device__ __forceinline__ void tile_node_sum(const R* fe, const uint16_t* incs, int beg, int end, double& s0,
                                               double& s1, double& s2) {
