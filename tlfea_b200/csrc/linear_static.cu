@@ -492,7 +492,7 @@ __global__ void k_pcg_axpy_dot(int N, const double* __restrict__ dinv, double* u
 
 static int cg_grid(const tlfea_solver_s* s) { return s->cg_blocks; }
 
-// At deformed positions and on curved elements (lin_applies below has the others): the
+// At deformed positions, on curved elements and for the budgets that lin_applies below leaves: the
 // matrix-free product where it applies -- SVK without damping, no preconditioner, TET10 -- and,
 // by default, where it pays: with the earlier per-node-gradient product the
 // assembled SpMV measured faster on TET4 (few QPs, small K blocks: 7.5 against 5.7
