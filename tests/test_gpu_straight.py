@@ -746,12 +746,15 @@ def test_static_solves_report_an_expired_wait(cells, operator):
     capi.call("tlfea_test_expire_wait", el._handle())
     late(s.Solve)
     assert np.array_equal(np.stack(el.RetrievePositionToCPU()), np.stack([x, y, z]))
+    v = torch.zeros(3 * len(x), dtype=torch.float64, device="cuda")
+    w = torch.empty_like(v)
+    torch.cuda.synchronize()
+    if operator == "auto":  # (with the assembled operator K stands)
+        with pytest.raises(T.TLFEAError, match="NOT_SETUP"):
+            s.Apply(v.data_ptr(), w.data_ptr())
     s.Solve()
     assert s.GetLastIterCount() == 25
     if operator == "auto":
-        v = torch.zeros(3 * len(x), dtype=torch.float64, device="cuda")
-        w = torch.empty_like(v)
-        torch.cuda.synchronize()
         capi.call("tlfea_test_expire_wait", el._handle())
         late(s.Apply, v.data_ptr(), w.data_ptr())
         s.Apply(v.data_ptr(), w.data_ptr())

@@ -951,8 +951,6 @@ static int lin_solve(tlfea_solver_s* s, bool* solved) {
     }
     *solved = true;
     s->lin_last = true;
-    s->mf_last = false;
-    s->k_built = false;
     if ((rc = keep_positions(s))) return rc;
     return finish_solve(s, h);
 }
@@ -969,6 +967,7 @@ int linear_static_solve(tlfea_solver_s* s) {
     const int N = el->N, n3 = 3 * N;
     s->op = {el->material, el->lambda, el->mu,    el->eta_d,            el->lambda_d,
              el->mu10,     el->mu01,   el->kappa, el->n_constraint > 0, el->geometry_version};
+    s->lin_last = s->mf_last = s->k_built = false;  // a solve that fails leaves no operator
     // the right-hand side and the Dirichlet DOFs
     TLFEA_CUDA(cudaMemcpyAsync(s->f, el->f_ext, sizeof(double) * n3, cudaMemcpyDeviceToDevice, stream));
     TLFEA_CUDA(cudaMemsetAsync(s->is_fixed, 0, n3, stream));
@@ -982,7 +981,6 @@ int linear_static_solve(tlfea_solver_s* s) {
         if ((st = lin_solve(s, &solved))) return st;
         if (solved) return TLFEA_OK;
     }
-    s->lin_last = false;
     const bool mf = use_matrix_free(s);
     if (mf) {
         // matrix-free K p at these positions: keep a copy (the products' tangent stream is
@@ -1015,12 +1013,10 @@ int linear_static_solve(tlfea_solver_s* s) {
         if (smem > 48 * 1024)
             TLFEA_CUDA(cudaFuncSetAttribute((const void*)mf_kernel(s), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             (int)smem));
-        s->k_built = false;
         s->mf_last = true;
     } else {
         if ((st = prepare_k(s))) return st;
         if ((st = assemble_k(s, el->x, el->y, el->z))) return st;
-        s->mf_last = false;
     }
     // SolveLinearSystemCG
     const int G = cg_grid(s);
